@@ -62,76 +62,175 @@ __device__ __forceinline__ bool grid_barrier(unsigned int* bar, unsigned int nbl
     return s_ok != 0;
 }
 
-// Grid barrier taken by ONE thread per block (the caller synchronises its block around
-// it).  bar[0] counts arrivals and only grows: it is a multiple of nblocks between
-// barriers (the host zeroes it before the launch), so an arrival's target is the next
-// multiple.  One atomic per block, then acquire loads.  A thread that waits longer than
-// the limit (bar[3]) sets the error flag bar[2]; every waiter sees the flag and returns
-// false, so the kernel ends with an error status instead of hanging.  Blocks must not mix
-// it with grid_barrier after their first call (grid_barrier resets bar[0]).
-__device__ __forceinline__ unsigned int ld_acquire_u32(const unsigned int* p) {
-    unsigned int v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+// ---- grid-wide sums that are the barrier as well
+//
+// A phase of the persistent kernels ends with every block publishing its partial sums and
+// every block reading all of them: nobody can have them all before everybody has arrived,
+// so reading the sums IS the barrier.  Against a counter and a second read of the partials
+// this saves the serialised atomics of 148 blocks and one L2 round trip per phase (FP32
+// sphere solve, 450k contacts: see k_apgd_sph for both sides measured).
+//
+// A slot holds 8 doubles per block; an unpublished value is all ones bits (a NaN that
+// publish() never writes).  Phase m uses slot m & 3, and at phase m a block empties its own
+// record of slot (m + 2) & 3: it was last read in phase m - 2, and this block has passed
+// phase m - 1, which every block enters only after its phase m - 2 reads.  The emptied
+// record is ordered before this block's next publication by the fence of publish().
+// The host sets all slots to all ones before the launch.
+constexpr int kSumSlots = 4;
+constexpr int kSumRec = 8;
+constexpr int kSumMaxBlocks = 160;  // five records per lane of the collecting warp
+
+__device__ __forceinline__ double sum_empty() { return __longlong_as_double(-1ll); }
+__device__ __forceinline__ bool sum_is_empty(double v) { return __double_as_longlong(v) == -1ll; }
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+__device__ __forceinline__ void st_relaxed_f64(double* p, double v) {
+    asm volatile("st.relaxed.gpu.global.f64 [%0], %1;" ::"l"(p), "d"(v) : "memory");
+}
+__device__ __forceinline__ double ld_relaxed_f64(const double* p) {
+    double v;
+    asm volatile("ld.relaxed.gpu.global.f64 %0, [%1];" : "=d"(v) : "l"(p) : "memory");
     return v;
 }
-// Split form: grid_arrive publishes this block's writes and returns the arrival target;
-// the block may do independent work before grid_wait.
-__device__ __forceinline__ unsigned int atom_add_release_u32(unsigned int* p, unsigned int v) {
-    unsigned int old;
-    asm volatile("atom.release.gpu.global.add.u32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
+__device__ __forceinline__ void ld_relaxed_2f64(const double* p, double& a, double& b) {
+    asm volatile("ld.relaxed.gpu.global.v2.f64 {%0, %1}, [%2];" : "=d"(a), "=d"(b) : "l"(p) : "memory");
 }
-// The arrival is a release at GPU scope: it orders before it every write this thread has
-// observed, which after the block barrier that precedes the call are all the block's
-// writes (release is cumulative), so no separate fence is needed.  withhold: compute the
-// target without counting this block (the timeout test: the barrier never completes and
-// every waiter gives up after the limit).
-__device__ __forceinline__ unsigned int grid_arrive(unsigned int* bar, unsigned int nblocks, bool withhold = false) {
-    const unsigned int old = withhold ? ld_acquire_u32(bar) : atom_add_release_u32(bar, 1u);
-    return (old / nblocks + 1u) * nblocks;
+
+template <int NP>
+struct SumShift {
+    // lanes per value of multi_reduce<NP> (NP = 1, 2, 4 or 8), as a shift
+    static constexpr int value = NP == 1 ? 5 : NP == 2 ? 4 : NP == 4 ? 3 : 2;
+};
+// Sums of NP values over the warp: lane l returns the sum of value l >> SumShift<NP>.  Each
+// exchange halves the values a lane carries (9 shuffles for 8 values instead of 40); the
+// additions are those of a shfl_down tree over lanes (+16, +8, +4, +2, +1), pair by pair.
+template <int NP>
+__device__ __forceinline__ double multi_reduce(double* v) {
+    const int lane = threadIdx.x & 31;
+    int o = 16;
+#pragma unroll
+    for (int h = NP / 2; h >= 1; h >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < h; ++i) {
+            const double send = up ? v[i] : v[i + h];
+            const double keep = up ? v[i + h] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+        }
+    }
+    double x = v[0];
+#pragma unroll
+    for (; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    return x;
 }
-__device__ __forceinline__ bool grid_wait(unsigned int* bar, unsigned int target) {
-    volatile unsigned int* verr = bar + 2;
+
+// Value k of this block's record for phase m (called by whole warp 0; `holds` marks the lanes
+// with a value).  Everything the block wrote before the block barrier that precedes the call
+// is visible to whoever collects the record (fence, then relaxed stores).
+__device__ __forceinline__ void sum_publish(double* slots, unsigned int nb, unsigned int m, bool holds, int k, double v,
+                                            bool withhold) {
+    const size_t rec = (size_t)blockIdx.x * kSumRec + k;
+    if (holds) st_relaxed_f64(slots + (size_t)((m + 2) & 3) * nb * kSumRec + rec, sum_empty());
+    fence_gpu();
+    if (holds && !withhold)
+        st_relaxed_f64(slots + (size_t)(m & 3) * nb * kSumRec + rec, v == v ? v : __longlong_as_double(0x7ff8000000000000ll));
+}
+
+// The NP values of all nb blocks (nb <= kSumMaxBlocks): lane l gets blocks l, l + 32, ... in
+// x[0..4] (zeros past nb).  Called by one whole warp.  A wait longer than the limit (bar[3])
+// sets the error flag bar[2]; every waiter sees the flag and returns false.
+template <int NP>
+__device__ __forceinline__ bool sum_collect(const double* slots, unsigned int nb, unsigned int m, unsigned int* bar,
+                                            double (&x)[5][NP]) {
+    const unsigned int lane = threadIdx.x & 31;
+    const double* base = slots + (size_t)(m & 3) * nb * kSumRec;
+    unsigned int pending = 0;
+#pragma unroll
+    for (int w = 0; w < 5; ++w) {
+#pragma unroll
+        for (int k = 0; k < NP; ++k) x[w][k] = 0.0;
+        if (lane + 32u * w < nb) pending |= 1u << w;
+    }
     const unsigned long long limit = barrier_limit_ns(bar);
-    unsigned int it = 0;
     unsigned long long t0 = 0;
-    for (;;) {
-        if ((int)(ld_acquire_u32(bar) - target) >= 0) break;
-        if (*verr) return false;
-        if (((++it) & 1023u) == 0) {
+    bool ok = true;
+    for (unsigned int it = 1;; ++it) {
+#pragma unroll
+        for (int w = 0; w < 5; ++w) {
+            if (!(pending & (1u << w))) continue;
+            const double* r = base + (size_t)(lane + 32u * w) * kSumRec;
+            if (NP == 1) {
+                x[w][0] = ld_relaxed_f64(r);
+            } else {
+#pragma unroll
+                for (int k = 0; k + 1 < NP; k += 2) ld_relaxed_2f64(r + k, x[w][k], x[w][k + 1]);
+            }
+        }
+#pragma unroll
+        for (int w = 0; w < 5; ++w) {
+            if (!(pending & (1u << w))) continue;
+            bool got = true;
+#pragma unroll
+            for (int k = 0; k < NP; ++k) got = got && !sum_is_empty(x[w][k]);
+            if (got) pending &= ~(1u << w);
+        }
+        if (__all_sync(0xffffffffu, pending == 0)) break;
+        if ((it & 63u) == 0) {
             const unsigned long long t = global_ns();
+            bool late = *(volatile unsigned int*)(bar + 2) != 0u;
             if (t0 == 0) {
                 t0 = t;
             } else if (t - t0 > limit) {
                 atomicExch(bar + 2, 1u);
-                return false;
+                late = true;
+            }
+            if (__any_sync(0xffffffffu, late)) {
+                ok = false;
+                break;
             }
         }
-        if (it > 32) __nanosleep(32);
+        if (it > 8) __nanosleep(32);
     }
-    // the acquire load that saw the target orders the reads after it (the block barrier that
-    // follows extends that to the other threads of the block)
-    return *verr == 0u;
+    fence_gpu();
+    return ok;
 }
-__device__ __forceinline__ bool grid_arrive_wait(unsigned int* bar, unsigned int nblocks) {
-    return grid_wait(bar, grid_arrive(bar, nblocks));
+// Orders of the grid sum.  Lane order: lane l adds its blocks l, l + 32, ..., then the tree
+// over lanes.  Group order: a tree per 32 consecutive blocks, then the groups in order.  Both
+// give lane l the total of value l >> SumShift<NP>, the same bits in every block.
+template <int NP>
+__device__ __forceinline__ double sum_lane_order(const double (&x)[5][NP]) {
+    double t[NP];
+#pragma unroll
+    for (int k = 0; k < NP; ++k) {
+        t[k] = 0.0;
+#pragma unroll
+        for (int w = 0; w < 5; ++w) t[k] += x[w][k];
+    }
+    return multi_reduce<NP>(t);
+}
+template <int NP>
+__device__ __forceinline__ double sum_group_order(double (&x)[5][NP]) {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < 5; ++w) s += multi_reduce<NP>(x[w]);
+    return s;
 }
 
-// Sum over the grid of per-block partials part[b*stride + k] (b < nb), computed by one
-// warp: lane l adds blocks l, l+32, ... in order, then a fixed shuffle tree.  Every block
-// gets the same bits.  The result is in lane 0.
+// Block partials of NP per-thread values, first half: per-warp sums into sh[k][warp].  After a
+// block barrier, warp 0 finishes with block_sums_tree (tree over warps) or
+// block_sums_in_order (warps one after the other); lane l gets value l >> SumShift<NP>.
 template <int NP>
-__device__ __forceinline__ void warp_grid_sum(const double* part, unsigned int nb, int stride, double* t) {
+__device__ __forceinline__ void warp_sums(double* v, double (*sh)[32]) {
     const int lane = threadIdx.x & 31;
+    const double x = multi_reduce<NP>(v);
+    if ((lane & ((1 << SumShift<NP>::value) - 1)) == 0) sh[lane >> SumShift<NP>::value][threadIdx.x >> 5] = x;
+}
+template <int NP>
+__device__ __forceinline__ double block_sums_tree(const double (*sh)[32]) {
+    const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    double v[NP];
 #pragma unroll
-    for (int k = 0; k < NP; ++k) t[k] = 0.0;
-    for (unsigned int b = lane; b < nb; b += 32)
-#pragma unroll
-        for (int k = 0; k < NP; ++k) t[k] += __ldcg(part + (size_t)b * stride + k);
-#pragma unroll
-    for (int k = 0; k < NP; ++k)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) t[k] += __shfl_down_sync(0xffffffffu, t[k], o);
+    for (int k = 0; k < NP; ++k) v[k] = lane < nw ? sh[k][lane] : 0.0;
+    return multi_reduce<NP>(v);
 }
 
 // Fixed-order sum of NP doubles over the block (up to 1024 threads); the result is
@@ -186,16 +285,57 @@ __device__ __forceinline__ void block_reduce_t0(double* v) {
     }
 }
 
-// Every block sums the per-block partials part[b*stride + k] (b < nb) in the same order.
-template <int NP>
-__device__ __forceinline__ void grid_sum(const double* part, unsigned int nb, int stride, double* t) {
+// The sums of one phase after the other over the grid (every block of a cooperative launch).
+// publish: all threads, their NP values (block sums in tree order); collect: warp 0, the
+// totals in lane order in every lane; next: all threads, once per phase.
+struct GridSums {
+    double* slots;
+    unsigned int nb;
+    unsigned int* bar;
+    unsigned int m;   // phase
+    bool withhold;    // test of the wait limit: this block never publishes its first phase
+
+    template <int NP>
+    __device__ __forceinline__ void publish(double* v, double (*sh)[32]) {
+        warp_sums<NP>(v, sh);
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            constexpr int sf = SumShift<NP>::value;
+            const double x = block_sums_tree<NP>(sh);
+            sum_publish(slots, nb, m, (threadIdx.x & ((1 << sf) - 1)) == 0, threadIdx.x >> sf, x, withhold && m == 0);
+        }
+    }
+    template <int NP>
+    __device__ __forceinline__ bool collect(double* t) {
+        double x[5][NP];
+        const bool ok = sum_collect<NP>(slots, nb, m, bar, x);
+        const double y = sum_lane_order<NP>(x);
 #pragma unroll
-    for (int k = 0; k < NP; ++k) t[k] = 0.0;
-    for (unsigned int b = threadIdx.x; b < nb; b += blockDim.x)
-#pragma unroll
-        for (int k = 0; k < NP; ++k) t[k] += __ldcg(part + (size_t)b * stride + k);
-    block_sum<NP>(t);
-}
+        for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, y, k << SumShift<NP>::value);
+        return ok;
+    }
+    __device__ __forceinline__ void next() { ++m; }
+    // one value per block (the same in all its threads), summed in group order; a full barrier
+    __device__ __forceinline__ bool exchange(double v, double& total) {
+        __shared__ double s_t;
+        __shared__ int s_ok;
+        __syncthreads();
+        if (threadIdx.x < 32) {
+            sum_publish(slots, nb, m, threadIdx.x == 0, 0, v, withhold && m == 0);
+            double x[5][1];
+            const bool ok = sum_collect<1>(slots, nb, m, bar, x);
+            const double y = sum_group_order<1>(x);
+            if (threadIdx.x == 0) {
+                s_t = y;
+                s_ok = ok;
+            }
+        }
+        ++m;
+        __syncthreads();
+        total = s_t;
+        return s_ok != 0;
+    }
+};
 
 // LagrangeMultiplier<Friction>::projection, include/scopi/solvers/lagrange_multiplier.hpp:243-268
 template <int DIM>

@@ -94,7 +94,7 @@ struct SphArgs {
     V4<T>* u1;
     V4<T>* u2;
     V4<T>* u3;
-    double* partials;
+    double* sums;  // kSumSlots x blocks x kSumRec, all ones at launch
     unsigned int* bar;
     ApgdResult* result;
     const Sizes* sizes;
@@ -156,8 +156,133 @@ struct SphState {
     double alpha, lipsch, theta, beta, beta_n, theta1, Fy, last_step, lgood;
     double tk[4];  // g.d, |d|^2, c.l+ and |l+|^2 of the candidate (contact pass sums)
     long long ite, nbt, nrs;
-    int il, ip, in_, jL, jN, jY, jYN, parity, bt, use_prev, restart, done, conv, err;
+    int il, ip, in_, jL, jN, jY, jYN, bt, use_prev, restart, done, conv, err;
 };
+__device__ __forceinline__ void state_init(SphState& S, double alpha) {
+    S.alpha = alpha;
+    S.lipsch = 1.0 / alpha;
+    S.lgood = S.lipsch;
+    S.theta = 1.0;
+    S.beta = 0.0;
+    S.beta_n = 0.0;
+    S.theta1 = 1.0;
+    S.Fy = 0.0;
+    S.last_step = 0.0;
+    S.ite = S.nbt = S.nrs = 0;
+    S.il = 0; S.ip = 1; S.in_ = 2;           // lambda buffers: current, previous, candidate
+    S.jL = 0; S.jN = 1; S.jY = 2; S.jYN = 3;  // u buffers: u(l), u(candidate), u(y), u(next y)
+    S.bt = 0;
+    S.use_prev = 0;
+    S.restart = 0;
+    S.done = 0;
+    S.conv = 0;
+    S.err = 0;
+}
+
+// The two decisions of an iteration, taken by thread 0 of every block from the same sums.
+// What does not depend on the sums (momentum, both candidate steps, square roots) is computed
+// by prepare_* while the sums are still on their way.
+struct Momentum {
+    double theta1, beta;
+};
+__device__ __forceinline__ Momentum prepare_momentum(const SphState& S) {
+    const double th = S.theta;
+    Momentum m;
+    m.theta1 = 0.5 * (th * sqrt(4 + th * th) - th * th);
+    m.beta = th * (1 - th) / (th * th + m.theta1);
+    return m;
+}
+// after the contact pass: momentum for the next y if this candidate is accepted
+// (apgd.hpp:196-206); t: FP64 g.d, |d|^2, c.l+, F(y), |l+ - l|^2, g.(l+ - l), |l+|^2;
+// FP32 |d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2
+template <typename T>
+__device__ __forceinline__ void decide_momentum(SphState& S, const double* t, bool bt, int dynamic, Momentum m) {
+    constexpr bool f32 = sizeof(T) == 4;
+    S.theta1 = m.theta1;
+    S.restart = (dynamic && t[f32 ? 2 : 5] > 0) ? 1 : 0;
+    S.beta_n = S.restart ? 0.0 : m.beta;
+    if (!f32 && !bt) S.Fy = t[f32 ? 0 : 3];
+    // the scalars the decision needs after the second pass
+    S.last_step = t[f32 ? 1 : 4];
+    S.tk[0] = f32 ? 0.0 : t[0];
+    S.tk[1] = t[f32 ? 0 : 1];
+    S.tk[2] = f32 ? 0.0 : t[f32 ? 0 : 2];
+    S.tk[3] = t[f32 ? 3 : 6];
+}
+struct NextStep {
+    double tol, step, alpha_bt, lip_ok, alpha_ok;
+};
+template <typename T>
+__device__ __forceinline__ NextStep prepare_step(const SphState& S, double tol) {
+    NextStep n;
+    n.tol = tol;
+    if (sizeof(T) == 4) {
+        // FP32 iterations stall at their rounding floor; the FP64 correction recovers the rest
+        const double floor32 = 4.0 * 1.1920929e-7 * sqrt(S.tk[3]);
+        if (floor32 > n.tol) n.tol = floor32;
+    }
+    n.step = sqrt(S.last_step);
+    n.alpha_bt = 1. / (S.lipsch * 2);
+    n.lip_ok = S.lipsch * 0.97;
+    n.alpha_ok = 1. / n.lip_ok;
+    return n;
+}
+// after the particle pass: backtrack or accept (apgd.hpp:172-221); wu = w.u (FP64), curv =
+// |u(l+) - u(y)|^2_M (FP32)
+template <typename T>
+__device__ __forceinline__ void decide_step(SphState& S, double wu, double curv, double dt2, int dynamic,
+                                            long long max_ite, NextStep n) {
+    const double* tk = S.tk;
+    const double F_lp = 0.5 * dt2 * wu + tk[2];
+    if (dynamic && tk[1] == 0.0) {
+        double lip = S.lipsch, al = S.alpha;
+        long long nbt = S.nbt;
+        overflow_cascade(lip, al, nbt);
+        S.lipsch = lip;
+        S.alpha = al;
+        S.nbt = nbt;
+        n.lip_ok = lip * 0.97;
+        n.alpha_ok = 1. / n.lip_ok;
+    } else if (dynamic && sufficient_decrease_fails<T>(F_lp, S.Fy, tk[0], tk[1], dt2 * curv, S.lipsch)) {
+        S.lipsch *= 2;  // backtracking, apgd.hpp:172-182
+        S.alpha = n.alpha_bt;
+        S.bt = 1;
+        ++S.nbt;
+        return;
+    }
+    ++S.ite;
+    S.bt = 0;
+    if (isfinite(S.lipsch)) S.lgood = S.lipsch;
+    S.last_step = n.step;
+    int tmp = S.ip; S.ip = S.il; S.il = S.in_; S.in_ = tmp;
+    tmp = S.jL; S.jL = S.jN; S.jN = tmp;
+    tmp = S.jY; S.jY = S.jYN; S.jYN = tmp;
+    if (n.step < n.tol) {
+        S.conv = 1;
+        S.done = 1;
+        return;
+    }
+    S.beta = S.beta_n;
+    S.theta = S.restart ? 1.0 : S.theta1;
+    if (S.restart) ++S.nrs;
+    if (dynamic) {
+        S.lipsch = n.lip_ok;
+        S.alpha = n.alpha_ok;
+    }
+    S.use_prev = (S.beta != 0.0) ? 1 : 0;
+    if (S.ite >= max_ite) S.done = 1;
+}
+__device__ __forceinline__ void write_result(ApgdResult* r, const SphState& S) {
+    r->iterations = S.ite;
+    r->backtracks = S.nbt;
+    r->restarts = S.nrs;
+    r->converged = S.conv;
+    r->lam_buf = S.il;
+    r->u_buf = S.jL;
+    r->error = S.err;
+    r->last_step = S.last_step;
+    r->lipsch = S.lgood;
+}
 
 // One block per SM (SphShape): FP32 768 threads (80 registers, no spills), FP64 512 (128).
 // Per-phase globaltimer stamps at 1M spheres (3.0M contacts): FP32 70.6 us per iteration
@@ -165,6 +290,11 @@ struct SphState {
 // threads and the gathers one trip ahead; FP64 110.9 against 117.1.  Shared memory and L1
 // share the SM: the particle pass's incidence records live in L1, so deeper stages that
 // grow the shared memory slow it down (FP64 with 5 contact stages: 115.1 us).
+//
+// Each pass ends in grid sums that serve as the barrier (GridSums).  Against a barrier counter,
+// a second read of the partials and 40 shuffles per warp for eight sums, microseconds per
+// iteration: FP32 450k contacts 18.4 -> 16.8, 4.6M 112.0 -> 108.4; FP64 2k contacts 12.5 -> 10.8,
+// 133k 18.0 -> 16.0, 4.6M 197.5 -> 188.6 (same bits: the order of every sum is unchanged).
 //
 // Both passes stream their per-item records through a cp.async pipeline in dynamic shared
 // memory (the passes are separated by grid barriers, so they share it):
@@ -214,30 +344,11 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
     T* s_im = reinterpret_cast<T*>(s_ul + (sizeof(T) == 4 ? 2 : 1) * GP * NT);
     int* s_p0 = reinterpret_cast<int*>(s_im + GP * NT);
     int* s_p1 = s_p0 + GP * NT;
-    if (threadIdx.x == 0) {
-        S.alpha = A.alpha;
-        S.lipsch = 1.0 / A.alpha;
-        S.lgood = S.lipsch;
-        S.theta = 1.0;
-        S.beta = 0.0;
-        S.beta_n = 0.0;
-        S.theta1 = 1.0;
-        S.Fy = 0.0;
-        S.last_step = 0.0;
-        S.ite = S.nbt = S.nrs = 0;
-        S.il = 0; S.ip = 1; S.in_ = 2;           // lambda buffers: current, previous, candidate
-        S.jL = 0; S.jN = 1; S.jY = 2; S.jYN = 3;  // u buffers: u(l), u(candidate), u(y), u(next y)
-        S.parity = 0;
-        S.bt = 0;
-        S.use_prev = 0;
-        S.restart = 0;
-        S.done = 0;
-        S.conv = 0;
-        S.err = 0;
-    }
+    __shared__ double red[8][32];
+    if (threadIdx.x == 0) state_init(S, A.alpha);
     __syncthreads();
     const int C = A.sizes->C;
-    const unsigned int nb = gridDim.x;
+    GridSums G{A.sums, gridDim.x, A.bar, 0u, A.stall != 0 && blockIdx.x == 0};
     // Trip k of a thread handles item base + k*S (the grid-stride order) in both passes.
     const long long S_ = (long long)gridDim.x * NT, base = (long long)blockIdx.x * NT + tid;
     const long long ntrip_c = ((long long)C - (long long)blockIdx.x * NT + S_ - 1) / S_;
@@ -266,12 +377,11 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
         cp_commit();
     };
     bool geom_issued = false;
-    bool withhold = A.stall != 0 && blockIdx.x == 0;
     if (A.curvature_start) {
         // initial step from the curvature along the first descent direction d (stored in
-        // the candidate buffer, which the first contact pass overwrites); partial-sum
-        // regions 1 and 3 are first reused by the second iteration, after two barriers
+        // the candidate buffer, which the first contact pass overwrites)
         T* dbuf = A.lam2;
+        double t1 = 0.0, t3 = 0.0;
         double a2[2] = {0.0, 0.0};
         GRID_STRIDE(c, C) {
             const T cc = ld4(A.nc + c).w;
@@ -288,9 +398,7 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
             }
         }
         block_sum<2>(a2);
-        if (threadIdx.x == 0) A.partials[(size_t)1 * nb * 8 + blockIdx.x * 8] = a2[0];
-        bool ok = grid_barrier(A.bar, nb, withhold);
-        withhold = false;
+        bool ok = G.exchange(a2[0], t1);
         double wm[2] = {0.0, 0.0};
         if (ok) GRID_STRIDE(p, A.na) {
             T w0 = 0, w1 = 0, w2 = 0;
@@ -310,16 +418,10 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
             wm[0] += im * ((double)w0 * w0 + (double)w1 * w1 + (double)w2 * w2);
         }
         block_sum<2>(wm);
-        if (threadIdx.x == 0) A.partials[(size_t)3 * nb * 8 + blockIdx.x * 8] = wm[0];
-        if (ok) ok = grid_barrier(A.bar, nb);
-        double t1[1] = {0.0}, t3[1] = {0.0};
-        if (ok) {
-            grid_sum<1>(A.partials + (size_t)1 * nb * 8, nb, 8, t1);
-            grid_sum<1>(A.partials + (size_t)3 * nb * 8, nb, 8, t3);
-        }
+        if (ok) ok = G.exchange(wm[0], t3);
         if (threadIdx.x == 0) {
             double l;
-            if (ok && initial_lipschitz(t1[0], t3[0], A.dt2, l)) {
+            if (ok && initial_lipschitz(t1, t3, A.dt2, l)) {
                 S.lipsch = l;
                 S.alpha = 1.0 / l;
                 S.lgood = l;
@@ -340,8 +442,6 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
         const T* lprev = pick(S.ip, A.lam0, A.lam1, A.lam2);
         T* lnew = pick(S.in_, A.lam0, A.lam1, A.lam2);
         const V4<T>* uY = pick4(S.jY, A.u0, A.u1, A.u2, A.u3);
-        double* part = A.partials + (size_t)S.parity * nb * 8;
-        double* part2 = A.partials + (size_t)(2 + S.parity) * nb * 8;
         {
             double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
             // ---- contact pass: g = dt^2 n.(u_i(y) - u_j(y)) + c, l+ = P(y - alpha g)
@@ -419,72 +519,35 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
                 trip(k + 2, g2, g1);
             }
             cp_wait<0>();
-            // block partials to thread 0, grid barrier and grid sum in warp 0 only
-            // FP32 needs four of the sums (|d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2): they are
-            // reduced packed, in the first four slots of the block's record
+            // FP32 needs four of the sums (|d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2)
             constexpr int NS = sizeof(T) == 4 ? 4 : 8;
-            double r[NS];
             if (NS == 4) {
-                r[0] = s[1];
-                r[1 % NS] = s[4];
-                r[2 % NS] = s[5];
-                r[3 % NS] = s[6];
-            } else {
-#pragma unroll
-                for (int k = 0; k < NS; ++k) r[k] = s[k];
+                s[0] = s[1];
+                s[1] = s[4];
+                s[2] = s[5];
+                s[3] = s[6];
             }
-            block_reduce_t0<NS>(r);
-            unsigned int target = 0;
-            if (tid == 0) {
-                for (int k = 0; k < NS; ++k) part[blockIdx.x * 8 + k] = r[k];
-                target = grid_arrive(A.bar, nb, withhold);
-            }
-            withhold = false;
+            G.template publish<NS>(s, red);
             // every thread is past its contact loop: the particle pass's first stages fill
-            // the shared memory while the barrier waits (u(l) copied whatever beta is)
+            // the shared memory while the sums travel (u(l) copied whatever beta is)
             {
                 const V4<T>* uL0 = pick4(S.jL, A.u0, A.u1, A.u2, A.u3);
 #pragma unroll 1
                 for (int k = 0; k < GP - 1; ++k) issue_body(k, uL0, uY, true);
             }
             if (tid < 32) {
-                bool ok = true;
-                if (tid == 0) ok = grid_wait(A.bar, target);
-                ok = __shfl_sync(0xffffffffu, ok, 0) != 0;
-                __syncwarp();  // the lanes' partial loads come after lane 0's acquire
-                double t[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-                {
-                    double tt[NS];
-                    warp_grid_sum<NS>(part, nb, 8, tt);
-                    if (NS == 4) {
-                        t[1] = tt[0];
-                        t[4] = tt[1 % NS];
-                        t[5] = tt[2 % NS];
-                        t[6] = tt[3 % NS];
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < NS; ++k) t[k] = tt[k];
-                    }
-                }
+                const Momentum mo = prepare_momentum(S);
+                double t[NS];
+                const bool ok = G.template collect<NS>(t);
                 if (tid == 0) {
                     if (!ok) {
                         S.err = 1;
                         S.done = 1;
                     }
-                    // momentum for the next y if this candidate is accepted (apgd.hpp:196-206)
-                    const double th = S.theta;
-                    S.theta1 = 0.5 * (th * sqrt(4 + th * th) - th * th);
-                    S.restart = (A.dynamic && t[5] > 0) ? 1 : 0;
-                    S.beta_n = S.restart ? 0.0 : th * (1 - th) / (th * th + S.theta1);
-                    if (!bt) S.Fy = t[3];
-                    // the scalars the decision needs after the second pass
-                    S.last_step = t[4];
-                    S.tk[0] = t[0];
-                    S.tk[1] = t[1];
-                    S.tk[2] = t[2];
-                    S.tk[3] = t[6];
+                    decide_momentum<T>(S, t, bt, A.dynamic, mo);
                 }
             }
+            G.next();
         }
         __syncthreads();
         if (S.err) break;
@@ -560,90 +623,27 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
                 }
             }
             cp_wait<0>();
-            // FP64 reduces w.u (slot 0), FP32 the curvature (slot 1)
-            constexpr int NQ = sizeof(T) == 4 ? 1 : 2;
-            double sw8[2] = {sizeof(T) == 4 ? sq : sw, sq};
-            block_reduce_t0<NQ>(sw8);
-            unsigned int target2 = 0;
-            if (tid == 0) {
-                if (NQ == 1) {
-                    part2[blockIdx.x * 8 + 1] = sw8[0];
-                } else {
-                    part2[blockIdx.x * 8] = sw8[0];
-                    part2[blockIdx.x * 8 + 1] = sw8[1 % NQ];
-                }
-                target2 = grid_arrive(A.bar, nb);
-            }
-            // the next iteration's first contact geometry, while the barrier waits
+            // FP64 reduces w.u, FP32 the curvature
+            double sw1[1] = {sizeof(T) == 4 ? sq : sw};
+            G.template publish<1>(sw1, red);
+            // the next iteration's first contact geometry, while the sums travel
 #pragma unroll 1
             for (int k = 0; k < GC - 1; ++k) issue_geom(k);
             geom_issued = true;
-            bool ok = true;
-            double t6[2];
             if (tid < 32) {
-                if (tid == 0) ok = grid_wait(A.bar, target2);
-                ok = __shfl_sync(0xffffffffu, ok, 0) != 0;
-                __syncwarp();
-                if (NQ == 1) {
-                    t6[0] = 0.0;
-                    warp_grid_sum<1>(part2 + 1, nb, 8, t6 + 1);
-                } else {
-                    warp_grid_sum<2>(part2, nb, 8, t6);
-                }
-            }
-            if (tid == 0 && !ok) {
-                S.err = 1;
-                S.done = 1;
-            } else if (tid == 0) {
-                const double* tk = S.tk;
-                S.parity ^= 1;
-                const double F_lp = 0.5 * A.dt2 * t6[0] + tk[2];
-                bool accept = true;
-                if (A.dynamic && tk[1] == 0.0) {
-                    double lip = S.lipsch, al = S.alpha;
-                    long long nbt = S.nbt;
-                    overflow_cascade(lip, al, nbt);
-                    S.lipsch = lip;
-                    S.alpha = al;
-                    S.nbt = nbt;
-                } else if (A.dynamic && sufficient_decrease_fails<T>(F_lp, S.Fy, tk[0], tk[1], A.dt2 * t6[1],
-                                                                      S.lipsch)) {
-                    S.lipsch *= 2;  // backtracking, apgd.hpp:172-182
-                    S.alpha = 1. / S.lipsch;
-                    S.bt = 1;
-                    ++S.nbt;
-                    accept = false;
-                }
-                if (accept) {
-                    ++S.ite;
-                    S.bt = 0;
-                    if (isfinite(S.lipsch)) S.lgood = S.lipsch;
-                    S.last_step = sqrt(S.last_step);
-                    double tol = A.tol;
-                    if (sizeof(T) == 4) {
-                        // FP32 iterations stall at their rounding floor; the FP64 correction recovers the rest
-                        const double floor32 = 4.0 * 1.1920929e-7 * sqrt(tk[3]);
-                        if (floor32 > tol) tol = floor32;
-                    }
-                    int tmp = S.ip; S.ip = S.il; S.il = S.in_; S.in_ = tmp;
-                    tmp = S.jL; S.jL = S.jN; S.jN = tmp;
-                    tmp = S.jY; S.jY = S.jYN; S.jYN = tmp;
-                    if (S.last_step < tol) {
-                        S.conv = 1;
+                const NextStep ns = prepare_step<T>(S, A.tol);
+                double t[1];
+                const bool ok = G.template collect<1>(t);
+                if (tid == 0) {
+                    if (!ok) {
+                        S.err = 1;
                         S.done = 1;
                     } else {
-                        S.beta = S.beta_n;
-                        S.theta = S.restart ? 1.0 : S.theta1;
-                        if (S.restart) ++S.nrs;
-                        if (A.dynamic) {
-                            S.lipsch *= 0.97;
-                            S.alpha = 1. / S.lipsch;
-                        }
-                        S.use_prev = (S.beta != 0.0) ? 1 : 0;
-                        if (S.ite >= A.max_ite) S.done = 1;
+                        decide_step<T>(S, t[0], t[0], A.dt2, A.dynamic, A.max_ite, ns);
                     }
                 }
             }
+            G.next();
             __syncthreads();
             if (S.done) break;
         }
@@ -652,17 +652,7 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
     // uncommitted copies: commit them first)
     cp_commit();
     cp_wait<0>();
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        A.result->iterations = S.ite;
-        A.result->backtracks = S.nbt;
-        A.result->restarts = S.nrs;
-        A.result->converged = S.conv;
-        A.result->lam_buf = S.il;
-        A.result->u_buf = S.jL;
-        A.result->error = S.err;
-        A.result->last_step = S.last_step;
-        A.result->lipsch = S.lgood;
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) write_result(A.result, S);
 }
 
 // ------------------------------------------------------------------ packing
@@ -774,7 +764,7 @@ int max_blocks_sph() {
     int dev = 0, sms = kSMs;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    return per_sm * sms;
+    return std::min(per_sm * sms, kSumMaxBlocks);
 }
 
 template <typename T, int DIM, int PROB>
@@ -830,7 +820,7 @@ cudaError_t launch_apgd_sph(int nin, int na, int dim, int problem, const ApgdSet
     A.u1 = sb.u[1];
     A.u2 = sb.u[2];
     A.u3 = sb.u[3];
-    A.partials = sb.partials;
+    A.sums = sb.sums;
     A.bar = sb.barrier;
     A.result = sb.result;
     A.sizes = sizes;
@@ -917,7 +907,6 @@ namespace {
 
 constexpr long long kNoAllocMaxContacts = 16384;
 constexpr long long kNoAllocMaxBodies = 8192;
-constexpr int kNoAllocMaxBlocks = 4 * kSMs;
 
 constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
@@ -928,7 +917,7 @@ constexpr size_t kOffInvm = align_up(kOffInc + sizeof(dvec4) * 2 * kNoAllocMaxCo
 constexpr size_t kOffLam = align_up(kOffInvm + sizeof(double) * kNoAllocMaxBodies);
 constexpr size_t kOffU = align_up(kOffLam + sizeof(double) * 3 * kNoAllocMaxContacts);
 constexpr size_t kOffPart = align_up(kOffU + sizeof(dvec4) * 4 * kNoAllocMaxBodies);
-constexpr size_t kOffBar = align_up(kOffPart + sizeof(double) * 4 * kNoAllocMaxBlocks * 8);
+constexpr size_t kOffBar = align_up(kOffPart + (size_t)kSumBytesPerBlock * apgdc::kSumMaxBlocks);
 constexpr size_t kOffRes = align_up(kOffBar + 4 * sizeof(unsigned int));
 constexpr size_t kOffSizes = align_up(kOffRes + sizeof(ApgdResult));
 constexpr size_t kOffFlag = align_up(kOffSizes + sizeof(Sizes));
@@ -1142,7 +1131,7 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
     A.u1 = ub + kNoAllocMaxBodies;
     A.u2 = ub + 2 * kNoAllocMaxBodies;
     A.u3 = ub + 3 * kNoAllocMaxBodies;
-    A.partials = part;
+    A.sums = part;
     A.bar = bar;
     A.result = res;
     A.sizes = sizes;
@@ -1154,11 +1143,15 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
     A.curvature_start = 0;
     A.stall = 0;
     int maxb = apgd_sph_max_blocks(kNoFriction, dim, false);
-    if (maxb > kNoAllocMaxBlocks) maxb = kNoAllocMaxBlocks;
     const int thr = SphOcc<double>::threads;
     long long nb = (std::max<long long>(C, na) + thr - 1) / thr;
     if (nb < 1) nb = 1;
     if (nb > maxb) nb = maxb;
+    e = cudaMemsetAsync(part, 0xff, (size_t)kSumBytesPerBlock * nb, s);
+    if (e != cudaSuccess) {
+        set_global_error2("scopi_gpu_apgd_noalloc: cudaMemsetAsync: ", cudaGetErrorString(e));
+        return SCOPI_GPU_ECUDA;
+    }
     e = dim == 3 ? launch_t<double, 3, kNoFriction>(A, (int)nb, s) : launch_t<double, 2, kNoFriction>(A, (int)nb, s);
     if (e != cudaSuccess) {
         set_global_error2("scopi_gpu_apgd_noalloc: launch: ", cudaGetErrorString(e));

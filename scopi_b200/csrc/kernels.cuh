@@ -260,6 +260,9 @@ struct V4_of<double> {
 template <typename T>
 using V4 = typename V4_of<T>::type;
 
+// grid sums of a persistent launch: 4 slots of 8 doubles per block (apgd_common.cuh)
+constexpr int kSumBytesPerBlock = 4 * 8 * 8;
+
 template <typename T>
 struct SphSolve {
     const int2* cij;
@@ -271,7 +274,7 @@ struct SphSolve {
     const T* invm;            // 1/m per active body, contiguous
     T* lam[3];
     V4<T>* u[4];
-    double* partials;         // 4 * max_blocks * 8
+    double* sums;             // apgdc::kSumSlots * blocks * kSumRec, all ones at launch
     unsigned int* barrier;
     ApgdResult* result;
 };

@@ -114,6 +114,8 @@ struct scopi_gpu_handle {
     // fixed small buffers
     DevMem fixed_mem;
     double* d_partials = nullptr;
+    double* d_sums = nullptr;  // grid sums of the torque-free solve
+    size_t sums_bytes = 0;
     unsigned int* d_barrier = nullptr;
     ApgdResult* d_result = nullptr;
     unsigned long long* d_viol = nullptr;
@@ -555,6 +557,8 @@ struct scopi_gpu_handle {
         }
         const int mb = std::max({max_blocks64, max_blocks32, max_sph64, max_sph32, 1});
         if ((e = alloc(fixed_mem, d_partials, 4 * (size_t)mb * 8)) != cudaSuccess) return cuda_fail(e, "alloc");
+        sums_bytes = (size_t)kSumBytesPerBlock * mb;
+        if ((e = alloc(fixed_mem, d_sums, sums_bytes / sizeof(double))) != cudaSuccess) return cuda_fail(e, "alloc");
         if ((e = alloc(fixed_mem, d_barrier, 4)) != cudaSuccess) return cuda_fail(e, "alloc");
         if ((e = alloc(fixed_mem, d_result, 1)) != cudaSuccess) return cuda_fail(e, "alloc");
         if ((e = alloc(fixed_mem, d_viol, 1)) != cudaSuccess) return cuda_fail(e, "alloc");
@@ -893,6 +897,7 @@ struct scopi_gpu_handle {
         cudaError_t e = reset_barrier(st);
         if (e != cudaSuccess) return cuda_fail(e, "APGD barrier words");
         const int nb = nblocks_for(maxb, std::max<long long>(h_sizes->C, na), apgd_sph_threads(sizeof(T) == 4));
+        cudaMemsetAsync(sb.sums, 0xff, (size_t)kSumBytesPerBlock * nb, stream);
         e = launch_apgd_sph<T>(nin, na, P.dim, P.problem, st, sb, d_sizes_cur, nb, stream);
         if (e != cudaSuccess) return cuda_fail(e, "APGD launch");
         cudaMemcpyAsync(h_result, d_result, sizeof(ApgdResult), cudaMemcpyDeviceToHost, stream);
@@ -914,7 +919,7 @@ struct scopi_gpu_handle {
         sb.invm = imt;
         for (int k = 0; k < 3; ++k) sb.lam[k] = lam[k];
         for (int k = 0; k < 4; ++k) sb.u[k] = u[k];
-        sb.partials = d_partials;
+        sb.sums = d_sums;
         sb.barrier = d_barrier;
         sb.result = d_result;
         return sb;
