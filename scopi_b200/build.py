@@ -19,6 +19,7 @@ COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler",
 SOURCES = {
     "detect.cu": ["-fmad=false"],
     "apgd.cu": [],
+    "apgd_fric.cu": [],
     "apgd_sph.cu": [],
     "apgd_batch.cu": [],
     "se.cu": ["-fmad=false"],

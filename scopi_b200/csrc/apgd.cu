@@ -1,4 +1,5 @@
-// apgd.cu -- persistent, grid-synchronised APGD (accelerated projected gradient with
+// apgd.cu -- 6-dof rows of the normal problems and ViscousFriction (Friction: apgd_fric.cu):
+// persistent, grid-synchronised APGD (accelerated projected gradient with
 // backtracking Lipschitz estimate and gradient restart) on the contact QP
 //     min_l  1/2 l^T Q l + c^T l,  Q = dt^2 B M^-1 B^T,  l in K (R+ or the friction cone)
 // following apgd::operator() (include/scopi/solvers/apgd.hpp:148-221) step for step:
@@ -515,19 +516,6 @@ __global__ void __launch_bounds__(kApgdThreads) k_apgd(ApgdArgs<T> A) {
                 for (int k = 0; k < 4; ++k) {
                     const T v = (T)(z[k] - (A.shift ? A.shift[4 * c + k] : 0.0));
                     dbuf[4 * c + k] = v;
-                    s[1] += (double)v * (double)v;
-                }
-            } else if (PROB == kFriction) {
-                double z[3], n[3];
-                for (int d = 0; d < 3; ++d) {
-                    n[d] = (double)A.bn[3 * c + d];
-                    z[d] = -(double)A.cvec[3 * c + d] + (A.shift ? A.shift[3 * c + d] : 0.0);
-                }
-                if (DIM == 2) z[2] = A.shift ? A.shift[3 * c + 2] : 0.0;
-                cone_project<DIM>(z, n, A.mu);
-                for (int d = 0; d < 3; ++d) {
-                    const T v = (T)(z[d] - (A.shift ? A.shift[3 * c + d] : 0.0));
-                    dbuf[3 * c + d] = v;
                     s[1] += (double)v * (double)v;
                 }
             } else {
@@ -1164,11 +1152,9 @@ int apgd_max_blocks(int problem, int dim, bool fp32) {
 #define MB(T, D, P) \
     if (dim == D && problem == P) return max_blocks_t<T, D, P>();
     if (fp32) {
-        MB(float, 2, 0) MB(float, 2, 1) MB(float, 2, 2) MB(float, 2, 4)
-        MB(float, 3, 0) MB(float, 3, 1) MB(float, 3, 2) MB(float, 3, 4)
+        MB(float, 2, 0) MB(float, 2, 2) MB(float, 2, 4) MB(float, 3, 0) MB(float, 3, 2) MB(float, 3, 4)
     } else {
-        MB(double, 2, 0) MB(double, 2, 1) MB(double, 2, 2) MB(double, 2, 4)
-        MB(double, 3, 0) MB(double, 3, 1) MB(double, 3, 2) MB(double, 3, 4)
+        MB(double, 2, 0) MB(double, 2, 2) MB(double, 2, 4) MB(double, 3, 0) MB(double, 3, 2) MB(double, 3, 4)
     }
 #undef MB
     return 0;
@@ -1216,7 +1202,7 @@ cudaError_t launch_apgd_invm(const Bodies& b, const StepParams& p, const ApgdSet
     A.dynamic = st.dynamic;
 #define LA(D, P) \
     if (p.dim == D && p.problem == P) return launch_apgd_t<T, D, P>(A, nblocks, s);
-    LA(2, 0) LA(2, 1) LA(2, 2) LA(2, 4) LA(3, 0) LA(3, 1) LA(3, 2) LA(3, 4)
+    LA(2, 0) LA(2, 2) LA(2, 4) LA(3, 0) LA(3, 2) LA(3, 4)
 #undef LA
     return cudaErrorInvalidValue;
 }

@@ -286,8 +286,11 @@ __device__ __forceinline__ void block_reduce_t0(double* v) {
 }
 
 // The sums of one phase after the other over the grid (every block of a cooperative launch).
-// publish: all threads, their NP values (block sums in tree order); collect: warp 0, the
-// totals in lane order in every lane; next: all threads, once per phase.
+// publish: all threads, their NP values; collect: warp 0, the totals in every lane; next: all
+// threads, once per phase.  TREE: block sums as a tree over warps and lane order over blocks;
+// else warps one after the other and group order over blocks (each solve keeps one order, so
+// that its FP64 decisions do not depend on the launch).
+template <bool TREE>
 struct GridSums {
     double* slots;
     unsigned int nb;
@@ -300,16 +303,24 @@ struct GridSums {
         warp_sums<NP>(v, sh);
         __syncthreads();
         if (threadIdx.x < 32) {
-            constexpr int sf = SumShift<NP>::value;
-            const double x = block_sums_tree<NP>(sh);
-            sum_publish(slots, nb, m, (threadIdx.x & ((1 << sf) - 1)) == 0, threadIdx.x >> sf, x, withhold && m == 0);
+            if (TREE) {
+                constexpr int sf = SumShift<NP>::value;
+                const double x = block_sums_tree<NP>(sh);
+                sum_publish(slots, nb, m, (threadIdx.x & ((1 << sf) - 1)) == 0, threadIdx.x >> sf, x,
+                            withhold && m == 0);
+            } else {
+                double x = 0.0;
+                if (threadIdx.x < NP)
+                    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += sh[threadIdx.x][w];
+                sum_publish(slots, nb, m, threadIdx.x < NP, threadIdx.x, x, withhold && m == 0);
+            }
         }
     }
     template <int NP>
     __device__ __forceinline__ bool collect(double* t) {
         double x[5][NP];
         const bool ok = sum_collect<NP>(slots, nb, m, bar, x);
-        const double y = sum_lane_order<NP>(x);
+        const double y = TREE ? sum_lane_order<NP>(x) : sum_group_order<NP>(x);
 #pragma unroll
         for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, y, k << SumShift<NP>::value);
         return ok;
@@ -401,6 +412,144 @@ __device__ __forceinline__ void overflow_cascade(double& lipsch, double& alpha, 
         ++nbt;
     }
     alpha = 1. / lipsch;
+}
+
+// Loop-carried scalars of the iteration (block-uniform) live in shared memory and are
+// updated by thread 0, so the registers go to the two passes.
+struct ApgdState {
+    double alpha, lipsch, theta, beta, beta_n, theta1, Fy, last_step, lgood;
+    double tk[4];  // g.d, |d|^2, c.l+ and |l+|^2 of the candidate (contact pass sums)
+    long long ite, nbt, nrs;
+    int il, ip, in_, jL, jN, jY, jYN, bt, use_prev, restart, done, conv, err;
+};
+__device__ __forceinline__ void state_init(ApgdState& S, double alpha) {
+    S.alpha = alpha;
+    S.lipsch = 1.0 / alpha;
+    S.lgood = S.lipsch;
+    S.theta = 1.0;
+    S.beta = 0.0;
+    S.beta_n = 0.0;
+    S.theta1 = 1.0;
+    S.Fy = 0.0;
+    S.last_step = 0.0;
+    S.ite = S.nbt = S.nrs = 0;
+    S.il = 0; S.ip = 1; S.in_ = 2;           // lambda buffers: current, previous, candidate
+    S.jL = 0; S.jN = 1; S.jY = 2; S.jYN = 3;  // u buffers: u(l), u(candidate), u(y), u(next y)
+    S.bt = 0;
+    S.use_prev = 0;
+    S.restart = 0;
+    S.done = 0;
+    S.conv = 0;
+    S.err = 0;
+}
+
+// The two decisions of an iteration, taken by thread 0 of every block from the same sums.
+// What does not depend on the sums (momentum, both candidate steps, square roots) is computed
+// by prepare_* while the sums are still on their way.
+struct Momentum {
+    double theta1, beta;
+};
+__device__ __forceinline__ Momentum prepare_momentum(const ApgdState& S) {
+    const double th = S.theta;
+    Momentum m;
+    m.theta1 = 0.5 * (th * sqrt(4 + th * th) - th * th);
+    m.beta = th * (1 - th) / (th * th + m.theta1);
+    return m;
+}
+// after the contact pass: momentum for the next y if this candidate is accepted
+// (apgd.hpp:196-206); t: FP64 g.d, |d|^2, c.l+, F(y), |l+ - l|^2, g.(l+ - l), |l+|^2;
+// FP32 |d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2
+template <typename T>
+__device__ __forceinline__ void decide_momentum(ApgdState& S, const double* t, bool bt, int dynamic, Momentum m) {
+    constexpr bool f32 = sizeof(T) == 4;
+    S.theta1 = m.theta1;
+    S.restart = (dynamic && t[f32 ? 2 : 5] > 0) ? 1 : 0;
+    S.beta_n = S.restart ? 0.0 : m.beta;
+    if (!f32 && !bt) S.Fy = t[f32 ? 0 : 3];
+    // the scalars the decision needs after the second pass
+    S.last_step = t[f32 ? 1 : 4];
+    S.tk[0] = f32 ? 0.0 : t[0];
+    S.tk[1] = t[f32 ? 0 : 1];
+    S.tk[2] = f32 ? 0.0 : t[f32 ? 0 : 2];
+    S.tk[3] = t[f32 ? 3 : 6];
+}
+struct NextStep {
+    double tol, step, alpha_bt, lip_ok, alpha_ok;
+};
+template <typename T>
+__device__ __forceinline__ NextStep prepare_step(const ApgdState& S, double tol) {
+    NextStep n;
+    n.tol = tol;
+    if (sizeof(T) == 4) {
+        // FP32 iterations stall at their rounding floor; the FP64 correction recovers the rest
+        const double floor32 = 4.0 * 1.1920929e-7 * sqrt(S.tk[3]);
+        if (floor32 > n.tol) n.tol = floor32;
+    }
+    n.step = sqrt(S.last_step);
+    n.alpha_bt = 1. / (S.lipsch * 2);
+    n.lip_ok = S.lipsch * 0.97;
+    n.alpha_ok = 1. / n.lip_ok;
+    return n;
+}
+// after the particle pass: backtrack or accept (apgd.hpp:172-221); wu = w.u (FP64), curv =
+// |u(l+) - u(y)|^2_M (FP32); more than max_bt backtracks (0: no limit) end the solve with error 2
+template <typename T>
+__device__ __forceinline__ void decide_step(ApgdState& S, double wu, double curv, double dt2, int dynamic,
+                                            long long max_ite, NextStep n, long long max_bt = 0) {
+    const double* tk = S.tk;
+    const double F_lp = 0.5 * dt2 * wu + tk[2];
+    if (dynamic && tk[1] == 0.0) {
+        double lip = S.lipsch, al = S.alpha;
+        long long nbt = S.nbt;
+        overflow_cascade(lip, al, nbt);
+        S.lipsch = lip;
+        S.alpha = al;
+        S.nbt = nbt;
+        n.lip_ok = lip * 0.97;
+        n.alpha_ok = 1. / n.lip_ok;
+    } else if (dynamic && sufficient_decrease_fails<T>(F_lp, S.Fy, tk[0], tk[1], dt2 * curv, S.lipsch)) {
+        S.lipsch *= 2;  // backtracking, apgd.hpp:172-182
+        S.alpha = n.alpha_bt;
+        S.bt = 1;
+        ++S.nbt;
+        if (max_bt > 0 && S.nbt > max_bt) {  // alpha underflow guard
+            S.err = 2;
+            S.done = 1;
+        }
+        return;
+    }
+    ++S.ite;
+    S.bt = 0;
+    if (isfinite(S.lipsch)) S.lgood = S.lipsch;
+    S.last_step = n.step;
+    int tmp = S.ip; S.ip = S.il; S.il = S.in_; S.in_ = tmp;
+    tmp = S.jL; S.jL = S.jN; S.jN = tmp;
+    tmp = S.jY; S.jY = S.jYN; S.jYN = tmp;
+    if (n.step < n.tol) {
+        S.conv = 1;
+        S.done = 1;
+        return;
+    }
+    S.beta = S.beta_n;
+    S.theta = S.restart ? 1.0 : S.theta1;
+    if (S.restart) ++S.nrs;
+    if (dynamic) {
+        S.lipsch = n.lip_ok;
+        S.alpha = n.alpha_ok;
+    }
+    S.use_prev = (S.beta != 0.0) ? 1 : 0;
+    if (S.ite >= max_ite) S.done = 1;
+}
+__device__ __forceinline__ void write_result(ApgdResult* r, const ApgdState& S) {
+    r->iterations = S.ite;
+    r->backtracks = S.nbt;
+    r->restarts = S.nrs;
+    r->converged = S.conv;
+    r->lam_buf = S.il;
+    r->u_buf = S.jL;
+    r->error = S.err;
+    r->last_step = S.last_step;
+    r->lipsch = S.lgood;
 }
 
 }  // namespace apgdc

@@ -298,6 +298,42 @@ void launch_sph_residual64(int nin, int dim, int problem, const int2* cij, const
                            const dvec4* u, double* g, unsigned long long* viol, const Sizes* sizes, long long c_cap,
                            cudaStream_t s);
 
+// ---------------------------------------------------------- apgd_fric.cu
+// Friction: contact rows in planes, incidence records in walking order, multipliers and
+// velocities in 16-byte vectors; the result in the layouts of the other kernels.
+template <typename T>
+struct FricSolve {
+    long long cap;            // plane stride of rec (contacts)
+    int2* cij;
+    void* rec;                // cap * fric_rec_bytes
+    void* inc;                // 2 * cap * fric_inc_bytes
+    const double* shift;      // correction solves: solution offset (null = none)
+    const int* inc_ptr;
+    const T* invm;            // 4 per active body
+    V4<T>* lam[3];
+    V4<T>* u[4];              // fric_u_vectors(dim) per active body
+    T* lam_out;               // 3 per contact
+    T* u_out;                 // 6 per active body (null: not wanted)
+    double* sums;             // kSumBytesPerBlock per block, all ones at launch
+    unsigned int* barrier;
+    ApgdResult* result;
+};
+size_t fric_rec_bytes(int dim, bool fp32);
+size_t fric_inc_bytes(int dim, bool fp32);
+int fric_u_vectors(int dim);
+int apgd_fric_max_blocks();
+long long apgd_fric_launches();
+template <typename T>
+void launch_fric_pack(int dim, int na, const Contacts& c, const Assembly& a, const Incidence& inc, FricSolve<T>& f,
+                      const Sizes* sizes, cudaStream_t s);
+// another linear term (3 per contact) in rows already packed
+template <typename T>
+void launch_fric_pack_c(int dim, const double* cvec, FricSolve<T>& f, const Sizes* sizes, cudaStream_t s);
+// at most apgd_fric_max_blocks() blocks, one per 256 contacts or bodies
+template <typename T>
+cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, FricSolve<T>& f, const Sizes* sizes,
+                             int nblocks, cudaStream_t s);
+
 // --------------------------------------------------------- apgd_batch.cu
 struct BatchSceneStats {
     long long contacts;

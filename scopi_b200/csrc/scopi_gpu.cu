@@ -111,6 +111,14 @@ struct scopi_gpu_handle {
     float4* d_us32[4] = {nullptr, nullptr, nullptr, nullptr};
     dvec4* d_usfin = nullptr;
 
+    // Friction (apgd_fric.cu): rows, incidence records and iterates of the solve; the FP64 set of
+    // a mixed handle is allocated when its first FP64 correction runs
+    struct FricBuffers {
+        void *rec = nullptr, *inc = nullptr, *lam[3] = {}, *u[4] = {};
+    };
+    FricBuffers fb64{}, fb32{};
+    DevMem fric_mem;
+
     // fixed small buffers
     DevMem fixed_mem;
     double* d_partials = nullptr;
@@ -127,7 +135,7 @@ struct scopi_gpu_handle {
     int* d_census = nullptr;           // shape census of an upload (k_shape_census)
     int* h_census = nullptr;           // pinned copy
     bool stall_next = false;           // scopi_gpu_test_barrier_stall: withhold one arrival once
-    int max_blocks64 = 0, max_blocks32 = 0, max_sph64 = 0, max_sph32 = 0;
+    int max_fric = 0, max_blocks64 = 0, max_blocks32 = 0, max_sph64 = 0, max_sph32 = 0;
     // FrictionFixedPoint: P.problem holds FRICTION (the kernels' problem), this flag the loop
     // (ViscousFriction keeps its own problem code and runs the same loop)
     bool fixed_point = false;
@@ -158,6 +166,8 @@ struct scopi_gpu_handle {
     // multipliers in c (and the Jacobian kept as the three rows of A) per contact
     int cvec_per() const { return P.problem == SCOPI_GPU_VISCOUS_FRICTION ? 4 : (friction_rows() ? 3 : 1); }
     bool friction_rows() const { return P.problem == SCOPI_GPU_FRICTION || P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
+    // single scenes of the Friction problem (and FrictionFixedPoint): apgd_fric.cu
+    bool fric() const { return P.problem == SCOPI_GPU_FRICTION && !batch; }
     bool viscous_friction() const { return P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
     bool fp_loop() const { return fixed_point || viscous_friction(); }
     // the viscous problems carry each contact's gamma from the previous list by (i, j)
@@ -555,7 +565,8 @@ struct scopi_gpu_handle {
             max_sph64 = apgd_sph_max_blocks(P.problem, P.dim, false);
             max_sph32 = apgd_sph_max_blocks(P.problem, P.dim, true);
         }
-        const int mb = std::max({max_blocks64, max_blocks32, max_sph64, max_sph32, 1});
+        if (fric()) max_fric = apgd_fric_max_blocks();
+        const int mb = std::max({max_fric, max_blocks64, max_blocks32, max_sph64, max_sph32, 1});
         if ((e = alloc(fixed_mem, d_partials, 4 * (size_t)mb * 8)) != cudaSuccess) return cuda_fail(e, "alloc");
         sums_bytes = (size_t)kSumBytesPerBlock * mb;
         if ((e = alloc(fixed_mem, d_sums, sums_bytes / sizeof(double))) != cudaSuccess) return cuda_fail(e, "alloc");
@@ -642,6 +653,31 @@ struct scopi_gpu_handle {
         return 0;
     }
 
+    template <typename T>
+    int alloc_fric(DevMem& mem, FricBuffers& b) {
+        cudaError_t e;
+        const bool f32 = sizeof(T) == 4;
+        auto get = [&](void*& p, size_t bytes) {
+            unsigned char* q = nullptr;
+            e = alloc(mem, q, bytes);
+            p = q;
+            return e == cudaSuccess;
+        };
+        bool ok = get(b.rec, c_cap * fric_rec_bytes(P.dim, f32)) && get(b.inc, 2 * c_cap * fric_inc_bytes(P.dim, f32));
+        for (int k = 0; k < 3 && ok; ++k) ok = get(b.lam[k], c_cap * sizeof(V4<T>));
+        for (int k = 0; k < 4 && ok; ++k) ok = get(b.u[k], ((size_t)na + 1) * fric_u_vectors(P.dim) * sizeof(V4<T>));
+        if (!ok) b = FricBuffers{};
+        return ok ? 0 : cuda_fail(e, "cudaMalloc(friction rows)");
+    }
+
+    // the friction solve's buffers, whose sizes follow the contact capacity and the bodies
+    int alloc_fric_set() {
+        fric_mem.release();
+        fb64 = fb32 = FricBuffers{};
+        if (!fric()) return 0;
+        return mixed() ? alloc_fric<float>(fric_mem, fb32) : alloc_fric<double>(fric_mem, fb64);
+    }
+
     // Buffers whose size follows the contact capacity.
     int alloc_contacts(long long cap) {
         cap_mem.release();
@@ -668,10 +704,19 @@ struct scopi_gpu_handle {
         if (fp_loop()) {
             A(d_cvec_base, cvec_per() * cap) A(d_fp_s, cap)
         }
-        A(inc.idx, 2 * cap) A(inc.coef, 12 * cap)
-        for (int k = 0; k < 3; ++k) A(d_lam64[k], M)
-        A(d_g64, M) A(d_res64, M) A(d_lamacc, M)
-        if (mixed()) {
+        A(inc.idx, 2 * cap)
+        A(d_res64, M) A(d_lamacc, M)
+        if (fric()) {
+            A(d_lam64[0], M)
+            if (mixed()) A(d_lam32[0], M)
+            int rc = alloc_fric_set();
+            if (rc) return rc;
+        } else {
+            A(inc.coef, 12 * cap)
+            for (int k = 0; k < 3; ++k) A(d_lam64[k], M)
+            A(d_g64, M)
+        }
+        if (mixed() && !fric()) {
             A(d_bn32, 3 * cap) A(d_bai32, 3 * cap) A(d_baj32, 3 * cap)
             if (friction_rows()) A(d_bP32, 18 * cap)
             A(d_cvec32, cvec_per() * cap) A(d_coef32, 12 * cap)
@@ -695,7 +740,8 @@ struct scopi_gpu_handle {
     }
 
     long long launches() const {
-        return detect_launches() + apgd_launches() + apgd_sph_launches() + apgd_batch_launches() + se_launches() +
+        return detect_launches() + apgd_launches() + apgd_sph_launches() + apgd_batch_launches() + apgd_fric_launches() +
+               se_launches() +
                replayed;
     }
 
@@ -908,6 +954,56 @@ struct scopi_gpu_handle {
     }
 
     template <typename T>
+    int run_apgd_fric(FricSolve<T>& f, double dt, double tol, long long max_ite, double alpha0 = 0.0) {
+        ApgdSettings st{};
+        st.alpha = alpha0 > 0.0 ? alpha0 : P.alpha;
+        st.tol = tol;
+        st.max_ite = max_ite;
+        st.dynamic = P.dynamic_descent;
+        st.dt = dt;
+        st.mu = P.mu;
+        // a correction solve starts from the step size of the solve before it
+        st.curvature_start = alpha0 > 0.0 ? 0 : curvature_start();
+        const size_t ub = (size_t)na * fric_u_vectors(P.dim) * sizeof(V4<T>);
+        // lambda = lambda_prev = 0 and u(lambda) = u(y) = 0 (cold start, apgd.hpp:152-159)
+        cudaMemsetAsync(f.lam[0], 0, h_sizes->C * sizeof(V4<T>), stream);
+        cudaMemsetAsync(f.lam[1], 0, h_sizes->C * sizeof(V4<T>), stream);
+        cudaMemsetAsync(f.u[0], 0, ub, stream);
+        cudaMemsetAsync(f.u[2], 0, ub, stream);
+        cudaError_t e = reset_barrier(st);
+        if (e != cudaSuccess) return cuda_fail(e, "APGD barrier words");
+        const int nb = nblocks_for(max_fric, std::max<long long>(h_sizes->C, na));
+        cudaMemsetAsync(f.sums, 0xff, (size_t)kSumBytesPerBlock * nb, stream);
+        e = launch_apgd_fric<T>(nin, na, P.dim, st, f, d_sizes_cur, nb, stream);
+        if (e != cudaSuccess) return cuda_fail(e, "APGD launch");
+        cudaMemcpyAsync(h_result, d_result, sizeof(ApgdResult), cudaMemcpyDeviceToHost, stream);
+        e = cudaStreamSynchronize(stream);
+        if (e != cudaSuccess) return cuda_fail(e, "APGD");
+        if (h_result->error == 1) return fail(SCOPI_GPU_ETIMEOUT, "APGD grid barrier timed out");
+        h_result->lam_buf = h_result->u_buf = 0;  // the kernel copied them to lam_out and u_out
+        return 0;
+    }
+
+    template <typename T>
+    FricSolve<T> fric_buffers(const FricBuffers& b, const T* invm, T* lam_out, T* u_out) const {
+        FricSolve<T> f{};
+        f.cap = c_cap;
+        f.cij = d_cij;
+        f.rec = b.rec;
+        f.inc = b.inc;
+        f.inc_ptr = inc.ptr;
+        f.invm = invm;
+        for (int k = 0; k < 3; ++k) f.lam[k] = static_cast<V4<T>*>(b.lam[k]);
+        for (int k = 0; k < 4; ++k) f.u[k] = static_cast<V4<T>*>(b.u[k]);
+        f.lam_out = lam_out;
+        f.u_out = u_out;
+        f.sums = d_sums;
+        f.barrier = d_barrier;
+        f.result = d_result;
+        return f;
+    }
+
+    template <typename T>
     SphSolve<T> sph_buffers(const V4<T>* nc, const V4<T>* incv, const T* imt, T* const* lam, V4<T>* const* u) const {
         SphSolve<T> sb{};
         sb.cij = d_cij;
@@ -962,6 +1058,12 @@ struct scopi_gpu_handle {
                     rc = run_apgd_sph<double>(sb, max_sph64, dt, P.tolerance, P.max_ite, M);
                     if (rc) return rc;
                     ufin = reinterpret_cast<const double*>(d_us64[h_result->u_buf]);
+                } else if (fric()) {
+                    FricSolve<double> f = fric_buffers<double>(fb64, d_invm64, d_lam64[0], d_u64[0]);
+                    launch_fric_pack<double>(P.dim, na, cur, as, inc, f, d_sizes_cur, stream);
+                    rc = run_apgd_fric<double>(f, dt, P.tolerance, P.max_ite);
+                    if (rc) return rc;
+                    ufin = d_u64[0];
                 } else {
                     SolveBuffers<double> sb{};
                     sb.bn = as.bn;
@@ -1111,10 +1213,14 @@ struct scopi_gpu_handle {
         const int per = cvec_per();
         SphSolve<float> sbs{};
         SolveBuffers<float> sb{};
+        FricSolve<float> sf{};
         if (sphere_mode()) {
             launch_pack_nc<float>(as.bn, as.cvec, d_nc32, d_sizes_cur, c_cap, stream);
             launch_pack_inc<float>(na, inc.ptr, inc.idx, as.bn, d_incv32, 2 * c_cap, stream);
             sbs = sph_buffers<float>(d_nc32, d_incv32, d_imt32, d_lam32, d_us32);
+        } else if (fric()) {
+            sf = fric_buffers<float>(fb32, d_invm32, d_lam32[0], nullptr);
+            launch_fric_pack<float>(P.dim, na, cur, as, inc, sf, d_sizes_cur, stream);
         } else {
             launch_convert<double, float>(as.bn, d_bn32, 3 * c_cap, &d_sizes_cur->C, 3, stream);
             launch_convert<double, float>(as.bai, d_bai32, 3 * c_cap, &d_sizes_cur->C, 3, stream);
@@ -1150,6 +1256,7 @@ struct scopi_gpu_handle {
         auto solve32 = [&]() -> int {
             cudaEventRecord(ev_a[0], stream);
             int r = sphere_mode() ? run_apgd_sph<float>(sbs, max_sph32, dt, P.tolerance, P.max_ite, M, alpha0)
+                    : fric()      ? run_apgd_fric<float>(sf, dt, P.tolerance, P.max_ite, alpha0)
                                   : run_apgd<float>(sb, d_invm32, max_blocks32, dt, P.tolerance, P.max_ite, M, alpha0);
             cudaEventRecord(ev_a[1], stream);
             if (r) return r;
@@ -1173,6 +1280,17 @@ struct scopi_gpu_handle {
                 r = run_apgd_sph<double>(s64, max_sph64, dt, P.tolerance, P.max_ite, M, alpha0);
                 // the FP64 residual reads (n, c) from the same records
                 launch_pack_nc<double>(as.bn, as.cvec, d_nc64, d_sizes_cur, c_cap, stream);
+            } else if (fric()) {
+                if (!fb64.rec) {
+                    r = alloc_fric<double>(fric_mem, fb64);
+                    if (r) return r;
+                }
+                FricSolve<double> f = fric_buffers<double>(fb64, d_invm64, d_lam64[0], nullptr);
+                Assembly ar = as;
+                ar.cvec = d_res64;
+                f.shift = d_lamacc;
+                launch_fric_pack<double>(P.dim, na, cur, ar, inc, f, d_sizes_cur, stream);
+                r = run_apgd_fric<double>(f, dt, P.tolerance, P.max_ite, alpha0);
             } else {
                 SolveBuffers<double> s64{};
                 s64.bn = as.bn;
@@ -1236,6 +1354,9 @@ struct scopi_gpu_handle {
             if (sphere_mode()) {
                 launch_pack_nc<float>(as.bn, d_res64, d_nc32, d_sizes_cur, c_cap, stream);
                 sbs.shift = d_lamacc;
+            } else if (fric()) {
+                launch_fric_pack_c<float>(P.dim, d_res64, sf, d_sizes_cur, stream);
+                sf.shift = d_lamacc;
             } else {
                 launch_convert<double, float>(d_res64, d_cvec32, per * c_cap, &d_sizes_cur->C, per, stream);
                 sb.shift = d_lamacc;
@@ -1479,6 +1600,8 @@ static int32_t upload_particles(scopi_gpu_handle* h, const scopi_gpu_particles* 
             if (rc) return rc;
         } else {
             h->has_old = false;
+            rc = h->alloc_fric_set();
+            if (rc) return rc;
         }
     }
     cudaStream_t s = h->stream;
