@@ -28,17 +28,7 @@ namespace {
 using namespace apgdc;
 
 template <typename T>
-struct Q4_of;  // the 16-byte vector of T
-template <>
-struct Q4_of<float> {
-    using type = float4;
-};
-template <>
-struct Q4_of<double> {
-    using type = double2;
-};
-template <typename T>
-using Q4 = typename Q4_of<T>::type;
+using Q4 = Q16<T>;
 
 // values per contact row and per incidence record, and their 16-byte vectors.  Contact 3D:
 // P_i (9), P_j (9), n, c; 2D: P_i[6..7], P_j[6..7], n, c.  Incidence 3D: +-P (9), index (, pad);
@@ -100,7 +90,8 @@ struct FricArgs {
     const Q4<T>* rec;
     const double* shift;   // correction solves: 3 per contact (null = none)
     const int* inc_ptr;
-    const Q4<T>* inc;
+    const Q4<T>* inc;      // IncLayout
+    long long inc_slots;
     const V4<T>* invm;     // 1/m, 1/Jx, 1/Jy, 1/Jz (2D: 1/m, 0, 0, 1/Jz)
     V4<T>* lam0;
     V4<T>* lam1;
@@ -231,25 +222,26 @@ __device__ __forceinline__ void contact_row(const T* r, const T* ui, const T* uj
     if (DIM == 2) lout[2] = (T)0;
 }
 
-// w = A^T l+ of one body over its incidences [k0, k1), KB records and multipliers in flight
+// w = A^T l+ of one body over its n incidences, KB records and multipliers in flight
 template <typename T, int DIM, int KB>
-__device__ __forceinline__ void body_force(const Q4<T>* inc, const V4<T>* lnew, int k0, int k1, T* w) {
+__device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, const V4<T>* lnew, int n, T* w) {
     using F = FricShape<T, DIM>;
 #pragma unroll
     for (int d = 0; d < F::dof; ++d) w[d] = (T)0;
-    for (int kb = k0; kb < k1; kb += KB) {
+    for (int kb = 0; kb < n; kb += KB) {
         T e[KB][F::inc], l[KB][4];
 #pragma unroll
         for (int q = 0; q < KB; ++q)
-            if (kb + q < k1)
+            if (kb + q < n)
 #pragma unroll
-                for (int v = 0; v < F::ni; ++v) put4(e[q] + v * F::per, inc[(long long)(kb + q) * F::ni + v]);
+                for (int v = 0; v < F::ni; ++v)
+                    put4(e[q] + v * F::per, inc[wk.first + (long long)(kb + q) * wk.rs + v * wk.vs]);
 #pragma unroll
         for (int q = 0; q < KB; ++q)
-            if (kb + q < k1) fld4cg(lnew + (fidx(e[q][F::at_idx]) & 0x7fffffffu), l[q]);
+            if (kb + q < n) fld4cg(lnew + (fidx(e[q][F::at_idx]) & 0x7fffffffu), l[q]);
 #pragma unroll
         for (int q = 0; q < KB; ++q) {
-            if (kb + q >= k1) continue;
+            if (kb + q >= n) continue;
             const T* P = e[q];
             const T* f = l[q];
             const bool neg = (fidx(e[q][F::at_idx]) >> 31) != 0;
@@ -316,6 +308,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
     __shared__ double red[8][32];
     const int tid = threadIdx.x;
     const int C = A.sizes->C;
+    const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
     GridSums<false> G{A.sums, gridDim.x, A.bar, 0u, A.stall != 0 && blockIdx.x == 0};
     if (tid == 0) state_init(S, A.alpha);
     __syncthreads();
@@ -350,7 +343,8 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
         if (ok && tid < 256)
             for (long long p = b0; p < A.na; p += S0) {
                 T w[F::dof], u[F::dof], im[4];
-                body_force<T, DIM, KB>(A.inc, A.lam2, A.inc_ptr[p], A.inc_ptr[p + 1], w);
+                const int k0 = A.inc_ptr[p];
+                body_force<T, DIM, KB>(A.inc, inc_walk(lay, F::ni, p, k0), A.lam2, A.inc_ptr[p + 1] - k0, w);
                 fld4(A.invm + p, im);
                 body_velocity<T, DIM>(im, w, u);
                 b[0] += body_wu<T, DIM>(w, u);
@@ -430,7 +424,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
                 fld4(A.invm + p, im);
                 if (bn_ != (T)0) load_u<T, DIM>(uL, p, ul);
                 if (sizeof(T) == 4) load_u<T, DIM>(uY, p, uy);
-                body_force<T, DIM, KB>(A.inc, lnew, k0, k1, w);
+                body_force<T, DIM, KB>(A.inc, inc_walk(lay, F::ni, p, k0), lnew, k1 - k0, w);
                 body_velocity<T, DIM>(im, w, u);
                 store_u<T, DIM>(uN, p, u);
                 // w.u gives F(l+) for the reference's test (FP64); FP32 tests the curvature
@@ -530,31 +524,48 @@ __global__ void k_fric_pack_c(const Sizes* sizes, long long cap, const double* c
     }
 }
 template <typename T, int DIM>
-__global__ void k_fric_pack_inc(int na, const int* ptr, const int* idx, const double* bP, Q4<T>* inc) {
+__device__ __forceinline__ void store_inc(unsigned e, const double* bP, Q4<T>* inc, long long at, int vs) {
     using F = FricShape<T, DIM>;
-    const long long tot = ptr[na];
-    GRID_STRIDE(k, tot) {
-        const unsigned e = (unsigned)idx[k];
-        const long long c = e & 0x7fffffffu;
-        const int side = (int)(e >> 31);
-        const double* P = bP + 18 * c + 9 * side;
-        const T sg = side == 0 ? (T)1 : (T)-1;
-        T r[F::inc];
-        for (int q = 0; q < F::inc; ++q) r[q] = (T)0;
-        if (DIM == 3) {
-            for (int q = 0; q < 9; ++q) r[q] = sg * (T)P[q];
-        } else {
-            r[0] = sg * (T)P[6];
-            r[1] = sg * (T)P[7];
-        }
-        r[F::at_idx] = fidx_bits<T>(e);
-        for (int v = 0; v < F::ni; ++v) {
-            Q4<T> q;
-            T* o = reinterpret_cast<T*>(&q);
-            for (int j = 0; j < F::per; ++j) o[j] = r[v * F::per + j];
-            inc[k * F::ni + v] = q;
-        }
+    const long long c = e & 0x7fffffffu;
+    const int side = (int)(e >> 31);
+    const double* P = bP + 18 * c + 9 * side;
+    const T sg = side == 0 ? (T)1 : (T)-1;
+    T r[F::inc];
+    for (int q = 0; q < F::inc; ++q) r[q] = (T)0;
+    if (DIM == 3) {
+        for (int q = 0; q < 9; ++q) r[q] = sg * (T)P[q];
+    } else {
+        r[0] = sg * (T)P[6];
+        r[1] = sg * (T)P[7];
     }
+    r[F::at_idx] = fidx_bits<T>(e);
+#pragma unroll
+    for (int v = 0; v < F::ni; ++v) {
+        Q4<T> q;
+        T* o = reinterpret_cast<T*>(&q);
+        for (int j = 0; j < F::per; ++j) o[j] = r[v * F::per + j];
+        inc[at + v * vs] = q;
+    }
+}
+template <typename T, int DIM>
+__global__ void k_fric_pack_inc(int na, const int* ptr, const int* idx, const double* bP, Q4<T>* inc, long long slots,
+                                const Sizes* sizes) {
+    using F = FricShape<T, DIM>;
+    const IncLayout lay = inc_layout(sizes, na, slots);
+    if (lay.width) {
+        const long long tot = (long long)lay.width * 32 * ((na + 31) / 32);
+        GRID_STRIDE(t, tot) {
+            const long long row = t >> 5, g = row / lay.width, p = g * 32 + (t & 31);
+            const int r = (int)(row - g * lay.width);
+            if (p >= na) continue;
+            const int k0 = ptr[p];
+            if (r < ptr[p + 1] - k0)
+                store_inc<T, DIM>((unsigned)idx[k0 + r], bP, inc, row * F::ni * 32 + (t & 31), 32);
+        }
+        return;
+    }
+    const long long tot = ptr[na];
+    GRID_STRIDE(k, tot) store_inc<T, DIM>((unsigned)idx[k], bP, inc, k * F::ni, 1);
 }
 
 int blocks(long long n) {
@@ -597,10 +608,12 @@ void launch_fric_pack(int dim, int na, const Contacts& c, const Assembly& a, con
     Q4<T>* iv = static_cast<Q4<T>*>(f.inc);
     if (dim == 3) {
         k_fric_pack<T, 3><<<blocks(f.cap), 256, 0, s>>>(sizes, f.cap, c.ci, c.cj, a.bP, a.bn, a.cvec, f.cij, rec);
-        k_fric_pack_inc<T, 3><<<blocks(2 * f.cap), 256, 0, s>>>(na, inc.ptr, inc.idx, a.bP, iv);
+        k_fric_pack_inc<T, 3><<<blocks(f.inc_slots), 256, 0, s>>>(na, inc.ptr, inc.idx, a.bP, iv, f.inc_slots,
+                                                                     sizes);
     } else {
         k_fric_pack<T, 2><<<blocks(f.cap), 256, 0, s>>>(sizes, f.cap, c.ci, c.cj, a.bP, a.bn, a.cvec, f.cij, rec);
-        k_fric_pack_inc<T, 2><<<blocks(2 * f.cap), 256, 0, s>>>(na, inc.ptr, inc.idx, a.bP, iv);
+        k_fric_pack_inc<T, 2><<<blocks(f.inc_slots), 256, 0, s>>>(na, inc.ptr, inc.idx, a.bP, iv, f.inc_slots,
+                                                                     sizes);
     }
     g_fric_launches += 2;
 }
@@ -625,6 +638,7 @@ cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, F
     A.shift = f.shift;
     A.inc_ptr = f.inc_ptr;
     A.inc = static_cast<const Q4<T>*>(f.inc);
+    A.inc_slots = f.inc_slots;
     A.invm = reinterpret_cast<const V4<T>*>(f.invm);
     A.lam0 = f.lam[0];
     A.lam1 = f.lam[1];

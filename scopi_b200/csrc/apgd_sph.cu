@@ -44,6 +44,13 @@ __device__ __forceinline__ void st4(dvec4* p, double x, double y, double z) {
     q[0] = make_double2(x, y);
     q[1] = make_double2(z, 0.0);
 }
+// incidence record r of a body: (+-n, contact index)
+__device__ __forceinline__ float4 ld_inc(const float4* inc, const IncWalk& w, int r) { return inc[w.first + (long long)r * w.rs]; }
+__device__ __forceinline__ dvec4 ld_inc(const double2* inc, const IncWalk& w, int r) {
+    const double2* q = inc + w.first + (long long)r * w.rs;
+    const double2 a = q[0], b = q[w.vs];
+    return dvec4{a.x, a.y, b.x, b.y};
+}
 __device__ __forceinline__ int idx_of(float w) { return __float_as_int(w); }
 __device__ __forceinline__ int idx_of(double w) { return (int)__double_as_longlong(w); }
 
@@ -85,7 +92,8 @@ struct SphArgs {
     const int* slot;
     const double* shift;
     const int* inc_ptr;
-    const V4<T>* inc;
+    const Q16<T>* inc;
+    long long inc_slots;
     const T* invm;  // 1/m per active body, contiguous
     T* lam0;
     T* lam1;
@@ -214,6 +222,7 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
     if (threadIdx.x == 0) state_init(S, A.alpha);
     __syncthreads();
     const int C = A.sizes->C;
+    const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
     GridSums<true> G{A.sums, gridDim.x, A.bar, 0u, A.stall != 0 && blockIdx.x == 0};
     // Trip k of a thread handles item base + k*S (the grid-stride order) in both passes.
     const long long S_ = (long long)gridDim.x * NT, base = (long long)blockIdx.x * NT + tid;
@@ -268,8 +277,10 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
         double wm[2] = {0.0, 0.0};
         if (ok) GRID_STRIDE(p, A.na) {
             T w0 = 0, w1 = 0, w2 = 0;
-            for (int k = A.inc_ptr[p]; k < A.inc_ptr[p + 1]; ++k) {
-                const V4<T> e = ld4(A.inc + k);
+            const int k0 = A.inc_ptr[p], n = A.inc_ptr[p + 1] - k0;
+            const IncWalk wk = inc_walk(lay, sizeof(T) / 4, p, k0);
+            for (int k = 0; k < n; ++k) {
+                const V4<T> e = ld_inc(A.inc, wk, k);
                 const int ci = idx_of(e.w);
                 T mu = __ldcg(dbuf + ci);
                 if (PROB == kViscous) {
@@ -437,8 +448,9 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
                 if (p >= A.na) continue;
                 const int sl = (int)(kt % GP) * NT + tid;
                 T w0 = 0, w1 = 0, w2 = 0;
-                const int k0 = s_p0[sl], k1 = s_p1[sl];
-                for (int kb = k0; kb < k1; kb += KB) {
+                const int k0 = s_p0[sl], k1 = s_p1[sl] - k0;
+                const IncWalk wk = inc_walk(lay, sizeof(T) / 4, p, k0);
+                for (int kb = 0; kb < k1; kb += KB) {
                     T ex[KB], ey[KB], ez[KB], mu[KB];
                     int ci[KB];
 #pragma unroll
@@ -446,7 +458,7 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
                         ex[q] = ey[q] = ez[q] = mu[q] = (T)0;
                         ci[q] = -1;
                         if (kb + q < k1) {
-                            const V4<T> e = ld4(A.inc + kb + q);
+                            const V4<T> e = ld_inc(A.inc, wk, kb + q);
                             ex[q] = e.x;
                             ey[q] = e.y;
                             ez[q] = e.z;
@@ -543,32 +555,57 @@ __device__ __forceinline__ float idx_bits<float>(int c) { return __int_as_float(
 template <>
 __device__ __forceinline__ double idx_bits<double>(int c) { return __longlong_as_double((long long)c); }
 
-// cap: the records `inc` holds; a list longer than that is cut (the no-allocation entry
+template <typename T>
+__device__ __forceinline__ void st_inc(Q16<T>* inc, long long at, int vs, double sg, const double* n, int c);
+template <>
+__device__ __forceinline__ void st_inc<float>(float4* inc, long long at, int, double sg, const double* n, int c) {
+    inc[at] = make_float4((float)(sg * n[0]), (float)(sg * n[1]), (float)(sg * n[2]), idx_bits<float>(c));
+}
+template <>
+__device__ __forceinline__ void st_inc<double>(double2* inc, long long at, int vs, double sg, const double* n, int c) {
+    inc[at] = make_double2(sg * n[0], sg * n[1]);
+    inc[at + vs] = make_double2(sg * n[2], idx_bits<double>(c));
+}
+// slots: the records `inc` holds; a list longer than that is cut (the no-allocation entry
 // point rejects such lists before this runs; the engine sizes `inc` for every list)
 template <typename T>
-__global__ void k_pack_inc(int na, const int* ptr, const int* idx, const double* bn, V4<T>* inc, long long cap) {
-    const long long tot = ptr[na] < cap ? (long long)ptr[na] : cap;
+__global__ void k_pack_inc(int na, const int* ptr, const int* idx, const double* bn, Q16<T>* inc, long long slots,
+                           const Sizes* sizes) {
+    constexpr int nv = sizeof(T) / 4;
+    const IncLayout lay = inc_layout(sizes, na, slots);
+    if (lay.width) {
+        const long long tot = (long long)lay.width * 32 * ((na + 31) / 32);
+        GRID_STRIDE(t, tot) {
+            const long long row = t >> 5, g = row / lay.width, p = g * 32 + (t & 31);
+            const int r = (int)(row - g * lay.width);
+            if (p >= na) continue;
+            const int k0 = ptr[p];
+            if (r >= ptr[p + 1] - k0) continue;
+            const unsigned e = (unsigned)idx[k0 + r];
+            const int c = (int)(e & 0x7fffffffu);
+            st_inc<T>(inc, row * nv * 32 + (t & 31), 32, (e >> 31) ? -1.0 : 1.0, bn + 3 * (long long)c, c);
+        }
+        return;
+    }
+    const long long tot = ptr[na] < slots ? (long long)ptr[na] : slots;
     GRID_STRIDE(k, tot) {
         const unsigned e = (unsigned)idx[k];
         const int c = (int)(e & 0x7fffffffu);
-        const double sg = (e >> 31) ? -1.0 : 1.0;
-        V4<T> r;
-        r.x = (T)(sg * bn[3 * (long long)c]);
-        r.y = (T)(sg * bn[3 * (long long)c + 1]);
-        r.z = (T)(sg * bn[3 * (long long)c + 2]);
-        r.w = idx_bits<T>(c);
-        inc[k] = r;
+        st_inc<T>(inc, k * nv, 1, (e >> 31) ? -1.0 : 1.0, bn + 3 * (long long)c, c);
     }
 }
 
 // ------------------------------------------------------------------ FP64 helpers (mixed form)
 template <int DIM, int PROB>
-__global__ void k_sph_particle64(int na, const int* ptr, const dvec4* inc, const int* slot, const double* invm,
-                                 const double* lam, dvec4* u) {
+__global__ void k_sph_particle64(int na, const int* ptr, const double2* inc, long long slots, const Sizes* sizes,
+                                 const int* slot, const double* invm, const double* lam, dvec4* u) {
+    const IncLayout lay = inc_layout(sizes, na, slots);
     GRID_STRIDE(p, na) {
         double w0 = 0, w1 = 0, w2 = 0;
-        for (int k = ptr[p]; k < ptr[p + 1]; ++k) {
-            const dvec4 e = ld4(inc + k);
+        const int k0 = ptr[p], n = ptr[p + 1] - k0;
+        const IncWalk wk = inc_walk(lay, 2, p, k0);
+        for (int k = 0; k < n; ++k) {
+            const dvec4 e = ld_inc(inc, wk, k);
             const int c = idx_of(e.w);
             double mu = lam[c];
             if (PROB == kViscous && slot[c] >= 0) mu -= lam[slot[c]];
@@ -678,6 +715,7 @@ cudaError_t launch_apgd_sph(int nin, int na, int dim, int problem, const ApgdSet
     A.shift = sb.shift;
     A.inc_ptr = sb.inc_ptr;
     A.inc = sb.inc;
+    A.inc_slots = sb.inc_slots;
     A.invm = sb.invm;
     A.lam0 = sb.lam[0];
     A.lam1 = sb.lam[1];
@@ -721,20 +759,23 @@ void launch_pack_nc(const double* bn, const double* cvec, V4<T>* nc, const Sizes
 template void launch_pack_nc<double>(const double*, const double*, dvec4*, const Sizes*, long long, cudaStream_t);
 template void launch_pack_nc<float>(const double*, const double*, float4*, const Sizes*, long long, cudaStream_t);
 template <typename T>
-void launch_pack_inc(int na, const int* ptr, const int* idx, const double* bn, V4<T>* inc, long long inc_cap,
-                     cudaStream_t s) {
+void launch_pack_inc(int na, const int* ptr, const int* idx, const double* bn, Q16<T>* inc, long long slots,
+                     const Sizes* sizes, cudaStream_t s) {
     if (na <= 0) return;
-    k_pack_inc<T><<<blocks(inc_cap), 256, 0, s>>>(na, ptr, idx, bn, inc, inc_cap);
+    k_pack_inc<T><<<blocks(slots), 256, 0, s>>>(na, ptr, idx, bn, inc, slots, sizes);
     g_sph_launches += 1;
 }
-template void launch_pack_inc<double>(int, const int*, const int*, const double*, dvec4*, long long, cudaStream_t);
-template void launch_pack_inc<float>(int, const int*, const int*, const double*, float4*, long long, cudaStream_t);
+template void launch_pack_inc<double>(int, const int*, const int*, const double*, double2*, long long, const Sizes*,
+                                      cudaStream_t);
+template void launch_pack_inc<float>(int, const int*, const int*, const double*, float4*, long long, const Sizes*,
+                                     cudaStream_t);
 
-void launch_sph_particle64(int na, int dim, int problem, const int* ptr, const dvec4* inc, const int* slot,
-                           const double* invm, const double* lam, dvec4* u, cudaStream_t s) {
+void launch_sph_particle64(int na, int dim, int problem, const int* ptr, const double2* inc, long long slots,
+                           const Sizes* sizes, const int* slot, const double* invm, const double* lam, dvec4* u,
+                           cudaStream_t s) {
     if (na <= 0) return;
 #define PP(D, P) \
-    if (dim == D && problem == P) k_sph_particle64<D, P><<<blocks(na), 256, 0, s>>>(na, ptr, inc, slot, invm, lam, u);
+    if (dim == D && problem == P) k_sph_particle64<D, P><<<blocks(na), 256, 0, s>>>(na, ptr, inc, slots, sizes, slot, invm, lam, u);
     PP(2, 0) PP(2, 2) PP(3, 0) PP(3, 2)
 #undef PP
     g_sph_launches += 1;
@@ -843,6 +884,7 @@ __global__ void k_noalloc_prepare(Sizes* sizes, int C, int na, const double* inv
         sizes->C_obs = 0;
         sizes->n_extra = 0;
         sizes->overflow = 0;
+        sizes->inc_width = 0;  // rows one after the other: the fixed array has no room for columns
     }
     GRID_STRIDE(p, na) { invm[p] = inv_mass[p]; }
 }
@@ -923,7 +965,7 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
     const int C = (int)n_contacts, na = (int)n_active;
     int2* cij = reinterpret_cast<int2*>(base + kOffCij);
     dvec4* nc = reinterpret_cast<dvec4*>(base + kOffNc);
-    dvec4* inc = reinterpret_cast<dvec4*>(base + kOffInc);
+    double2* inc = reinterpret_cast<double2*>(base + kOffInc);
     double* invm = reinterpret_cast<double*>(base + kOffInvm);
     double* lam = reinterpret_cast<double*>(base + kOffLam);
     dvec4* ub = reinterpret_cast<dvec4*>(base + kOffU);
@@ -979,7 +1021,7 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
     k_noalloc_prepare<<<blocks(na), 256, 0, s>>>(sizes, C, na, inv_mass, invm);
     launch_pack_cij(ci, cj, cij, sizes, C, s);
     k_noalloc_pack_nc<<<blocks(C), 256, 0, s>>>(normal, c, nc, C);
-    launch_pack_inc<double>(na, inc_ptr, inc_idx, normal, inc, 2 * (long long)C, s);
+    launch_pack_inc<double>(na, inc_ptr, inc_idx, normal, inc, 2 * (long long)C, sizes, s);
     SphArgs<double> A;
     A.nin = (int)nb_inactive;
     A.na = na;
@@ -989,6 +1031,7 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
     A.shift = nullptr;
     A.inc_ptr = inc_ptr;
     A.inc = inc;
+    A.inc_slots = 2 * (long long)C;
     A.invm = invm;
     A.lam0 = lam;
     A.lam1 = lam + kNoAllocMaxContacts;

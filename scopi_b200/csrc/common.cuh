@@ -48,7 +48,8 @@ struct Sizes {
     int overflow;       // capacity exceeded somewhere (host grows and redoes the step)
     int ncell;          // cells of the uniform grid
     int n_links;        // worm links: the last n_links contacts (normal and distance negated)
-    int pad[2];
+    int inc_width;      // most incidences of one body (columns of the incidence layout)
+    int pad[1];
 };
 
 struct Grid {

@@ -938,9 +938,12 @@ __global__ void k_inc_fill(int nin, Contacts c, const Sizes* sizes, const int* p
 }
 
 // sort each particle's incidences by contact index: a deterministic summation order for B^T x
-__global__ void k_inc_sort(int na, const int* ptr, int* idx) {
+// (and the longest list, the width of the packed incidence records, where width is given)
+__global__ void k_inc_sort(int na, const int* ptr, int* idx, int* width) {
+    int most = 0;
     GRID_STRIDE(p, na) {
         const int s = ptr[p], e = ptr[p + 1];
+        most = max(most, e - s);
         for (int x = s + 1; x < e; ++x) {
             const int key = idx[x];
             const unsigned kk = (unsigned)key & 0x7fffffffu;
@@ -952,6 +955,9 @@ __global__ void k_inc_sort(int na, const int* ptr, int* idx) {
             idx[y + 1] = key;
         }
     }
+    if (!width) return;
+    most = __reduce_max_sync(0xffffffffu, most);
+    if ((threadIdx.x & 31) == 0 && most > 0) atomicMax(width, most);
 }
 
 __global__ void k_inc_coef(int na, const int* ptr, const int* idx, Assembly a, double* coef) {
@@ -1395,7 +1401,7 @@ void launch_assemble(const Bodies& b, const StepParams& p, const Contacts& c, As
 }
 
 void launch_incidence(const Bodies& b, const StepParams& p, const Contacts& c, const Assembly& a, Incidence& inc,
-                      const Sizes* sizes, long long c_cap, int* scan_work, int* tmp_total, cudaStream_t s,
+                      Sizes* sizes, long long c_cap, int* scan_work, int* tmp_total, cudaStream_t s,
                       bool with_coef) {
     const int na = b.n - b.nin;
     if (na <= 0) return;
@@ -1404,7 +1410,8 @@ void launch_incidence(const Bodies& b, const StepParams& p, const Contacts& c, c
     k_inc_count<<<blocks_for(c_cap), kThreads, 0, s>>>(b.nin, c, sizes, inc.count);
     scan_exclusive(inc.count, inc.ptr, nullptr, na + 1, na + 1, tmp_total, scan_work, s, &g_detect_launches);
     k_inc_fill<<<blocks_for(c_cap), kThreads, 0, s>>>(b.nin, c, sizes, inc.ptr, inc.jcount, inc.idx);
-    k_inc_sort<<<blocks_for(na), kThreads, 0, s>>>(na, inc.ptr, inc.idx);
+    // a batch keeps its records in rows
+    k_inc_sort<<<blocks_for(na), kThreads, 0, s>>>(na, inc.ptr, inc.idx, b.scene ? nullptr : &sizes->inc_width);
     LAUNCHED(3);
     if (with_coef && p.problem != kFriction && p.problem != kViscousFriction) {
         k_inc_coef<<<blocks_for(2 * c_cap), kThreads, 0, s>>>(na, inc.ptr, inc.idx, a, inc.coef);

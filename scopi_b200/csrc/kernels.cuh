@@ -90,7 +90,7 @@ void launch_assemble(const Bodies& b, const StepParams& p, const Contacts& c, As
 // with_coef: also the 6 FP64 coefficients per incidence (inc.coef) that the 6-dof
 // normal-row kernels read; the torque-free kernels pack their own records instead
 void launch_incidence(const Bodies& b, const StepParams& p, const Contacts& c, const Assembly& a, Incidence& inc,
-                      const Sizes* sizes, long long c_cap, int* scan_work, int* tmp_total, cudaStream_t s,
+                      Sizes* sizes, long long c_cap, int* scan_work, int* tmp_total, cudaStream_t s,
                       bool with_coef);
 // Worm links (compute_contacts, solver.hpp:358-367): contacts (links[k], links[k] + 1) appended
 // at C..C+W-1 after the sorted list (C on the host, the list's count), sizes->C = C + W and
@@ -259,6 +259,45 @@ struct V4_of<double> {
 };
 template <typename T>
 using V4 = typename V4_of<T>::type;
+template <typename T>
+struct Q16_of;  // the 16-byte vector of T
+template <>
+struct Q16_of<float> {
+    using type = float4;
+};
+template <>
+struct Q16_of<double> {
+    using type = double2;
+};
+template <typename T>
+using Q16 = typename Q16_of<T>::type;
+
+// Packed incidence records (nv 16-byte vectors each).  Columns: the bodies in groups of 32, record
+// r of a group's 32 bodies side by side, vector by vector, so that a warp that walks 32 bodies
+// loads 512 contiguous bytes per vector; every group has the width of the longest list
+// (Sizes::inc_width).  Rows one after the other as in ptr/idx touch 32 cache lines per load
+// instead; they are kept for lists so uneven that the columns would not fit in `slots` records
+// (one body with very many contacts), and in batches, whose scenes keep their records in the L1
+// of their SM between iterations (256 pile scenes, 1024 threads, FP64: columns 5-10 % slower).
+// Columns against rows, microseconds per APGD iteration: FP64 133k contacts 16.0 -> 13.9, 4.6M
+// 188.6 -> 175; FP32 451k 16.8 -> 16.0, 4.6M 108.4 -> 100.8; FP64 friction 44k 18.3 -> 16.4.
+constexpr long long kIncSlotsPerContact = 4;  // two incidences a contact, lists up to twice the mean
+struct IncLayout {
+    int width;  // 0: rows one after the other
+};
+__host__ __device__ inline IncLayout inc_layout(const Sizes* sizes, int na, long long slots) {
+    const long long w = sizes->inc_width, groups = ((long long)na + 31) / 32;
+    return IncLayout{w * 32 * groups <= slots ? (int)w : 0};
+}
+// vector v of record r of body p (its list starts at k0) is at first + r * rs + v * vs
+struct IncWalk {
+    long long first;
+    int rs, vs;
+};
+__host__ __device__ inline IncWalk inc_walk(IncLayout l, int nv, long long p, int k0) {
+    if (l.width) return IncWalk{(p >> 5) * l.width * nv * 32 + (p & 31), 32 * nv, 32};
+    return IncWalk{(long long)k0 * nv, nv, 1};
+}
 
 // grid sums of a persistent launch: 4 slots of 8 doubles per block (apgd_common.cuh)
 constexpr int kSumBytesPerBlock = 4 * 8 * 8;
@@ -270,7 +309,8 @@ struct SphSolve {
     const int* slot;
     const double* shift;
     const int* inc_ptr;
-    const V4<T>* inc;
+    const Q16<T>* inc;        // +-n, contact index (IncLayout, one vector in FP32, two in FP64)
+    long long inc_slots;
     const T* invm;            // 1/m per active body, contiguous
     T* lam[3];
     V4<T>* u[4];
@@ -290,10 +330,11 @@ template <typename T>
 void launch_pack_nc(const double* bn, const double* cvec, V4<T>* nc, const Sizes* sizes, long long c_cap,
                     cudaStream_t s);
 template <typename T>
-void launch_pack_inc(int na, const int* ptr, const int* idx, const double* bn, V4<T>* inc, long long inc_cap,
-                     cudaStream_t s);
-void launch_sph_particle64(int na, int dim, int problem, const int* ptr, const dvec4* inc, const int* slot,
-                           const double* invm, const double* lam, dvec4* u, cudaStream_t s);
+void launch_pack_inc(int na, const int* ptr, const int* idx, const double* bn, Q16<T>* inc, long long slots,
+                     const Sizes* sizes, cudaStream_t s);
+void launch_sph_particle64(int na, int dim, int problem, const int* ptr, const double2* inc, long long slots,
+                           const Sizes* sizes, const int* slot, const double* invm, const double* lam, dvec4* u,
+                           cudaStream_t s);
 void launch_sph_residual64(int nin, int dim, int problem, const int2* cij, const dvec4* nc, const int* slot, double dt2,
                            const dvec4* u, double* g, unsigned long long* viol, const Sizes* sizes, long long c_cap,
                            cudaStream_t s);
@@ -306,7 +347,8 @@ struct FricSolve {
     long long cap;            // plane stride of rec (contacts)
     int2* cij;
     void* rec;                // cap * fric_rec_bytes
-    void* inc;                // 2 * cap * fric_inc_bytes
+    void* inc;                // inc_slots * fric_inc_bytes
+    long long inc_slots;
     const double* shift;      // correction solves: solution offset (null = none)
     const int* inc_ptr;
     const T* invm;            // 4 per active body
@@ -356,7 +398,7 @@ struct BatchSolve {
     V4<T>* nc;
     const dvec4* nc64;
     const int* inc_ptr;
-    const V4<T>* inc;
+    const V4<T>* inc;         // rows one after the other
     const dvec4* inc64;
     const double* invm;
     T* lam[3];

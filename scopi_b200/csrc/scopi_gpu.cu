@@ -105,7 +105,7 @@ struct scopi_gpu_handle {
     int2* d_cij = nullptr;
     dvec4* d_nc64 = nullptr;
     float4* d_nc32 = nullptr;
-    dvec4* d_incv64 = nullptr;
+    double2* d_incv64 = nullptr;
     float4* d_incv32 = nullptr;
     dvec4* d_us64[4] = {nullptr, nullptr, nullptr, nullptr};
     float4* d_us32[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -168,6 +168,7 @@ struct scopi_gpu_handle {
     bool friction_rows() const { return P.problem == SCOPI_GPU_FRICTION || P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
     // single scenes of the Friction problem (and FrictionFixedPoint): apgd_fric.cu
     bool fric() const { return P.problem == SCOPI_GPU_FRICTION && !batch; }
+    long long inc_slots() const { return kIncSlotsPerContact * c_cap; }
     bool viscous_friction() const { return P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
     bool fp_loop() const { return fixed_point || viscous_friction(); }
     // the viscous problems carry each contact's gamma from the previous list by (i, j)
@@ -292,10 +293,10 @@ struct scopi_gpu_handle {
         }
         launch_pack_cij(cur.ci, cur.cj, d_cij, d_sizes_cur, c_cap, stream);
         launch_pack_nc<double>(as.bn, as.cvec, d_nc64, d_sizes_cur, c_cap, stream);
-        launch_pack_inc<double>(na, inc.ptr, inc.idx, as.bn, d_incv64, 2 * c_cap, stream);
+        launch_pack_inc<double>(na, inc.ptr, inc.idx, as.bn, d_incv64, inc_slots(), d_sizes_cur, stream);
         if (mixed()) {
             launch_pack_nc<float>(as.bn, as.cvec, d_nc32, d_sizes_cur, c_cap, stream);
-            launch_pack_inc<float>(na, inc.ptr, inc.idx, as.bn, d_incv32, 2 * c_cap, stream);
+            launch_pack_inc<float>(na, inc.ptr, inc.idx, as.bn, d_incv32, inc_slots(), d_sizes_cur, stream);
         }
         launch_batch_ranges(n_scenes, nin, d_sc_obs0, d_sc_obs1, d_sc_p0, d_sc_p1, d_obs_off, dw.obs_pos, dw.row_ptr,
                             d_sizes_cur, d_sc_o0, d_sc_o1, d_sc_a0, d_sc_a1, stream);
@@ -362,7 +363,7 @@ struct scopi_gpu_handle {
             bs.cij = d_cij;
             bs.nc64 = d_nc64;
             bs.inc_ptr = inc.ptr;
-            bs.inc64 = d_incv64;
+            bs.inc64 = reinterpret_cast<const dvec4*>(d_incv64);
             bs.invm = d_invm64;
             bs.lam64 = d_lamacc;
             bs.ufin = d_usfin;
@@ -389,7 +390,7 @@ struct scopi_gpu_handle {
             BatchSolve<double> bs{};
             fill(bs);
             bs.nc = d_nc64;
-            bs.inc = d_incv64;
+            bs.inc = reinterpret_cast<const dvec4*>(d_incv64);
             for (int k = 0; k < 3; ++k) bs.lam[k] = d_lam64[k];
             for (int k = 0; k < 4; ++k) bs.u[k] = d_us64[k];
             launch_apgd_batch<double>(P.dim, bt, tile, bs, n_scenes, stream);
@@ -663,7 +664,7 @@ struct scopi_gpu_handle {
             p = q;
             return e == cudaSuccess;
         };
-        bool ok = get(b.rec, c_cap * fric_rec_bytes(P.dim, f32)) && get(b.inc, 2 * c_cap * fric_inc_bytes(P.dim, f32));
+        bool ok = get(b.rec, c_cap * fric_rec_bytes(P.dim, f32)) && get(b.inc, inc_slots() * fric_inc_bytes(P.dim, f32));
         for (int k = 0; k < 3 && ok; ++k) ok = get(b.lam[k], c_cap * sizeof(V4<T>));
         for (int k = 0; k < 4 && ok; ++k) ok = get(b.u[k], ((size_t)na + 1) * fric_u_vectors(P.dim) * sizeof(V4<T>));
         if (!ok) b = FricBuffers{};
@@ -723,9 +724,9 @@ struct scopi_gpu_handle {
             for (int k = 0; k < 3; ++k) A(d_lam32[k], M)
             A(d_g32, M)
         }
-        A(d_cij, cap) A(d_nc64, cap) A(d_incv64, 2 * cap) A(d_se_keep, cap + 1) A(d_se_pos, cap + 1) A(d_se_u, 4 * cap + 4)
+        A(d_cij, cap) A(d_nc64, cap) A(d_incv64, 2 * inc_slots()) A(d_se_keep, cap + 1) A(d_se_pos, cap + 1) A(d_se_u, 4 * cap + 4)
         if (mixed()) {
-            A(d_nc32, cap) A(d_incv32, 2 * cap)
+            A(d_nc32, cap) A(d_incv32, inc_slots())
         }
 #undef A
         cudaMemsetAsync(d_sizes_cur, 0, sizeof(Sizes), stream);
@@ -991,6 +992,7 @@ struct scopi_gpu_handle {
         f.cij = d_cij;
         f.rec = b.rec;
         f.inc = b.inc;
+        f.inc_slots = inc_slots();
         f.inc_ptr = inc.ptr;
         f.invm = invm;
         for (int k = 0; k < 3; ++k) f.lam[k] = static_cast<V4<T>*>(b.lam[k]);
@@ -1004,7 +1006,7 @@ struct scopi_gpu_handle {
     }
 
     template <typename T>
-    SphSolve<T> sph_buffers(const V4<T>* nc, const V4<T>* incv, const T* imt, T* const* lam, V4<T>* const* u) const {
+    SphSolve<T> sph_buffers(const V4<T>* nc, const Q16<T>* incv, const T* imt, T* const* lam, V4<T>* const* u) const {
         SphSolve<T> sb{};
         sb.cij = d_cij;
         sb.nc = nc;
@@ -1012,6 +1014,7 @@ struct scopi_gpu_handle {
         sb.shift = nullptr;
         sb.inc_ptr = inc.ptr;
         sb.inc = incv;
+        sb.inc_slots = inc_slots();
         sb.invm = imt;
         for (int k = 0; k < 3; ++k) sb.lam[k] = lam[k];
         for (int k = 0; k < 4; ++k) sb.u[k] = u[k];
@@ -1045,7 +1048,7 @@ struct scopi_gpu_handle {
             if (sphere_mode()) {
                 launch_pack_cij(cur.ci, cur.cj, d_cij, d_sizes_cur, c_cap, stream);
                 launch_pack_nc<double>(as.bn, as.cvec, d_nc64, d_sizes_cur, c_cap, stream);
-                launch_pack_inc<double>(na, inc.ptr, inc.idx, as.bn, d_incv64, 2 * c_cap, stream);
+                launch_pack_inc<double>(na, inc.ptr, inc.idx, as.bn, d_incv64, inc_slots(), d_sizes_cur, stream);
                 ustride = 4;
                 urot = 0;
             }
@@ -1216,7 +1219,7 @@ struct scopi_gpu_handle {
         FricSolve<float> sf{};
         if (sphere_mode()) {
             launch_pack_nc<float>(as.bn, as.cvec, d_nc32, d_sizes_cur, c_cap, stream);
-            launch_pack_inc<float>(na, inc.ptr, inc.idx, as.bn, d_incv32, 2 * c_cap, stream);
+            launch_pack_inc<float>(na, inc.ptr, inc.idx, as.bn, d_incv32, inc_slots(), d_sizes_cur, stream);
             sbs = sph_buffers<float>(d_nc32, d_incv32, d_imt32, d_lam32, d_us32);
         } else if (fric()) {
             sf = fric_buffers<float>(fb32, d_invm32, d_lam32[0], nullptr);
@@ -1330,8 +1333,8 @@ struct scopi_gpu_handle {
         for (int k = 0;; ++k) {
             cudaMemsetAsync(d_viol, 0, sizeof(unsigned long long), stream);
             if (sphere_mode()) {
-                launch_sph_particle64(na, P.dim, P.problem, inc.ptr, d_incv64, as.slot, d_invm64, d_lamacc, d_usfin,
-                                      stream);
+                launch_sph_particle64(na, P.dim, P.problem, inc.ptr, d_incv64, inc_slots(), d_sizes_cur, as.slot,
+                                      d_invm64, d_lamacc, d_usfin, stream);
                 launch_sph_residual64(nin, P.dim, P.problem, d_cij, d_nc64, as.slot, dt * dt, d_usfin, d_res64, d_viol,
                                       d_sizes_cur, c_cap, stream);
             } else {
