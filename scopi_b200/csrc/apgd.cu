@@ -262,7 +262,7 @@ __device__ __forceinline__ void contact_one(const ApgdArgs<T>& A, long long c, c
                                             double* s) {
     {
         const int i = A.ci[c], j = A.cj[c];
-        if (PROB != kFriction && PROB != kViscousFriction) {
+        if constexpr (PROB != kViscousFriction) {
             T qy = 0;
             if (!bt) {
                 T n[3];
@@ -299,7 +299,7 @@ __device__ __forceinline__ void contact_one(const ApgdArgs<T>& A, long long c, c
                 if (sl >= 0) contact_scalar<T, DIM, PROB>(A, sl, -qy, -cc, lam, lprev, lnew, beta, use_prev, bt, alpha, s);
             }
         } else {
-            // friction rows: A_c u = v_i + P_i^T w_i - v_j - P_j^T w_j (three per contact)
+            // A_c u = v_i + P_i^T w_i - v_j - P_j^T w_j
             T qy[3] = {0, 0, 0};
             if (!bt) {
                 for (int side = 0; side < 2; ++side) {
@@ -317,79 +317,41 @@ __device__ __forceinline__ void contact_one(const ApgdArgs<T>& A, long long c, c
                 }
                 for (int d = 0; d < 3; ++d) qy[d] *= (T)A.dt2;
             }
-            if constexpr (PROB == kViscousFriction) {
-                // four slots: g = global2local(Q y) + c, then the mode's projection
-                const int md = A.mode[c];
-                T nt[3] = {A.bn[3 * c], A.bn[3 * c + 1], A.bn[3 * c + 2]};
-                T ql[4];
-                vf_local<T, DIM>(md, qy, nt, ql);
-                double y[4], gm[4], lm[4], z[4], nd[3];
-                for (int k = 0; k < 4; ++k) {
-                    const long long m = 4 * c + k;
-                    lm[k] = (double)lam[m];
-                    y[k] = use_prev ? (double)(lam[m] + beta * (lam[m] - lprev[m])) : lm[k];
-                    if (bt) {
-                        gm[k] = (double)A.g[m];
-                    } else {
-                        const T gg = ql[k] + A.cvec[m];
-                        A.g[m] = gg;
-                        gm[k] = (double)gg;
-                    }
-                    z[k] = y[k] - alpha * gm[k];
-                    if (A.shift) z[k] += A.shift[m];
+            // four slots: g = global2local(Q y) + c, then the mode's projection
+            const int md = A.mode[c];
+            T nt[3] = {A.bn[3 * c], A.bn[3 * c + 1], A.bn[3 * c + 2]};
+            T ql[4];
+            vf_local<T, DIM>(md, qy, nt, ql);
+            double y[4], gm[4], lm[4], z[4], nd[3];
+            for (int k = 0; k < 4; ++k) {
+                const long long m = 4 * c + k;
+                lm[k] = (double)lam[m];
+                y[k] = use_prev ? (double)(lam[m] + beta * (lam[m] - lprev[m])) : lm[k];
+                if (bt) {
+                    gm[k] = (double)A.g[m];
+                } else {
+                    const T gg = ql[k] + A.cvec[m];
+                    A.g[m] = gg;
+                    gm[k] = (double)gg;
                 }
-                for (int d = 0; d < 3; ++d) nd[d] = (double)nt[d];
-                vf_project<DIM>(md, z, nd, A.mu);
-                for (int k = 0; k < 4; ++k) {
-                    const long long m = 4 * c + k;
-                    const T lp = (T)(A.shift ? z[k] - A.shift[m] : z[k]);
-                    lnew[m] = lp;
-                    const double dly = (double)lp - y[k], dll = (double)lp - lm[k];
-                    const double cc = (double)A.cvec[m];
-                    s[0] += gm[k] * dly;
-                    s[1] += dly * dly;
-                    s[2] += cc * (double)lp;
-                    if (!bt) s[3] += y[k] * (0.5 * (double)ql[k] + cc);
-                    s[4] += dll * dll;
-                    s[5] += gm[k] * dll;
-                    s[7] += (double)lp * (double)lp;
-                }
-            } else {
-                double y[3], gm[3], lm[3];
-                for (int d = 0; d < 3; ++d) {
-                    const long long m = 3 * c + d;
-                    lm[d] = (double)lam[m];
-                    y[d] = use_prev ? (double)(lam[m] + beta * (lam[m] - lprev[m])) : lm[d];
-                    if (bt) {
-                        gm[d] = (double)A.g[m];
-                    } else {
-                        const T gg = qy[d] + A.cvec[m];
-                        A.g[m] = gg;
-                        gm[d] = (double)gg;
-                    }
-                }
-                double z[3], n[3];
-                for (int d = 0; d < 3; ++d) {
-                    n[d] = (double)A.bn[3 * c + d];
-                    z[d] = y[d] - alpha * gm[d];
-                    if (A.shift) z[d] += A.shift[3 * c + d];
-                }
-                if (DIM == 2) z[2] = A.shift ? A.shift[3 * c + 2] : 0.0;
-                cone_project<DIM>(z, n, A.mu);
-                for (int d = 0; d < 3; ++d) {
-                    const long long m = 3 * c + d;
-                    const T lp = (T)(A.shift ? z[d] - A.shift[m] : z[d]);
-                    lnew[m] = lp;
-                    const double dly = (double)lp - y[d], dll = (double)lp - lm[d];
-                    const double cc = (double)A.cvec[m];
-                    s[0] += gm[d] * dly;
-                    s[1] += dly * dly;
-                    s[2] += cc * (double)lp;
-                    if (!bt) s[3] += y[d] * (0.5 * (double)qy[d] + cc);
-                    s[4] += dll * dll;
-                    s[5] += gm[d] * dll;
-                    s[7] += (double)lp * (double)lp;
-                }
+                z[k] = y[k] - alpha * gm[k];
+                if (A.shift) z[k] += A.shift[m];
+            }
+            for (int d = 0; d < 3; ++d) nd[d] = (double)nt[d];
+            vf_project<DIM>(md, z, nd, A.mu);
+            for (int k = 0; k < 4; ++k) {
+                const long long m = 4 * c + k;
+                const T lp = (T)(A.shift ? z[k] - A.shift[m] : z[k]);
+                lnew[m] = lp;
+                const double dly = (double)lp - y[k], dll = (double)lp - lm[k];
+                const double cc = (double)A.cvec[m];
+                s[0] += gm[k] * dly;
+                s[1] += dly * dly;
+                s[2] += cc * (double)lp;
+                if (!bt) s[3] += y[k] * (0.5 * (double)ql[k] + cc);
+                s[4] += dll * dll;
+                s[5] += gm[k] * dll;
+                s[7] += (double)lp * (double)lp;
             }
         }
     }
@@ -413,7 +375,7 @@ __device__ __forceinline__ void particle_one(const ApgdArgs<T>& A, long long p, 
         for (int k = k0; k < k1; ++k) {
             const unsigned e = (unsigned)A.inc_idx[k];
             const long long c = e & 0x7fffffffu;
-            if (PROB != kFriction && PROB != kViscousFriction) {
+            if (PROB != kViscousFriction) {
                 T mu = __ldcg(lnew + c);
                 if (PROB == kViscous) {
                     const int sl = A.slot[c];
@@ -427,16 +389,10 @@ __device__ __forceinline__ void particle_one(const ApgdArgs<T>& A, long long p, 
                 const int side = (int)(e >> 31);
                 const T sg = side == 0 ? (T)1 : (T)-1;
                 T f[3];
-                if (PROB == kViscousFriction) {
-                    const T l4[4] = {__ldcg(lnew + 4 * c), __ldcg(lnew + 4 * c + 1), __ldcg(lnew + 4 * c + 2),
-                                     __ldcg(lnew + 4 * c + 3)};
-                    const T nt[3] = {A.bn[3 * c], A.bn[3 * c + 1], A.bn[3 * c + 2]};
-                    vf_force<T, DIM>(A.mode[c], l4, nt, f);
-                } else {
-                    f[0] = __ldcg(lnew + 3 * c);
-                    f[1] = __ldcg(lnew + 3 * c + 1);
-                    f[2] = __ldcg(lnew + 3 * c + 2);
-                }
+                const T l4[4] = {__ldcg(lnew + 4 * c), __ldcg(lnew + 4 * c + 1), __ldcg(lnew + 4 * c + 2),
+                                 __ldcg(lnew + 4 * c + 3)};
+                const T nt[3] = {A.bn[3 * c], A.bn[3 * c + 1], A.bn[3 * c + 2]};
+                vf_force<T, DIM>(A.mode[c], l4, nt, f);
                 const T* P = A.bP + 18 * c + 9 * side;
                 for (int d = 0; d < 3; ++d) {
                     w[d] += sg * f[d];
@@ -635,7 +591,7 @@ __global__ void __launch_bounds__(kApgdThreads) k_apgd(ApgdArgs<T> A) {
     }
 }
 
-// ------------------------------------------------- batched scenes, 6-dof rows (FP64)
+// ------------------------------------------------- batched Viscous scenes, 6-dof rows (FP64)
 // One CTA per scene (scenes taken largest first): the iteration of k_apgd on the scene's
 // contacts (its obstacle rows [o0, o1), then its active rows [a0, a1)) and bodies [p0, p1),
 // with block barriers and block sums in place of the grid ones, so every scene iterates
@@ -660,7 +616,6 @@ __device__ __forceinline__ double block_max(double v) {
 template <int DIM, int PROB>
 __global__ void __launch_bounds__(kBatch6Threads) k_apgd_batch6(ApgdArgs<double> A, Batch6Scenes S) {
     using T = double;
-    constexpr int R = PROB == kFriction ? 3 : 1;  // multipliers per contact
     T* lamb[3] = {A.lam0, A.lam1, A.lam2};
     T* ub[3] = {A.u0, A.u1, A.u2};
     for (int q = blockIdx.x; q < S.n_scenes; q += gridDim.x) {
@@ -681,29 +636,15 @@ __global__ void __launch_bounds__(kBatch6Threads) k_apgd_batch6(ApgdArgs<double>
             double s[kPartials] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
             for (int k = threadIdx.x; k < nc; k += blockDim.x) {
                 const long long c = contact_at(k);
-                if (PROB == kFriction) {
-                    double z[3], n[3];
-                    for (int d = 0; d < 3; ++d) {
-                        n[d] = A.bn[3 * c + d];
-                        z[d] = -A.cvec[3 * c + d];
-                    }
-                    if (DIM == 2) z[2] = 0.0;
-                    cone_project<DIM>(z, n, A.mu);
-                    for (int d = 0; d < 3; ++d) {
-                        dbuf[3 * c + d] = z[d];
-                        s[1] += z[d] * z[d];
-                    }
-                } else {
-                    const T v = apgdc::first_descent<T>(A.cvec[c], nullptr, c);
-                    dbuf[c] = v;
-                    s[1] += v * v;
-                    if (PROB == kViscous) {
-                        const int sl = A.slot[c];
-                        if (sl >= 0) {
-                            const T v2 = apgdc::first_descent<T>(-A.cvec[c], nullptr, sl);
-                            dbuf[sl] = v2;
-                            s[1] += v2 * v2;
-                        }
+                const T v = apgdc::first_descent<T>(A.cvec[c], nullptr, c);
+                dbuf[c] = v;
+                s[1] += v * v;
+                if (PROB == kViscous) {
+                    const int sl = A.slot[c];
+                    if (sl >= 0) {
+                        const T v2 = apgdc::first_descent<T>(-A.cvec[c], nullptr, sl);
+                        dbuf[sl] = v2;
+                        s[1] += v2 * v2;
                     }
                 }
             }
@@ -782,35 +723,22 @@ __global__ void __launch_bounds__(kBatch6Threads) k_apgd_batch6(ApgdArgs<double>
         double vmax = 0.0;
         for (int k = threadIdx.x; k < nc; k += blockDim.x) {
             const long long c = contact_at(k);
-            for (int r = 0; r < R; ++r) S.lam_out[R * c + r] = lamb[il][R * c + r];
+            S.lam_out[c] = lamb[il][c];
             if (PROB == kViscous) {
                 const int sl = A.slot[c];
                 if (sl >= 0) S.lam_out[sl] = lamb[il][sl];
             }
             const int bi[2] = {A.ci[c], A.cj[c]};
-            double q3[3] = {0, 0, 0};
+            double q = 0.0;
             for (int side = 0; side < 2; ++side) {
                 if (bi[side] < A.nin) continue;
                 const T* uu = ub[jl] + 6 * (long long)(bi[side] - A.nin);
                 const double sg = side == 0 ? 1.0 : -1.0;
-                if (PROB == kFriction) {
-                    const T* P = A.bP + 18 * c + 9 * side;
-                    for (int d = 0; d < 3; ++d) {
-                        const double vd = (DIM == 2 && d == 2) ? 0.0 : uu[d];
-                        q3[d] += sg * (vd + P[d] * uu[3] + P[3 + d] * uu[4] + P[6 + d] * uu[5]);
-                    }
-                } else {
-                    const T* a = (side == 0 ? A.bai : A.baj) + 3 * c;
-                    for (int d = 0; d < DIM; ++d) q3[0] += sg * A.bn[3 * c + d] * uu[d];
-                    q3[0] += DIM == 3 ? a[0] * uu[3] + a[1] * uu[4] + a[2] * uu[5] : a[2] * uu[5];
-                }
+                const T* a = (side == 0 ? A.bai : A.baj) + 3 * c;
+                for (int d = 0; d < DIM; ++d) q += sg * A.bn[3 * c + d] * uu[d];
+                q += DIM == 3 ? a[0] * uu[3] + a[1] * uu[4] + a[2] * uu[5] : a[2] * uu[5];
             }
-            double gap = 0.0;
-            if (PROB == kFriction) {
-                for (int d = 0; d < DIM; ++d) gap += (A.dt2 * q3[d] + A.cvec[3 * c + d]) * A.bn[3 * c + d];
-            } else {
-                gap = A.dt2 * q3[0] + A.cvec[c];
-            }
+            const double gap = A.dt2 * q + A.cvec[c];
             vmax = fmax(vmax, -gap);
         }
         for (int p = p0 + threadIdx.x; p < p1; p += blockDim.x)
@@ -1131,12 +1059,7 @@ cudaError_t launch_apgd_batch6(const Bodies& b, const StepParams& p, const ApgdS
     A.max_ite = st.max_ite;
     A.dynamic = st.dynamic;
     const int grid = std::max(1, S.n_scenes);
-    if (p.problem == kFriction) {
-        if (p.dim == 3)
-            k_apgd_batch6<3, kFriction><<<grid, kBatch6Threads, 0, s>>>(A, S);
-        else
-            k_apgd_batch6<2, kFriction><<<grid, kBatch6Threads, 0, s>>>(A, S);
-    } else if (p.problem == kViscous) {
+    if (p.problem == kViscous) {
         if (p.dim == 3)
             k_apgd_batch6<3, kViscous><<<grid, kBatch6Threads, 0, s>>>(A, S);
         else

@@ -15,6 +15,8 @@
 // served this problem before (rows and gathers in 4- and 8-byte loads, two gathers per body,
 // 148 blocks of 256 threads, counter barriers), microseconds per iteration: 3D FP32 679k contacts
 // 164 -> 66, FP64 44k 34.2 -> 18.3; 2D FP64 1.7k 22.9 -> 9.3.  The iterates are the same bits.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "apgd_common.cuh"
@@ -45,6 +47,22 @@ struct FricShape {
     static constexpr int dof = DIM == 3 ? 6 : 3;
 };
 
+// multipliers of a contact: three values in 3D (padded to a vector), two in 2D
+template <typename T, int DIM>
+struct Lam_of {
+    using type = V4<T>;
+};
+template <>
+struct Lam_of<float, 2> {
+    using type = float2;
+};
+template <>
+struct Lam_of<double, 2> {
+    using type = double2;
+};
+template <typename T, int DIM>
+using Lam = typename Lam_of<T, DIM>::type;
+
 __device__ __forceinline__ void put4(float* o, const float4& v) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
 __device__ __forceinline__ void put4(double* o, const double2& v) { o[0] = v.x; o[1] = v.y; }
 __device__ __forceinline__ void fld4(const float4* p, float* o) { put4(o, *p); }
@@ -65,6 +83,12 @@ __device__ __forceinline__ void fst4(dvec4* p, const double* v) {
     q[0] = make_double2(v[0], v[1]);
     q[1] = make_double2(v[2], 0.0);
 }
+__device__ __forceinline__ void fld4(const float2* p, float* o) { const float2 v = *p; o[0] = v.x; o[1] = v.y; }
+__device__ __forceinline__ void fld4(const double2* p, double* o) { put4(o, *p); }
+__device__ __forceinline__ void fld4cg(const float2* p, float* o) { const float2 v = __ldcg(p); o[0] = v.x; o[1] = v.y; }
+__device__ __forceinline__ void fld4cg(const double2* p, double* o) { put4(o, __ldcg(p)); }
+__device__ __forceinline__ void fst4(float2* p, const float* v) { *p = make_float2(v[0], v[1]); }
+__device__ __forceinline__ void fst4(double2* p, const double* v) { *p = make_double2(v[0], v[1]); }
 // roundings written out where the compiler could contract in more than one way: a solve's
 // bits are then the same whatever kernel it runs in
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
@@ -93,13 +117,13 @@ struct FricArgs {
     const Q4<T>* inc;      // IncLayout
     long long inc_slots;
     const V4<T>* invm;     // 1/m, 1/Jx, 1/Jy, 1/Jz (2D: 1/m, 0, 0, 1/Jz)
-    V4<T>* lam0;
-    V4<T>* lam1;
-    V4<T>* lam2;
+    void* lam[3];          // Lam<T, DIM> per contact
     V4<T>* u0;
     V4<T>* u1;
     V4<T>* u2;
     V4<T>* u3;
+    void* qv;              // batches: dt^2 A u(y), Lam<T, DIM> per contact
+    double* wu;            // batches: w.u per body
     T* lam_out;            // 3 per contact
     T* u_out;              // 6 per body (null: not wanted)
     double* sums;
@@ -111,9 +135,9 @@ struct FricArgs {
     int dynamic, curvature_start, stall;
 };
 
-template <typename T>
-__device__ __forceinline__ V4<T>* pick_lam(const FricArgs<T>& A, int k) {
-    return k == 0 ? A.lam0 : (k == 1 ? A.lam1 : A.lam2);
+template <typename T, int DIM>
+__device__ __forceinline__ Lam<T, DIM>* pick_lam(const FricArgs<T>& A, int k) {
+    return static_cast<Lam<T, DIM>*>(k == 0 ? A.lam[0] : (k == 1 ? A.lam[1] : A.lam[2]));
 }
 template <typename T>
 __device__ __forceinline__ V4<T>* pick_u(const FricArgs<T>& A, int k) {
@@ -125,6 +149,17 @@ __device__ __forceinline__ void load_row(const Q4<T>* rec, long long cap, long l
     using F = FricShape<T, DIM>;
 #pragma unroll
     for (int v = 0; v < F::nv; ++v) put4(r + v * F::per, rec[v * cap + c]);
+}
+// the linear term of contact c alone
+template <typename T, int DIM>
+__device__ __forceinline__ void load_c(const Q4<T>* rec, long long cap, long long c, T* o) {
+    using F = FricShape<T, DIM>;
+    const T* r = reinterpret_cast<const T*>(rec);
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+        const int e = F::at_c + d;
+        o[d] = r[((e / F::per) * cap + c) * F::per + e % F::per];
+    }
 }
 // u of a body, written by other blocks: (v, w), 2D (vx, vy, w)
 template <typename T, int DIM>
@@ -180,10 +215,11 @@ __device__ __forceinline__ void point_velocity(const T* P, const T* u, T* o) {
 // One contact of the contact pass: its row r, u(y) of its bodies, l and l_prev; writes l+ and
 // adds its terms to s (FP64 g.d, |d|^2, c.l+, F(y), |l+ - l|^2, g.(l+ - l), |l+|^2; FP32
 // |d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2).
-template <typename T, int DIM>
+// SUMS false: s is left alone and dt^2 A u(y) goes to qout.
+template <typename T, int DIM, bool SUMS = true>
 __device__ __forceinline__ void contact_row(const T* r, const T* ui, const T* uj, const T* lam, const T* lprev,
                                             T beta, bool use_prev, bool bt, double alpha, double mu, T dt2,
-                                            const double* shift, T* lout, double* s) {
+                                            const double* shift, T* lout, double* s, T* qout = nullptr) {
     using F = FricShape<T, DIM>;
     T a[DIM], b[DIM];
     point_velocity<T, DIM>(r, ui, a);
@@ -207,6 +243,10 @@ __device__ __forceinline__ void contact_row(const T* r, const T* ui, const T* uj
     for (int d = 0; d < DIM; ++d) {
         const T lp = (T)(shift ? z[d] - shift[d] : z[d]);
         lout[d] = lp;
+        if (!SUMS) {
+            qout[d] = qy[d];
+            continue;
+        }
         const double dly = (double)lp - y[d], dll = (double)lp - (double)lam[d];
         if (!f32) {
             const double cc = (double)r[F::at_c + d];
@@ -220,11 +260,13 @@ __device__ __forceinline__ void contact_row(const T* r, const T* ui, const T* uj
         s[f32 ? 3 : 6] += (double)lp * (double)lp;
     }
     if (DIM == 2) lout[2] = (T)0;
+    if (DIM == 2 && !SUMS) qout[2] = (T)0;
 }
 
 // w = A^T l+ of one body over its n incidences, KB records and multipliers in flight
-template <typename T, int DIM, int KB>
-__device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, const V4<T>* lnew, int n, T* w) {
+// (CG: the multipliers come from other blocks, past the L1)
+template <typename T, int DIM, int KB, bool CG = true>
+__device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, const Lam<T, DIM>* lnew, int n, T* w) {
     using F = FricShape<T, DIM>;
 #pragma unroll
     for (int d = 0; d < F::dof; ++d) w[d] = (T)0;
@@ -238,7 +280,13 @@ __device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, 
                     put4(e[q] + v * F::per, inc[wk.first + (long long)(kb + q) * wk.rs + v * wk.vs]);
 #pragma unroll
         for (int q = 0; q < KB; ++q)
-            if (kb + q < n) fld4cg(lnew + (fidx(e[q][F::at_idx]) & 0x7fffffffu), l[q]);
+            if (kb + q < n) {
+                const Lam<T, DIM>* at = lnew + (fidx(e[q][F::at_idx]) & 0x7fffffffu);
+                if (CG)
+                    fld4cg(at, l[q]);
+                else
+                    fld4(at, l[q]);
+            }
 #pragma unroll
         for (int q = 0; q < KB; ++q) {
             if (kb + q >= n) continue;
@@ -317,6 +365,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
         // cold start (in the candidate buffer, which the first contact pass overwrites), with
         // 256 threads per block: the sums set the step, so their order is kept in FP32 too
         const long long S0 = (long long)gridDim.x * 256, b0 = (long long)blockIdx.x * 256 + tid;
+        Lam<T, DIM>* dbuf = pick_lam<T, DIM>(A, 2);
         double a[2] = {0.0, 0.0};
         if (tid < 256)
             for (long long c = b0; c < C; c += S0) {
@@ -334,7 +383,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
                     v[d] = (T)(z[d] - (A.shift ? A.shift[3 * c + d] : 0.0));
                     a[0] += (double)v[d] * (double)v[d];
                 }
-                fst4(A.lam2 + c, v);
+                fst4(dbuf + c, v);
             }
         double t1 = 0.0, t6 = 0.0;
         block_sum<2>(a);
@@ -344,7 +393,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
             for (long long p = b0; p < A.na; p += S0) {
                 T w[F::dof], u[F::dof], im[4];
                 const int k0 = A.inc_ptr[p];
-                body_force<T, DIM, KB>(A.inc, inc_walk(lay, F::ni, p, k0), A.lam2, A.inc_ptr[p + 1] - k0, w);
+                body_force<T, DIM, KB>(A.inc, inc_walk(lay, F::ni, p, k0), dbuf, A.inc_ptr[p + 1] - k0, w);
                 fld4(A.invm + p, im);
                 body_velocity<T, DIM>(im, w, u);
                 b[0] += body_wu<T, DIM>(w, u);
@@ -370,9 +419,9 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
         const double alpha = S.alpha;
         const bool bt = S.bt != 0, use_prev = S.use_prev != 0;
         const T beta = (T)S.beta;
-        const V4<T>* lam = pick_lam(A, S.il);
-        const V4<T>* lprev = pick_lam(A, S.ip);
-        V4<T>* lnew = pick_lam(A, S.in_);
+        const Lam<T, DIM>* lam = pick_lam<T, DIM>(A, S.il);
+        const Lam<T, DIM>* lprev = pick_lam<T, DIM>(A, S.ip);
+        Lam<T, DIM>* lnew = pick_lam<T, DIM>(A, S.in_);
         const V4<T>* uY = pick_u(A, S.jY);
         {
             double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
@@ -457,12 +506,12 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
         }
     }
     // the result, in the layouts of the other kernels (every thread its own contacts and bodies)
-    const V4<T>* lres = pick_lam(A, S.il);
+    const Lam<T, DIM>* lres = pick_lam<T, DIM>(A, S.il);
     const V4<T>* ures = pick_u(A, S.jL);
     for (long long c = base; c < C; c += S_) {
         T l[4];
         fld4(lres + c, l);
-        for (int d = 0; d < 3; ++d) A.lam_out[3 * c + d] = l[d];
+        for (int d = 0; d < 3; ++d) A.lam_out[3 * c + d] = d < DIM ? l[d] : (T)0;
     }
     if (A.u_out)
         for (long long p = base; p < A.na; p += S_) {
@@ -479,6 +528,343 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
             }
         }
     if (blockIdx.x == 0 && tid == 0) write_result(A.result, S);
+}
+
+// ------------------------------------------------------------------ batched scenes (FP64)
+// One CTA per scene, or a cluster of CS CTAs for a large one: the same iteration on the scene's
+// contacts (its obstacle rows [o0, o1), then its active rows [a0, a1)) and bodies [p0, p1), so
+// every scene iterates until its own stopping test holds; the multipliers, the velocities and
+// the scene's statistics with the violation max(0, -gap) of its final state go to fixed outputs.
+//
+// What bounds it: a scene's iteration is a chain of dependent FP64 work (square root and
+// divisions of the cone projection, ~150 instructions a contact) on very few SMs.  The passes
+// therefore run on all threads of the CTAs, whatever their number, and the sums are a pass of
+// their own: the scene's decisions are taken from sums over 256 chains (chain t adds contacts
+// t, t + 256, ... one after the other), whose bits do not depend on how the passes are split.
+// A contact leaves dt^2 A u(y) behind for it, a body w.u; the multipliers are there anyway.
+// The particle pass does not wait for the sums: it forms u(next y) with the momentum of an
+// accepted step, and after a restart u(l+) itself is the next y.  96 2D scenes of 200 to 2000
+// disks, milliseconds a step: the generic 6-dof rows on 256 threads 69.4; packed rows on 256
+// threads with two contacts at a time 23.1; this form, clusters of two for the largest, 15.5.
+constexpr int kChains = 256;
+template <int DIM>
+constexpr int kBatchFricThreads = DIM == 2 ? 512 : 256;  // 128 registers hold a 2D row, 255 a 3D one
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+template <int CS>
+__device__ __forceinline__ void scene_sync() {
+    if (CS == 1)
+        __syncthreads();
+    else
+        cluster_sync();
+}
+
+// Sums of a scene's chains: each warp's tree goes to every CTA of the scene (sh[value][warp of
+// chains]); after scene_sync, warps in order.
+struct SceneSums {
+    double w[8][kChains / 32];  // contact sums
+    double b[kChains / 32];     // w.u
+    double vmax[8];             // one per CTA
+    Momentum mo;                // of this iteration, and the steps after it
+    NextStep next;
+};
+template <int CS>
+__device__ __forceinline__ void share(double* at, double v) {
+    if (CS == 1) {
+        *at = v;
+    } else {
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        for (int r = 0; r < CS; ++r) *cl.map_shared_rank(at, r) = v;
+    }
+}
+
+template <int DIM, int CS>
+__device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, int sc, int rank, ApgdState& S,
+                           SceneSums& Q) {
+    using T = double;
+    using F = FricShape<T, DIM>;
+    using L = Lam<T, DIM>;
+    constexpr int NT = CS * kBatchFricThreads<DIM>, BT = kBatchFricThreads<DIM>;
+    constexpr int VT = kChains / CS;           // chains of this CTA: [rank * VT, rank * VT + VT)
+    constexpr int SPLIT = BT / VT >= 2 ? 2 : 1;  // threads per chain: the sums shared between two
+    const int lt = threadIdx.x, tid = rank * BT + lt;
+    const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
+    const int o0 = B.sc_o0[sc], n0 = B.sc_o1[sc] - o0, a0 = B.sc_a0[sc];
+    const int nc = n0 + (B.sc_a1[sc] - a0);
+    const int p0 = B.sc_p0[sc], p1 = B.sc_p1[sc];
+    L* qv = static_cast<L*>(A.qv);
+    auto contact_at = [&](int k) -> int { return k < n0 ? o0 + k : a0 + (k - n0); };
+    if (lt == 0) {
+        state_init(S, A.alpha);
+        if (nc == 0) S.done = S.conv = 1;
+    }
+    // lambda = lambda_prev = 0 and u(lambda) = u(y) = 0 (cold start, apgd.hpp:152-159)
+    const T zero[6] = {0, 0, 0, 0, 0, 0};
+    for (int k = tid; k < nc; k += NT) {
+        const int c = contact_at(k);
+        fst4(pick_lam<T, DIM>(A, 0) + c, zero);
+        fst4(pick_lam<T, DIM>(A, 1) + c, zero);
+    }
+    for (int p = p0 + tid; p < p1; p += NT) {
+        store_u<T, DIM>(A.u0, p, zero);
+        store_u<T, DIM>(A.u2, p, zero);
+    }
+    scene_sync<CS>();
+    if (nc > 0 && A.curvature_start) {
+        // L = 1.5 dt^2 |B^T d|^2_{M^-1} / |d|^2 along the first projected-gradient direction
+        L* dbuf = pick_lam<T, DIM>(A, 2);
+        for (int k = tid; k < nc; k += NT) {
+            const int c = contact_at(k);
+            T r[F::row];
+            load_row<T, DIM>(A.rec, A.cap, c, r);
+            double z[3], n[3];
+            n[2] = z[2] = 0.0;
+            for (int d = 0; d < DIM; ++d) {
+                n[d] = r[F::at_n + d];
+                z[d] = -r[F::at_c + d];
+            }
+            cone_project<DIM>(z, n, A.mu);
+            fst4(dbuf + c, z);
+        }
+        scene_sync<CS>();
+        for (int p = p0 + tid; p < p1; p += NT) {
+            T w[F::dof], u[F::dof], im[4];
+            const int k0 = A.inc_ptr[p];
+            body_force<T, DIM, 3>(A.inc, inc_walk(lay, F::ni, p, k0), dbuf, A.inc_ptr[p + 1] - k0, w);
+            fld4(A.invm + p, im);
+            body_velocity<T, DIM>(im, w, u);
+            A.wu[p] = body_wu<T, DIM>(w, u);
+        }
+        scene_sync<CS>();
+        double s[2] = {0.0, 0.0};
+        if (lt < VT) {
+            const int vt = rank * VT + lt;
+            for (int k = vt; k < nc; k += kChains) {
+                T z[4];
+                fld4cg(dbuf + contact_at(k), z);
+                for (int d = 0; d < DIM; ++d) s[0] += z[d] * z[d];
+            }
+            for (int p = p0 + vt; p < p1; p += kChains) s[1] += __ldcg(A.wu + p);
+            const double x0 = multi_reduce<1>(s), x1 = multi_reduce<1>(s + 1);
+            if ((lt & 31) == 0) {
+                share<CS>(&Q.w[0][vt >> 5], x0);
+                share<CS>(&Q.b[vt >> 5], x1);
+            }
+        }
+        scene_sync<CS>();
+        if (lt == 0) {
+            double t0 = 0.0, t1 = 0.0, l;
+            for (int w = 0; w < kChains / 32; ++w) t0 += Q.w[0][w];
+            for (int w = 0; w < kChains / 32; ++w) t1 += Q.b[w];
+            if (initial_lipschitz(t0, t1, A.dt2, l)) {
+                S.lipsch = l;
+                S.alpha = 1.0 / l;
+                S.lgood = l;
+            }
+        }
+    }
+    __syncthreads();
+    while (!S.done) {
+        const double alpha = S.alpha;
+        const bool bt = S.bt != 0, use_prev = S.use_prev != 0;
+        const T beta = S.beta;
+        const L* lam = pick_lam<T, DIM>(A, S.il);
+        const L* lprev = pick_lam<T, DIM>(A, S.ip);
+        L* lnew = pick_lam<T, DIM>(A, S.in_);
+        const V4<T>* uY = pick_u(A, S.jY);
+        const V4<T>* uL = pick_u(A, S.jL);
+        V4<T>* uN = pick_u(A, S.jN);
+        V4<T>* uYN = pick_u(A, S.jYN);
+        // square roots and divisions that the decisions need, on two warps while the others begin
+        if (lt == BT - 32) Q.mo = prepare_momentum(S);
+        if (lt == BT - 64) Q.next = prepare_step<T>(S, A.tol);
+        // ---- contact pass
+#pragma unroll 1
+        for (int k = tid; k < nc; k += NT) {
+            const int c = contact_at(k);
+            T ui[F::dof], uj[F::dof], r[F::row], lm[4], lq[4], lo[3], qo[3], s[8];
+            const int2 ij = A.cij[c];
+            load_row<T, DIM>(A.rec, A.cap, c, r);
+            fld4(lam + c, lm);
+            if (use_prev) fld4(lprev + c, lq);
+#pragma unroll
+            for (int d = 0; d < F::dof; ++d) ui[d] = uj[d] = (T)0;
+            if (ij.x >= A.nin) gather_u<T, DIM>(uY, ij.x - A.nin, ui);
+            if (ij.y >= A.nin) gather_u<T, DIM>(uY, ij.y - A.nin, uj);
+            contact_row<T, DIM, false>(r, ui, uj, lm, lq, beta, use_prev, bt, alpha, A.mu, A.dt2, nullptr, lo, s, qo);
+            fst4(lnew + c, lo);
+            fst4(qv + c, qo);
+        }
+        scene_sync<CS>();
+        // ---- the sums: chain vt, its first or second half of the values
+        {
+            constexpr int J = 2;  // contacts whose loads are in flight
+            const int part = SPLIT == 2 ? lt / VT : 0;
+            if (lt < SPLIT * VT) {
+                const int vt = rank * VT + (lt - part * VT);
+                double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll 1
+                for (int k = vt; k < nc; k += J * kChains) {
+                    T lm[J][4], lq[J][4], lp[J][4], q[J][4], cc[J][4];
+#pragma unroll
+                    for (int e = 0; e < J; ++e) {
+                        if (k + e * kChains >= nc) continue;
+                        const int c = contact_at(k + e * kChains);
+                        fld4cg(lam + c, lm[e]);
+                        if (use_prev) fld4cg(lprev + c, lq[e]);
+                        fld4cg(lnew + c, lp[e]);
+                        fld4cg(qv + c, q[e]);
+                        load_c<T, DIM>(A.rec, A.cap, c, cc[e]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < J; ++e) {
+                        if (k + e * kChains >= nc) continue;
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) {
+                            const double y =
+                                use_prev ? fma_rn(beta, add_rn(lm[e][d], -lq[e][d]), lm[e][d]) : lm[e][d];
+                            const double gm = add_rn(q[e][d], cc[e][d]), dly = add_rn(lp[e][d], -y),
+                                         dll = add_rn(lp[e][d], -lm[e][d]);
+                            if (SPLIT == 1 || part == 0) {
+                                s[0] = fma_rn(gm, dly, s[0]);
+                                s[1] = fma_rn(dly, dly, s[1]);
+                                s[2] = fma_rn(cc[e][d], lp[e][d], s[2]);
+                            }
+                            if (SPLIT == 1 || part == 1) {
+                                if (!bt) s[3] = fma_rn(y, fma_rn(0.5, q[e][d], cc[e][d]), s[3]);
+                                s[4] = fma_rn(dll, dll, s[4]);
+                                s[5] = fma_rn(gm, dll, s[5]);
+                                s[6] = fma_rn(lp[e][d], lp[e][d], s[6]);
+                            }
+                        }
+                    }
+                }
+                const double x = multi_reduce<8>(s);
+                const int v = (lt & 31) >> 2;
+                if ((lt & 3) == 0 && (SPLIT == 1 || (v >= 3) == (part == 1))) share<CS>(&Q.w[v][vt >> 5], x);
+            }
+        }
+        // ---- particle pass
+        const T bn_ = Q.mo.beta;
+#pragma unroll 1
+        for (int p = p0 + tid; p < p1; p += NT) {
+            const int k0 = A.inc_ptr[p];
+            T im[4], ul[F::dof], w[F::dof], u[F::dof];
+            fld4(A.invm + p, im);
+            if (bn_ != 0.0) load_u<T, DIM>(uL, p, ul);
+            body_force<T, DIM, DIM == 2 ? 4 : 3>(A.inc, inc_walk(lay, F::ni, p, k0), lnew, A.inc_ptr[p + 1] - k0, w);
+            body_velocity<T, DIM>(im, w, u);
+            store_u<T, DIM>(uN, p, u);
+            A.wu[p] = body_wu<T, DIM>(w, u);
+            if (bn_ != 0.0) {
+#pragma unroll
+                for (int d = 0; d < F::dof; ++d) u[d] = fma_rn(bn_, add_rn(u[d], -ul[d]), u[d]);
+            }
+            store_u<T, DIM>(uYN, p, u);
+        }
+        scene_sync<CS>();
+        // ---- w.u along the chains (every CTA all of them: one sum), then the decisions
+        {
+            double s[1] = {0.0};
+            if (lt < kChains)
+                for (int p = p0 + lt; p < p1; p += kChains) s[0] += __ldcg(A.wu + p);
+            const double x = multi_reduce<1>(s);
+            if (lt < kChains && (lt & 31) == 0) Q.b[lt >> 5] = x;
+        }
+        __syncthreads();
+        if (lt < 32) {
+            double x = 0.0;
+            const double* row = lt < 7 ? Q.w[lt] : Q.b;
+            if (lt < 8)
+                for (int w = 0; w < kChains / 32; ++w) x += row[w];
+            double t[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) t[k] = __shfl_sync(0xffffffffu, x, k);
+            if (lt == 0) {
+                decide_momentum<T>(S, t, bt, A.dynamic, Q.mo);
+                NextStep ns = Q.next;
+                ns.step = sqrt(S.last_step);
+                decide_step<T>(S, t[7], 0.0, A.dt2, A.dynamic, A.max_ite, ns, kMaxBacktracks);
+                if (!S.bt) {
+                    // after a restart y is l+ itself; the candidates take the two free buffers
+                    if (S.restart) S.jY = S.jL;
+                    int free[2] = {0, 0}, n = 0;
+                    for (int j = 0; j < 4 && n < 2; ++j)
+                        if (j != S.jL && j != S.jY) free[n++] = j;
+                    S.jN = free[0];
+                    S.jYN = free[1];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    // outputs and the violation max(0, -n.(dt^2 A u + C)) over the scene's contacts
+    const L* lres = pick_lam<T, DIM>(A, S.il);
+    const V4<T>* ures = pick_u(A, S.jL);
+    double vmax = 0.0;
+    for (int k = tid; k < nc; k += NT) {
+        const int c = contact_at(k);
+        const int2 ij = A.cij[c];
+        T r[F::row], l[4], ui[F::dof], uj[F::dof], a[3], b[3];
+        load_row<T, DIM>(A.rec, A.cap, c, r);
+        fld4(lres + c, l);
+        for (int d = 0; d < 3; ++d) A.lam_out[3 * (long long)c + d] = d < DIM ? l[d] : 0.0;
+        for (int d = 0; d < F::dof; ++d) ui[d] = uj[d] = 0.0;
+        if (ij.x >= A.nin) gather_u<T, DIM>(ures, ij.x - A.nin, ui);
+        if (ij.y >= A.nin) gather_u<T, DIM>(ures, ij.y - A.nin, uj);
+        point_velocity<T, DIM>(r, ui, a);
+        point_velocity<T, DIM>(r + (DIM == 3 ? 9 : 2), uj, b);
+        double gap = 0.0;
+        for (int d = 0; d < DIM; ++d) gap += (A.dt2 * (a[d] - b[d]) + r[F::at_c + d]) * r[F::at_n + d];
+        vmax = fmax(vmax, -gap);
+    }
+    for (int p = p0 + tid; p < p1; p += NT) {
+        T u[F::dof];
+        load_u<T, DIM>(ures, p, u);
+        T* o = A.u_out + 6 * (long long)p;
+        for (int d = 0; d < 6; ++d) o[d] = DIM == 3 ? u[d] : (d < 2 ? u[d] : (d == 5 ? u[2] : 0.0));
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) vmax = fmax(vmax, __shfl_xor_sync(0xffffffffu, vmax, o));
+    __shared__ double vm[32];
+    if ((lt & 31) == 0) vm[lt >> 5] = vmax;
+    __syncthreads();
+    if (lt == 0) {
+        for (int w = 0; w < BT / 32; ++w) vmax = fmax(vmax, vm[w]);
+        if (CS > 1) share<CS>(&Q.vmax[rank], vmax);
+    }
+    if (CS > 1) cluster_sync();  // also: no CTA leaves while another may still write into its shared memory
+    if (rank == 0 && lt == 0) {
+        for (int r = 0; r < CS; ++r)
+            if (CS > 1) vmax = fmax(vmax, Q.vmax[r]);
+        BatchSceneStats& st = B.stats[sc];
+        st.contacts = nc;
+        st.iterations = S.ite;
+        st.fp32_iterations = 0;
+        st.backtracks = S.nbt;
+        st.restarts = S.nrs;
+        st.corrections = 0;
+        st.converged = S.conv && !S.err;
+        st.violation = vmax;
+    }
+}
+
+// Clusters of CS CTAs: cluster q < n_big solves the q-th largest scene with all of them, every
+// later one CS of the other scenes, one per CTA (those never meet a cluster barrier).
+template <int DIM, int CS>
+__global__ void __launch_bounds__(kBatchFricThreads<DIM>, 1) k_fric_batch(FricArgs<double> A, BatchFricScenes B) {
+    __shared__ ApgdState S;
+    __shared__ SceneSums Q;
+    if (A.sizes->overflow) return;  // the step is redone after the buffers grow (all CTAs alike)
+    const int q = blockIdx.x / CS, rank = blockIdx.x % CS;
+    if (CS > 1 && q < B.n_big) {
+        fric_scene<DIM, CS>(A, B, B.order[q], rank, S, Q);
+    } else {
+        const int j = CS == 1 ? q : B.n_big + CS * (q - B.n_big) + rank;
+        if (j < B.n_scenes) fric_scene<DIM, 1>(A, B, B.order[j], 0, S, Q);
+    }
 }
 
 // ------------------------------------------------------------------ packing
@@ -592,6 +978,7 @@ cudaError_t launch_fric_t(FricArgs<T>& A, int nblocks, cudaStream_t s) {
 
 size_t fric_rec_bytes(int dim, bool fp32) { return (dim == 3 ? 24 : 8) * (fp32 ? 4 : 8); }
 size_t fric_inc_bytes(int dim, bool fp32) { return dim == 3 ? (fp32 ? 48 : 80) : (fp32 ? 16 : 32); }
+size_t fric_lam_bytes(int dim, bool fp32) { return (dim == 3 ? 4 : 2) * (fp32 ? 4 : 8); }
 int fric_u_vectors(int dim) { return dim == 3 ? 2 : 1; }
 
 int apgd_fric_max_blocks() {
@@ -626,9 +1013,9 @@ void launch_fric_pack_c(int dim, const double* cvec, FricSolve<T>& f, const Size
         k_fric_pack_c<T, 2><<<blocks(f.cap), 256, 0, s>>>(sizes, f.cap, cvec, rec);
     g_fric_launches += 1;
 }
+namespace {
 template <typename T>
-cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, FricSolve<T>& f, const Sizes* sizes,
-                             int nblocks, cudaStream_t s) {
+FricArgs<T> fric_args(int nin, int na, const ApgdSettings& st, const FricSolve<T>& f, const Sizes* sizes) {
     FricArgs<T> A;
     A.nin = nin;
     A.na = na;
@@ -640,13 +1027,13 @@ cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, F
     A.inc = static_cast<const Q4<T>*>(f.inc);
     A.inc_slots = f.inc_slots;
     A.invm = reinterpret_cast<const V4<T>*>(f.invm);
-    A.lam0 = f.lam[0];
-    A.lam1 = f.lam[1];
-    A.lam2 = f.lam[2];
+    for (int k = 0; k < 3; ++k) A.lam[k] = f.lam[k];
     A.u0 = f.u[0];
     A.u1 = f.u[1];
     A.u2 = f.u[2];
     A.u3 = f.u[3];
+    A.qv = f.qv;
+    A.wu = f.wu;
     A.lam_out = f.lam_out;
     A.u_out = f.u_out;
     A.sums = f.sums;
@@ -661,7 +1048,48 @@ cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, F
     A.dynamic = st.dynamic;
     A.curvature_start = st.curvature_start;
     A.stall = st.stall;
+    return A;
+}
+}  // namespace
+
+template <typename T>
+cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, FricSolve<T>& f, const Sizes* sizes,
+                             int nblocks, cudaStream_t s) {
+    FricArgs<T> A = fric_args<T>(nin, na, st, f, sizes);
     return dim == 3 ? launch_fric_t<T, 3>(A, nblocks, s) : launch_fric_t<T, 2>(A, nblocks, s);
+}
+namespace {
+template <int DIM, int CS>
+cudaError_t launch_fric_batch_t(const FricArgs<double>& A, const BatchFricScenes& B, cudaStream_t s) {
+    const int clusters = CS == 1 ? B.n_scenes : B.n_big + (B.n_scenes - B.n_big + CS - 1) / CS;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(CS * clusters);
+    cfg.blockDim = dim3(kBatchFricThreads<DIM>);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = CS;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    g_fric_launches += 1;
+    return cudaLaunchKernelEx(&cfg, k_fric_batch<DIM, CS>, A, B);
+}
+}  // namespace
+
+cudaError_t launch_fric_batch(int nin, int na, int dim, const ApgdSettings& st, FricSolve<double>& f,
+                              const Sizes* sizes, BatchFricScenes B, cudaStream_t s) {
+    if (B.n_scenes <= 0) return cudaSuccess;
+    const FricArgs<double> A = fric_args<double>(nin, na, st, f, sizes);
+    B.n_big = std::min(std::max(B.n_big, 0), B.n_scenes);
+    // the longest scene is the critical path: the scenes with at least half its bodies get four
+    // CTAs while all CTAs still run at once (3 scenes of up to 300 disks: 11.7 -> 4.6 ms a step
+    // against the generic rows), else two (200 scenes of up to 3000: 128.8 -> 29.2)
+    const int small = B.n_scenes - B.n_big;
+    if (4 * B.n_big + (small + 3) / 4 * 4 <= kSMs)
+        return dim == 3 ? launch_fric_batch_t<3, 4>(A, B, s) : launch_fric_batch_t<2, 4>(A, B, s);
+    return dim == 3 ? launch_fric_batch_t<3, 2>(A, B, s) : launch_fric_batch_t<2, 2>(A, B, s);
 }
 #define INST(T) \
     template void launch_fric_pack<T>(int, int, const Contacts&, const Assembly&, const Incidence&, FricSolve<T>&, \

@@ -352,8 +352,10 @@ struct FricSolve {
     const double* shift;      // correction solves: solution offset (null = none)
     const int* inc_ptr;
     const T* invm;            // 4 per active body
-    V4<T>* lam[3];
+    void* lam[3];             // fric_lam_bytes per contact
     V4<T>* u[4];              // fric_u_vectors(dim) per active body
+    void* qv;                 // batches: fric_lam_bytes per contact
+    double* wu;               // batches: 1 per active body
     T* lam_out;               // 3 per contact
     T* u_out;                 // 6 per active body (null: not wanted)
     double* sums;             // kSumBytesPerBlock per block, all ones at launch
@@ -362,6 +364,7 @@ struct FricSolve {
 };
 size_t fric_rec_bytes(int dim, bool fp32);
 size_t fric_inc_bytes(int dim, bool fp32);
+size_t fric_lam_bytes(int dim, bool fp32);
 int fric_u_vectors(int dim);
 int apgd_fric_max_blocks();
 long long apgd_fric_launches();
@@ -414,7 +417,7 @@ struct BatchSolve {
     int curvature_start;
 };
 
-// Batched scenes of a 6-dof problem (Friction), FP64: one CTA per scene over the scene
+// Batched scenes of a 6-dof problem, FP64: one CTA per scene over the scene
 // ranges of launch_batch_ranges; the multipliers (3 per contact) and u (6 per active body)
 // of every scene end in lam_out / u_out, its statistics in stats[scene].
 struct Batch6Scenes {
@@ -428,6 +431,16 @@ struct Batch6Scenes {
 cudaError_t launch_apgd_batch6(const Bodies& b, const StepParams& p, const ApgdSettings& st, const Contacts& c,
                                const Assembly& a, SolveBuffers<double>& sb, const double* invm,
                                const Batch6Scenes& S, cudaStream_t s);
+
+struct BatchFricScenes {
+    int n_scenes;
+    int n_big;          // the largest scenes (at least half the largest one's bodies)
+    const int* order;   // largest first
+    const int *sc_p0, *sc_p1, *sc_o0, *sc_o1, *sc_a0, *sc_a1;
+    BatchSceneStats* stats;
+};
+cudaError_t launch_fric_batch(int nin, int na, int dim, const ApgdSettings& st, FricSolve<double>& f,
+                              const Sizes* sizes, BatchFricScenes B, cudaStream_t s);
 
 long long apgd_batch_launches();
 void launch_batch_ranges(int n_scenes, int nin, const int* sc_obs0, const int* sc_obs1, const int* sc_p0,

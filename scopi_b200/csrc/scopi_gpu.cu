@@ -114,7 +114,7 @@ struct scopi_gpu_handle {
     // Friction (apgd_fric.cu): rows, incidence records and iterates of the solve; the FP64 set of
     // a mixed handle is allocated when its first FP64 correction runs
     struct FricBuffers {
-        void *rec = nullptr, *inc = nullptr, *lam[3] = {}, *u[4] = {};
+        void *rec = nullptr, *inc = nullptr, *lam[3] = {}, *u[4] = {}, *qv = nullptr, *wu = nullptr;
     };
     FricBuffers fb64{}, fb32{};
     DevMem fric_mem;
@@ -166,8 +166,8 @@ struct scopi_gpu_handle {
     // multipliers in c (and the Jacobian kept as the three rows of A) per contact
     int cvec_per() const { return P.problem == SCOPI_GPU_VISCOUS_FRICTION ? 4 : (friction_rows() ? 3 : 1); }
     bool friction_rows() const { return P.problem == SCOPI_GPU_FRICTION || P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
-    // single scenes of the Friction problem (and FrictionFixedPoint): apgd_fric.cu
-    bool fric() const { return P.problem == SCOPI_GPU_FRICTION && !batch; }
+    // the Friction problem (and FrictionFixedPoint): apgd_fric.cu
+    bool fric() const { return P.problem == SCOPI_GPU_FRICTION; }
     long long inc_slots() const { return kIncSlotsPerContact * c_cap; }
     bool viscous_friction() const { return P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
     bool fp_loop() const { return fixed_point || viscous_friction(); }
@@ -315,6 +315,26 @@ struct scopi_gpu_handle {
         st.dt = dt;
         st.mu = P.mu;
         st.curvature_start = curvature_start();
+        auto scenes = [&](auto& S) {
+            S.n_scenes = n_scenes;
+            S.order = d_order;
+            S.sc_p0 = d_sc_p0;
+            S.sc_p1 = d_sc_p1;
+            S.sc_o0 = d_sc_o0;
+            S.sc_o1 = d_sc_o1;
+            S.sc_a0 = d_sc_a0;
+            S.sc_a1 = d_sc_a1;
+            S.stats = d_bstats;
+        };
+        if (fric()) {
+            BatchFricScenes S{};
+            scenes(S);
+            S.n_big = batch_n_big;
+            FricSolve<double> f = fric_buffers<double>(fb64, d_invm64, d_lamacc, d_ufin);
+            launch_fric_pack<double>(P.dim, na, cur, as, inc, f, d_sizes_cur, stream);
+            launch_fric_batch(nin, na, P.dim, st, f, d_sizes_cur, S, stream);
+            return;
+        }
         const long long M = (long long)mult_per_contact() * c_cap;
         cudaMemsetAsync(d_lam64[0], 0, M * sizeof(double), stream);
         cudaMemsetAsync(d_lam64[1], 0, M * sizeof(double), stream);
@@ -335,15 +355,7 @@ struct scopi_gpu_handle {
         }
         sb.g = d_g64;
         Batch6Scenes S{};
-        S.n_scenes = n_scenes;
-        S.order = d_order;
-        S.sc_p0 = d_sc_p0;
-        S.sc_p1 = d_sc_p1;
-        S.sc_o0 = d_sc_o0;
-        S.sc_o1 = d_sc_o1;
-        S.sc_a0 = d_sc_a0;
-        S.sc_a1 = d_sc_a1;
-        S.stats = d_bstats;
+        scenes(S);
         S.lam_out = d_lamacc;
         S.u_out = d_ufin;
         launch_apgd_batch6(b, sp, st, cur, as, sb, d_invm64, S, stream);
@@ -665,8 +677,10 @@ struct scopi_gpu_handle {
             return e == cudaSuccess;
         };
         bool ok = get(b.rec, c_cap * fric_rec_bytes(P.dim, f32)) && get(b.inc, inc_slots() * fric_inc_bytes(P.dim, f32));
-        for (int k = 0; k < 3 && ok; ++k) ok = get(b.lam[k], c_cap * sizeof(V4<T>));
+        for (int k = 0; k < 3 && ok; ++k) ok = get(b.lam[k], c_cap * fric_lam_bytes(P.dim, f32));
         for (int k = 0; k < 4 && ok; ++k) ok = get(b.u[k], ((size_t)na + 1) * fric_u_vectors(P.dim) * sizeof(V4<T>));
+        if (batch && ok)
+            ok = get(b.qv, c_cap * fric_lam_bytes(P.dim, f32)) && get(b.wu, ((size_t)na + 1) * sizeof(double));
         if (!ok) b = FricBuffers{};
         return ok ? 0 : cuda_fail(e, "cudaMalloc(friction rows)");
     }
@@ -967,8 +981,9 @@ struct scopi_gpu_handle {
         st.curvature_start = alpha0 > 0.0 ? 0 : curvature_start();
         const size_t ub = (size_t)na * fric_u_vectors(P.dim) * sizeof(V4<T>);
         // lambda = lambda_prev = 0 and u(lambda) = u(y) = 0 (cold start, apgd.hpp:152-159)
-        cudaMemsetAsync(f.lam[0], 0, h_sizes->C * sizeof(V4<T>), stream);
-        cudaMemsetAsync(f.lam[1], 0, h_sizes->C * sizeof(V4<T>), stream);
+        const size_t lb = (size_t)h_sizes->C * fric_lam_bytes(P.dim, sizeof(T) == 4);
+        cudaMemsetAsync(f.lam[0], 0, lb, stream);
+        cudaMemsetAsync(f.lam[1], 0, lb, stream);
         cudaMemsetAsync(f.u[0], 0, ub, stream);
         cudaMemsetAsync(f.u[2], 0, ub, stream);
         cudaError_t e = reset_barrier(st);
@@ -995,8 +1010,10 @@ struct scopi_gpu_handle {
         f.inc_slots = inc_slots();
         f.inc_ptr = inc.ptr;
         f.invm = invm;
-        for (int k = 0; k < 3; ++k) f.lam[k] = static_cast<V4<T>*>(b.lam[k]);
+        for (int k = 0; k < 3; ++k) f.lam[k] = b.lam[k];
         for (int k = 0; k < 4; ++k) f.u[k] = static_cast<V4<T>*>(b.u[k]);
+        f.qv = b.qv;
+        f.wu = static_cast<double*>(b.wu);
         f.lam_out = lam_out;
         f.u_out = u_out;
         f.sums = d_sums;

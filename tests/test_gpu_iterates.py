@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 
 import py_oracle as orc
-from scopi_b200 import FP64, FRICTION, MIXED, NOFRICTION, VISCOUS, ScopiSolver, configs
+from scopi_b200 import FP64, FRICTION, MIXED, NOFRICTION, VISCOUS, ScopiBatch, ScopiSolver, configs
 
 pytestmark = pytest.mark.gpu
 
@@ -81,3 +81,23 @@ def test_friction_iterates(dim, count, precision):
 @pytest.mark.parametrize("dim,count", [(3, 2), (3, 200), (3, 27001), (3, 45007), (2, 3), (2, 300)])
 def test_normal_iterates(dim, count, problem, precision):
     check(dim, count, problem, precision)
+
+
+# Batched friction scenes: clusters of four CTAs (few scenes) and of two (many), the largest
+# scenes on a whole cluster, the others one CTA each; 256 chains of contacts in the sums.
+@pytest.mark.parametrize("dim,sizes", [(2, [300]), (2, [3, 700, 90, 1500]), (2, [40 + 7 * k for k in range(90)]),
+                                       (3, [250, 5, 600]), (3, [20 + k for k in range(80)])])
+def test_batch_friction_iterates(dim, sizes):
+    scenes = [bed(dim, n, seed=20 + k) for k, n in enumerate(sizes)]
+    kw = settings(dim, FRICTION)
+    b = ScopiBatch(scenes, **kw)
+    b.run(DT, 1)
+    for k, pa in enumerate(scenes):
+        o = orc.OracleSolver(pa, **kw).run(DT, 1)
+        st, so = b.scene_stats(k), o.stats()
+        assert st["contacts"] == so["contacts"]
+        assert (st["iterations"], st["backtracks"]) == (so["iterations"], so["backtracks"])
+        g = b.scene(k)
+        assert np.linalg.norm(g.v - o.pa.v) <= 1e-12 * np.linalg.norm(o.pa.v)
+        assert np.linalg.norm(g.omega - o.pa.omega) <= 1e-12 * np.linalg.norm(o.pa.omega)
+    b.close()
