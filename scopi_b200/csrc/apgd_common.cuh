@@ -135,17 +135,18 @@ __device__ __forceinline__ void sum_publish(double* slots, unsigned int nb, unsi
         st_relaxed_f64(slots + (size_t)(m & 3) * nb * kSumRec + rec, v == v ? v : __longlong_as_double(0x7ff8000000000000ll));
 }
 
-// The NP values of all nb blocks (nb <= kSumMaxBlocks): lane l gets blocks l, l + 32, ... in
-// x[0..4] (zeros past nb).  Called by one whole warp.  A wait longer than the limit (bar[3])
-// sets the error flag bar[2]; every waiter sees the flag and returns false.
-template <int NP>
+// The NP values of NW groups of 32 blocks from block b0 on (all of them: NW = 5, b0 = 0;
+// nb <= kSumMaxBlocks): lane l gets blocks b0 + l, b0 + l + 32, ... in x (zeros past nb).  Called
+// by one whole warp.  A wait longer than the limit (bar[3]) sets the error flag bar[2]; every
+// waiter sees the flag and returns false.
+template <int NP, int NW>
 __device__ __forceinline__ bool sum_collect(const double* slots, unsigned int nb, unsigned int m, unsigned int* bar,
-                                            double (&x)[5][NP]) {
-    const unsigned int lane = threadIdx.x & 31;
+                                            double (&x)[NW][NP], unsigned int b0 = 0) {
+    const unsigned int lane = b0 + (threadIdx.x & 31);
     const double* base = slots + (size_t)(m & 3) * nb * kSumRec;
     unsigned int pending = 0;
 #pragma unroll
-    for (int w = 0; w < 5; ++w) {
+    for (int w = 0; w < NW; ++w) {
 #pragma unroll
         for (int k = 0; k < NP; ++k) x[w][k] = 0.0;
         if (lane + 32u * w < nb) pending |= 1u << w;
@@ -155,7 +156,7 @@ __device__ __forceinline__ bool sum_collect(const double* slots, unsigned int nb
     bool ok = true;
     for (unsigned int it = 1;; ++it) {
 #pragma unroll
-        for (int w = 0; w < 5; ++w) {
+        for (int w = 0; w < NW; ++w) {
             if (!(pending & (1u << w))) continue;
             const double* r = base + (size_t)(lane + 32u * w) * kSumRec;
             if (NP == 1) {
@@ -166,7 +167,7 @@ __device__ __forceinline__ bool sum_collect(const double* slots, unsigned int nb
             }
         }
 #pragma unroll
-        for (int w = 0; w < 5; ++w) {
+        for (int w = 0; w < NW; ++w) {
             if (!(pending & (1u << w))) continue;
             bool got = true;
 #pragma unroll
@@ -319,13 +320,63 @@ struct GridSums {
     template <int NP>
     __device__ __forceinline__ bool collect(double* t) {
         double x[5][NP];
-        const bool ok = sum_collect<NP>(slots, nb, m, bar, x);
+        const bool ok = sum_collect<NP, 5>(slots, nb, m, bar, x);
         const double y = TREE ? sum_lane_order<NP>(x) : sum_group_order<NP>(x);
 #pragma unroll
         for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, y, k << SumShift<NP>::value);
         return ok;
     }
     __device__ __forceinline__ void next() { ++m; }
+    // a barrier without sums, split so that work can be done between the halves (all threads)
+    __device__ __forceinline__ void arrive() {
+        __syncthreads();
+        if (threadIdx.x < 32) sum_publish(slots, nb, m, threadIdx.x == 0, 0, 0.0, withhold && m == 0);
+    }
+    __device__ __forceinline__ bool wait() {
+        __shared__ int s_ok;
+        if (threadIdx.x < 32) {
+            double x[5][1];
+            const bool ok = sum_collect<1, 5>(slots, nb, m, bar, x);
+            if (threadIdx.x == 0) s_ok = ok;
+        }
+        ++m;
+        __syncthreads();
+        return s_ok != 0;
+    }
+    // publish and collect in one, in lane order (all threads, at least 160; the totals and the
+    // status are warp 0's).  Five warps collect a group of blocks each, so that no thread holds
+    // more than NP of the values.
+    template <int NP>
+    __device__ __forceinline__ bool sums(double* v, double (*sh)[32], double* t) {
+        __shared__ double raw[5][NP][32];
+        __shared__ int bad;
+        if (threadIdx.x == 0) bad = 0;
+        publish<NP>(v, sh);
+        const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (w < 5) {
+            double x[1][NP];
+            const bool ok = sum_collect<NP, 1>(slots, nb, m, bar, x, 32u * w);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) raw[w][k][lane] = x[0][k];
+            if (!ok && lane == 0) bad = 1;
+        }
+        ++m;
+        __syncthreads();
+        if (w == 0) {
+            double y[NP];
+#pragma unroll
+            for (int k = 0; k < NP; ++k) {
+                y[k] = 0.0;
+#pragma unroll
+                for (int g = 0; g < 5; ++g) y[k] += raw[g][k][lane];
+            }
+            const double z = multi_reduce<NP>(y);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, z, k << SumShift<NP>::value);
+        }
+        return bad == 0;
+    }
+    __device__ __forceinline__ void finish() {}
     // one value per block (the same in all its threads), summed in group order; a full barrier
     __device__ __forceinline__ bool exchange(double v, double& total) {
         __shared__ double s_t;
@@ -334,7 +385,7 @@ struct GridSums {
         if (threadIdx.x < 32) {
             sum_publish(slots, nb, m, threadIdx.x == 0, 0, v, withhold && m == 0);
             double x[5][1];
-            const bool ok = sum_collect<1>(slots, nb, m, bar, x);
+            const bool ok = sum_collect<1, 5>(slots, nb, m, bar, x);
             const double y = sum_group_order<1>(x);
             if (threadIdx.x == 0) {
                 s_t = y;
@@ -347,6 +398,15 @@ struct GridSums {
         return s_ok != 0;
     }
 };
+
+// roundings written out where the compiler could contract in more than one way: a solve's
+// bits are then the same whatever kernel it runs in
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 
 // LagrangeMultiplier<Friction>::projection, include/scopi/solvers/lagrange_multiplier.hpp:243-268
 template <int DIM>
@@ -413,6 +473,84 @@ __device__ __forceinline__ void overflow_cascade(double& lipsch, double& alpha, 
     }
     alpha = 1. / lipsch;
 }
+
+// The same for a launch of one cluster (up to 16 CTAs): hardware cluster barriers, block sums
+// read through distributed shared memory, in the order of GridSums<true>.  Nothing can be
+// missing from such a barrier (the CTAs of a cluster run together), so there is no limit.
+struct ClusterSums {
+    int par;
+
+    __device__ __forceinline__ void arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+    __device__ __forceinline__ bool wait() {
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
+    __device__ __forceinline__ static double remote(const double* own, unsigned int rank) {
+        const unsigned int a = (unsigned int)__cvta_generic_to_shared(own);
+        unsigned int r;
+        double v;
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+        asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(r) : "memory");
+        return v;
+    }
+    // a slot is written again two exchanges later, when every CTA has passed the barrier of the
+    // exchange between, which it enters after its reads
+    template <int NP>
+    __device__ __forceinline__ void read(const double* own, double (&x)[5][NP]) {
+        const unsigned int lane = threadIdx.x & 31;
+#pragma unroll
+        for (int w = 0; w < 5; ++w)
+#pragma unroll
+            for (int k = 0; k < NP; ++k) x[w][k] = 0.0;
+        if (lane < gridDim.x)
+#pragma unroll
+            for (int k = 0; k < NP; ++k) x[0][k] = remote(own + k, lane);
+    }
+    template <int NP>
+    __device__ __forceinline__ bool sums(double* v, double (*sh)[32], double* t) {
+        __shared__ double part[2][8];
+        warp_sums<NP>(v, sh);
+        __syncthreads();
+        constexpr int sf = SumShift<NP>::value;
+        if (threadIdx.x < 32) {
+            const double x = block_sums_tree<NP>(sh);
+            if ((threadIdx.x & ((1 << sf) - 1)) == 0) part[par][threadIdx.x >> sf] = x;
+        }
+        arrive();
+        wait();
+        if (threadIdx.x < 32) {
+            double x[5][NP];
+            read<NP>(part[par], x);
+            const double y = sum_lane_order<NP>(x);
+#pragma unroll
+            for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, y, k << sf);
+        }
+        par ^= 1;
+        return true;
+    }
+    __device__ __forceinline__ bool exchange(double v, double& total) {
+        __shared__ double one[2];
+        __shared__ double s_t;
+        if (threadIdx.x == 0) one[par] = v;
+        arrive();
+        wait();
+        if (threadIdx.x < 32) {
+            double x[5][1];
+            read<1>(&one[par], x);
+            const double y = sum_group_order<1>(x);
+            if (threadIdx.x == 0) s_t = y;
+        }
+        par ^= 1;
+        __syncthreads();
+        total = s_t;
+        return true;
+    }
+    // before a CTA leaves: nobody reads its shared memory any more
+    __device__ __forceinline__ void finish() {
+        arrive();
+        wait();
+    }
+};
 
 // Loop-carried scalars of the iteration (block-uniform) live in shared memory and are
 // updated by thread 0, so the registers go to the two passes.
@@ -539,6 +677,16 @@ __device__ __forceinline__ void decide_step(ApgdState& S, double wu, double curv
     }
     S.use_prev = (S.beta != 0.0) ? 1 : 0;
     if (S.ite >= max_ite) S.done = 1;
+}
+// After an accepted step of the kernels whose particle pass does not wait for the sums: a
+// restart makes u(l+) the next u(y); the candidates take the two free buffers.
+__device__ __forceinline__ void reuse_buffers(ApgdState& S) {
+    if (S.restart) S.jY = S.jL;
+    int free[2] = {0, 0}, n = 0;
+    for (int j = 0; j < 4 && n < 2; ++j)
+        if (j != S.jL && j != S.jY) free[n++] = j;
+    S.jN = free[0];
+    S.jYN = free[1];
 }
 __device__ __forceinline__ void write_result(ApgdResult* r, const ApgdState& S) {
     r->iterations = S.ite;

@@ -89,14 +89,6 @@ __device__ __forceinline__ void fld4cg(const float2* p, float* o) { const float2
 __device__ __forceinline__ void fld4cg(const double2* p, double* o) { put4(o, __ldcg(p)); }
 __device__ __forceinline__ void fst4(float2* p, const float* v) { *p = make_float2(v[0], v[1]); }
 __device__ __forceinline__ void fst4(double2* p, const double* v) { *p = make_double2(v[0], v[1]); }
-// roundings written out where the compiler could contract in more than one way: a solve's
-// bits are then the same whatever kernel it runs in
-__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
-__device__ __forceinline__ float add_rn(float a, float b) { return __fadd_rn(a, b); }
-__device__ __forceinline__ double add_rn(double a, double b) { return __dadd_rn(a, b); }
-__device__ __forceinline__ float fma_rn(float a, float b, float c) { return __fmaf_rn(a, b, c); }
-__device__ __forceinline__ double fma_rn(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ unsigned fidx(float w) { return (unsigned)__float_as_int(w); }
 __device__ __forceinline__ unsigned fidx(double w) { return (unsigned)__double_as_longlong(w); }
 template <typename T>
@@ -787,15 +779,7 @@ __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, 
                 NextStep ns = Q.next;
                 ns.step = sqrt(S.last_step);
                 decide_step<T>(S, t[7], 0.0, A.dt2, A.dynamic, A.max_ite, ns, kMaxBacktracks);
-                if (!S.bt) {
-                    // after a restart y is l+ itself; the candidates take the two free buffers
-                    if (S.restart) S.jY = S.jL;
-                    int free[2] = {0, 0}, n = 0;
-                    for (int j = 0; j < 4 && n < 2; ++j)
-                        if (j != S.jL && j != S.jY) free[n++] = j;
-                    S.jN = free[0];
-                    S.jYN = free[1];
-                }
+                if (!S.bt) reuse_buffers(S);
             }
         }
         __syncthreads();

@@ -12,6 +12,7 @@
 //   per body    : u(y) gathered once (u(y_next) = u(l+) + beta (u(l+) - u(l)) is formed in
 //                 the particle pass, the restart test being reduced after the first barrier).
 #include <algorithm>
+#include <atomic>
 #include <cstdio>
 #include <mutex>
 
@@ -122,12 +123,17 @@ __device__ __forceinline__ T pick4(int k, T a, T b, T c, T d) {
     return k == 0 ? a : (k == 1 ? b : (k == 2 ? c : d));
 }
 
-// one multiplier of the contact pass (lm, lpm: its current and previous values)
+// n.u, rounded as the streaming pass rounds it
+template <typename T, int DIM>
+__device__ __forceinline__ T normal_dot(const V4<T>& n, const V4<T>& u) {
+    const T xy = fma_rn(n.x, u.x, mul_rn(n.y, u.y));
+    return DIM == 3 ? fma_rn(n.z, u.z, xy) : xy;
+}
+// one multiplier of the contact pass (lm, lpm: its current and previous values); returns l+
 template <typename T>
-__device__ __forceinline__ void mult_update_v(const SphArgs<T>& A, long long m, T qy, T cc, T lm, T lpm, T* lnew,
+__device__ __forceinline__ T mult_update_v(const SphArgs<T>& A, long long m, T qy, T gm, T cc, T lm, T lpm, T* lnew,
                                               T beta, bool use_prev, bool bt, double alpha, double* s) {
-    const T y = use_prev ? lm + beta * (lm - lpm) : lm;
-    const T gm = qy + cc;
+    const T y = use_prev ? fma_rn(beta, add_rn(lm, -lpm), lm) : lm;
     T lp;
     if (A.shift) {
         const double sh = A.shift[m];
@@ -135,7 +141,7 @@ __device__ __forceinline__ void mult_update_v(const SphArgs<T>& A, long long m, 
         z = z > 0.0 ? z : 0.0;
         lp = (T)(z - sh);
     } else {
-        const T z = y - (T)alpha * gm;
+        const T z = fma_rn(-(T)alpha, gm, y);
         lp = z > (T)0 ? z : (T)0;
     }
     lnew[m] = lp;
@@ -151,11 +157,23 @@ __device__ __forceinline__ void mult_update_v(const SphArgs<T>& A, long long m, 
     s[4] += dll * dll;
     s[5] += (double)gm * dll;
     s[6] += (double)lp * (double)lp;
+    return lp;
 }
-template <typename T>
-__device__ __forceinline__ void mult_update(const SphArgs<T>& A, long long m, T qy, T cc, const T* lam, const T* lprev,
-                                            T* lnew, T beta, bool use_prev, bool bt, double alpha, double* s) {
-    mult_update_v<T>(A, m, qy, cc, lam[m], use_prev ? lprev[m] : (T)0, lnew, beta, use_prev, bt, alpha, s);
+// A contact: its row, u(y) of its bodies, the current and previous multipliers (lm2, lpm2: of the
+// viscous second multiplier at slot sv, if any); returns the candidate(s).
+template <typename T, int DIM, int PROB>
+__device__ __forceinline__ T contact_update(const SphArgs<T>& A, long long c, const V4<T>& nc, const V4<T>& ui,
+                                            const V4<T>& uj, T lm, T lpm, int sv, T lm2, T lpm2, T* lp2, T* lnew,
+                                            T beta, bool use_prev, bool bt, double alpha, double* s) {
+    // obstacles have u = 0
+    const T q0 = add_rn(normal_dot<T, DIM>(nc, ui), -normal_dot<T, DIM>(nc, uj));
+    const T qy = mul_rn(q0, (T)A.dt2);
+    // one rounding where the product is wanted for nothing else
+    const T gm = sizeof(T) == 4 && PROB == kNoFriction ? fma_rn(q0, (T)A.dt2, nc.w) : add_rn(qy, nc.w);
+    const T lp = mult_update_v<T>(A, c, qy, gm, nc.w, lm, lpm, lnew, beta, use_prev, bt, alpha, s);
+    if (PROB == kViscous && sv >= 0)
+        *lp2 = mult_update_v<T>(A, sv, -qy, -gm, -nc.w, lm2, lpm2, lnew, beta, use_prev, bt, alpha, s);
+    return lp;
 }
 
 // One block per SM (SphShape): FP32 768 threads (80 registers, no spills), FP64 512 (128).
@@ -175,8 +193,7 @@ __device__ __forceinline__ void mult_update(const SphArgs<T>& A, long long m, T 
 //   contact pass, GC stages, per contact : (ci, cj), (n, c), l, l_prev  -- 32 B (FP32), 56 B (FP64)
 //   particle pass, GP stages, per body   : inc_ptr[p], inc_ptr[p+1], 1/m, u(l) and (FP32) u(y)
 // and the gathers that depend on a staged record (u(y) of the contact's bodies) are issued
-// GD trips ahead.  The incidence records stay on plain loads: a body's records share L1
-// lines, which an L1-bypassing copy would fetch again from L2 for every record.
+// GD trips ahead.  The incidence records stay on plain loads.
 // Launch shape per precision: threads per block, contact-pass stages GC (the u(y) gathers
 // of trip k + GD are issued during trip k: an L2 round trip is about one trip long),
 // particle-pass stages GP.
@@ -199,6 +216,66 @@ struct SphOcc {
         (size_t)GP * threads * ((sizeof(T) == 4 ? 2 : 1) * sizeof(V4<T>) + sizeof(T) + 2 * sizeof(int));
     static constexpr size_t smem = contact_bytes > particle_bytes ? contact_bytes : particle_bytes;
 };
+
+// Initial step from the curvature along the first descent direction d (stored in the candidate
+// buffer, which the first contact pass overwrites).
+template <typename T, int DIM, int PROB, typename SY>
+__device__ __forceinline__ void curvature_step(const SphArgs<T>& A, int C, IncLayout lay, ApgdState& S, SY& G) {
+    T* dbuf = A.lam2;
+    double t1 = 0.0, t3 = 0.0;
+    double a2[2] = {0.0, 0.0};
+    GRID_STRIDE(c, C) {
+        const T cc = ld4(A.nc + c).w;
+        const T d = first_descent<T>(cc, A.shift, c);
+        dbuf[c] = d;
+        a2[0] += (double)d * (double)d;
+        if (PROB == kViscous) {
+            const int sl = A.slot[c];
+            if (sl >= 0) {
+                const T d2 = first_descent<T>(-cc, A.shift, sl);
+                dbuf[sl] = d2;
+                a2[0] += (double)d2 * (double)d2;
+            }
+        }
+    }
+    block_sum<2>(a2);
+    bool ok = G.exchange(a2[0], t1);
+    double wm[2] = {0.0, 0.0};
+    if (ok) GRID_STRIDE(p, A.na) {
+        T w0 = 0, w1 = 0, w2 = 0;
+        const int k0 = A.inc_ptr[p], n = A.inc_ptr[p + 1] - k0;
+        const IncWalk wk = inc_walk(lay, sizeof(T) / 4, p, k0);
+        for (int k = 0; k < n; ++k) {
+            const V4<T> e = ld_inc(A.inc, wk, k);
+            const int ci = idx_of(e.w);
+            T mu = __ldcg(dbuf + ci);
+            if (PROB == kViscous) {
+                const int sl = A.slot[ci];
+                if (sl >= 0) mu -= __ldcg(dbuf + sl);
+            }
+            w0 += mu * e.x;
+            w1 += mu * e.y;
+            if (DIM == 3) w2 += mu * e.z;
+        }
+        const double im = (double)A.invm[p];
+        wm[0] += im * ((double)w0 * w0 + (double)w1 * w1 + (double)w2 * w2);
+    }
+    block_sum<2>(wm);
+    if (ok) ok = G.exchange(wm[0], t3);
+    if (threadIdx.x == 0) {
+        double l;
+        if (ok && initial_lipschitz(t1, t3, A.dt2, l)) {
+            S.lipsch = l;
+            S.alpha = 1.0 / l;
+            S.lgood = l;
+        }
+        if (!ok) {
+            S.err = 1;
+            S.done = 1;
+        }
+    }
+    __syncthreads();
+}
 
 template <typename T, int DIM, int PROB>
 __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A) {
@@ -252,64 +329,7 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
         cp_commit();
     };
     bool geom_issued = false;
-    if (A.curvature_start) {
-        // initial step from the curvature along the first descent direction d (stored in
-        // the candidate buffer, which the first contact pass overwrites)
-        T* dbuf = A.lam2;
-        double t1 = 0.0, t3 = 0.0;
-        double a2[2] = {0.0, 0.0};
-        GRID_STRIDE(c, C) {
-            const T cc = ld4(A.nc + c).w;
-            const T d = first_descent<T>(cc, A.shift, c);
-            dbuf[c] = d;
-            a2[0] += (double)d * (double)d;
-            if (PROB == kViscous) {
-                const int sl = A.slot[c];
-                if (sl >= 0) {
-                    const T d2 = first_descent<T>(-cc, A.shift, sl);
-                    dbuf[sl] = d2;
-                    a2[0] += (double)d2 * (double)d2;
-                }
-            }
-        }
-        block_sum<2>(a2);
-        bool ok = G.exchange(a2[0], t1);
-        double wm[2] = {0.0, 0.0};
-        if (ok) GRID_STRIDE(p, A.na) {
-            T w0 = 0, w1 = 0, w2 = 0;
-            const int k0 = A.inc_ptr[p], n = A.inc_ptr[p + 1] - k0;
-            const IncWalk wk = inc_walk(lay, sizeof(T) / 4, p, k0);
-            for (int k = 0; k < n; ++k) {
-                const V4<T> e = ld_inc(A.inc, wk, k);
-                const int ci = idx_of(e.w);
-                T mu = __ldcg(dbuf + ci);
-                if (PROB == kViscous) {
-                    const int sl = A.slot[ci];
-                    if (sl >= 0) mu -= __ldcg(dbuf + sl);
-                }
-                w0 += mu * e.x;
-                w1 += mu * e.y;
-                if (DIM == 3) w2 += mu * e.z;
-            }
-            const double im = (double)A.invm[p];
-            wm[0] += im * ((double)w0 * w0 + (double)w1 * w1 + (double)w2 * w2);
-        }
-        block_sum<2>(wm);
-        if (ok) ok = G.exchange(wm[0], t3);
-        if (threadIdx.x == 0) {
-            double l;
-            if (ok && initial_lipschitz(t1, t3, A.dt2, l)) {
-                S.lipsch = l;
-                S.alpha = 1.0 / l;
-                S.lgood = l;
-            }
-            if (!ok) {
-                S.err = 1;
-                S.done = 1;
-            }
-        }
-        __syncthreads();
-    }
+    if (A.curvature_start) curvature_step<T, DIM, PROB>(A, C, lay, S, G);
     for (;;) {
         if (S.done) break;
         const double alpha = S.alpha;
@@ -375,15 +395,20 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
                     const int sl = (k % GC) * NT + tid;
                     const V4<T> nc = s_nc[sl];
                     // bodies below nin (obstacles) gathered as zeros: same sum as skipping them
-                    T qy = 0;
-                    qy += nc.x * g[0] + nc.y * g[1] + (DIM == 3 ? nc.z * g[2] : (T)0);
-                    qy -= nc.x * g[3] + nc.y * g[4] + (DIM == 3 ? nc.z * g[5] : (T)0);
-                    qy *= (T)A.dt2;
-                    mult_update_v<T>(A, c, qy, nc.w, s_l[sl], s_lp[sl], lnew, beta, use_prev, bt, alpha, s);
+                    V4<T> ui, uj;
+                    ui.x = g[0]; ui.y = g[1]; ui.z = g[2];
+                    uj.x = g[3]; uj.y = g[4]; uj.z = g[5];
+                    int sv = -1;
+                    T l2 = 0, q2 = 0, lp2 = 0;
                     if (PROB == kViscous) {
-                        const int sv = A.slot[c];
-                        if (sv >= 0) mult_update<T>(A, sv, -qy, -nc.w, lam, lprev, lnew, beta, use_prev, bt, alpha, s);
+                        sv = A.slot[c];
+                        if (sv >= 0) {
+                            l2 = lam[sv];
+                            if (use_prev) q2 = lprev[sv];
+                        }
                     }
+                    contact_update<T, DIM, PROB>(A, c, nc, ui, uj, s_l[sl], s_lp[sl], sv, l2, q2, &lp2, lnew, beta,
+                                                 use_prev, bt, alpha, s);
                 }
             };
             T g0[6], g1[6], g2[6];
@@ -533,6 +558,234 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
     if (blockIdx.x == 0 && threadIdx.x == 0) write_result(A.result, S);
 }
 
+// ------------------------------------------------------------------ resident form
+// Up to RC contacts and one body per thread of the grid: their records, multipliers and
+// velocities stay in registers for the whole solve, so a pass is its gathers (u(y) of a
+// contact's bodies, l+ of a body's contacts) and nothing else.  An iteration has one barrier
+// between the passes and one exchange of sums after them: the particle pass forms u(next y)
+// with the momentum of an accepted step, after a restart u(l+) itself is the next y.
+// Solves of up to 16 blocks with one contact a thread run as ONE cluster (CL): its barriers and
+// distributed shared memory take the place of 2 x ~5000 cycles of fences, stores and polls
+// through L2 per iteration.  What bounds either form is that chain of latencies.
+// Against the streaming form, microseconds per iteration: FP64 2k contacts 9.9 -> 4.7 (cluster),
+// 20k 13.8 -> 11.4, 133k 13.9 -> 11.4 (two contacts a thread); FP32 61k 12.9 -> 10.6, 451k 16.0 -> 15.7
+// (four a thread: the gathers' L2 traffic is the larger part there).
+template <bool CL>
+struct SphSync;
+template <>
+struct SphSync<false> {
+    using type = GridSums<true>;
+};
+template <>
+struct SphSync<true> {
+    using type = ClusterSums;
+};
+__device__ __forceinline__ void sync_init(GridSums<true>& G, double* slots, unsigned int* bar, bool stall) {
+    G = GridSums<true>{slots, gridDim.x, bar, 0u, stall};
+}
+__device__ __forceinline__ void sync_init(ClusterSums& G, double*, unsigned int*, bool) { G.par = 0; }
+
+template <typename T, int DIM, int PROB, int RC, bool CL>
+__global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArgs<T> A) {
+    __shared__ ApgdState S;
+    __shared__ double red[8][32];
+    __shared__ Momentum s_mo;
+    __shared__ NextStep s_ns;
+    constexpr int KB = sizeof(T) == 4 ? 6 : 4;  // incidence records loaded while the barrier waits
+    const int NT = blockDim.x, tid = threadIdx.x;
+    const int C = A.sizes->C;
+    const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
+    typename SphSync<CL>::type G;
+    sync_init(G, A.sums, A.bar, A.stall != 0 && blockIdx.x == 0);
+    if (tid == 0) state_init(S, A.alpha);
+    __syncthreads();
+    if (A.curvature_start) curvature_step<T, DIM, PROB>(A, C, lay, S, G);
+    const int base = (int)blockIdx.x * NT + tid, stride = (int)gridDim.x * NT;
+    // this thread's contacts
+    V4<T> nc[RC];
+    int2 ij[RC];
+    T lm[RC], lq[RC], ln[RC];
+    int sv[PROB == kViscous ? RC : 1];
+    T lm2[PROB == kViscous ? RC : 1], lq2[PROB == kViscous ? RC : 1], ln2[PROB == kViscous ? RC : 1];
+#pragma unroll
+    for (int r = 0; r < RC; ++r) {
+        const int c = base + r * stride;
+        ij[r] = make_int2(-1, -1);
+        nc[r].x = nc[r].y = nc[r].z = nc[r].w = (T)0;
+        lm[r] = lq[r] = ln[r] = (T)0;
+        if (c < C) {
+            nc[r] = ld4(A.nc + c);
+            ij[r] = A.cij[c];
+        }
+        if (PROB == kViscous) {
+            sv[r] = c < C ? A.slot[c] : -1;
+            lm2[r] = lq2[r] = ln2[r] = (T)0;
+        }
+    }
+    // this thread's body
+    const bool body = base < A.na;
+    const int k0 = body ? A.inc_ptr[base] : 0, cnt = body ? A.inc_ptr[base + 1] - k0 : 0;
+    const IncWalk wk = inc_walk(lay, sizeof(T) / 4, base, k0);
+    const T im = body ? A.invm[base] : (T)0;
+    T ul0 = 0, ul1 = 0, ul2 = 0, uy0 = 0, uy1 = 0, uy2 = 0;
+    for (;;) {
+        if (S.done) break;
+        const double alpha = S.alpha;
+        const bool bt = S.bt != 0, use_prev = S.use_prev != 0;
+        const T beta = (T)S.beta;
+        T* lnew = pick(S.in_, A.lam0, A.lam1, A.lam2);
+        const V4<T>* uY = pick4(S.jY, A.u0, A.u1, A.u2, A.u3);
+        V4<T>* uN = pick4(S.jN, A.u0, A.u1, A.u2, A.u3);
+        V4<T>* uYN = pick4(S.jYN, A.u0, A.u1, A.u2, A.u3);
+        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        // ---- contact pass
+        {
+            V4<T> gi[RC], gj[RC];
+#pragma unroll
+            for (int r = 0; r < RC; ++r) {
+                gi[r].x = gi[r].y = gi[r].z = gj[r].x = gj[r].y = gj[r].z = (T)0;
+                if (ij[r].x >= A.nin) gi[r] = ld4cg(uY + (ij[r].x - A.nin));
+                if (ij[r].y >= A.nin) gj[r] = ld4cg(uY + (ij[r].y - A.nin));
+            }
+#pragma unroll
+            for (int r = 0; r < RC; ++r) {
+                if (ij[r].y < 0) continue;
+                const int c = base + r * stride;
+                const int e = PROB == kViscous ? r : 0;
+                ln[r] = contact_update<T, DIM, PROB>(A, c, nc[r], gi[r], gj[r], lm[r], lq[r], PROB == kViscous ? sv[e] : -1,
+                                                     lm2[e], lq2[e], &ln2[e], lnew, beta, use_prev, bt, alpha, s);
+            }
+        }
+        G.arrive();
+        // while the barrier waits: what the decisions need, and the first incidence records
+        if (tid == 32) s_mo = prepare_momentum(S);
+        if (tid == 64) s_ns = prepare_step<T>(S, A.tol);
+        V4<T> e[KB];
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+            if (q < cnt) e[q] = ld_inc(A.inc, wk, q);
+        if (!G.wait()) {
+            if (tid == 0) {
+                S.err = 1;
+                S.done = 1;
+            }
+            break;
+        }
+        // the momentum was written after this block arrived: the cluster's wait does not order it
+        // (the grid's wait ends in a block barrier)
+        if (CL) __syncthreads();
+        const T bn_ = (T)s_mo.beta;
+        // ---- particle pass: w = B^T l+, u = M^-1 w, u(next y)
+        T n0 = 0, n1 = 0, n2 = 0, y0 = 0, y1 = 0, y2 = 0;
+        double sw = 0.0;
+        if (body) {
+            T w0 = 0, w1 = 0, w2 = 0;
+            for (int kb = 0; kb < cnt; kb += KB) {
+                T mu[KB];
+                if (kb > 0)
+#pragma unroll
+                    for (int q = 0; q < KB; ++q)
+                        if (kb + q < cnt) e[q] = ld_inc(A.inc, wk, kb + q);
+#pragma unroll
+                for (int q = 0; q < KB; ++q) {
+                    mu[q] = (T)0;
+                    if (kb + q < cnt) {
+                        const int ci = idx_of(e[q].w);
+                        mu[q] = __ldcg(lnew + ci);
+                        if (PROB == kViscous) {
+                            const int sl = A.slot[ci];
+                            if (sl >= 0) mu[q] -= __ldcg(lnew + sl);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int q = 0; q < KB; ++q) {
+                    if (kb + q >= cnt) continue;
+                    w0 += mu[q] * e[q].x;
+                    w1 += mu[q] * e[q].y;
+                    if (DIM == 3) w2 += mu[q] * e[q].z;
+                }
+            }
+            n0 = mul_rn(im, w0);
+            n1 = mul_rn(im, w1);
+            n2 = mul_rn(im, w2);
+            st4(uN + base, n0, n1, n2);
+            // w.u gives F(l+) for the reference's test (FP64); FP32 tests the curvature
+            if (sizeof(T) == 8) {
+                sw += (double)w0 * (double)n0 + (double)w1 * (double)n1 + (double)w2 * (double)n2;
+            } else {
+                const double d0 = (double)n0 - (double)uy0, d1 = (double)n1 - (double)uy1, d2 = (double)n2 - (double)uy2;
+                sw += (d0 * d0 + d1 * d1 + d2 * d2) / (double)im;
+            }
+            y0 = n0;
+            y1 = n1;
+            y2 = n2;
+            if (bn_ != (T)0) {
+                y0 = fma_rn(bn_, add_rn(n0, -ul0), n0);
+                y1 = fma_rn(bn_, add_rn(n1, -ul1), n1);
+                y2 = fma_rn(bn_, add_rn(n2, -ul2), n2);
+            }
+            st4(uYN + base, y0, y1, y2);
+        }
+        // ---- the sums (FP32 reads |d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2 and the curvature), the decisions
+        if (sizeof(T) == 4) {
+            s[0] = s[1];
+            s[1] = s[4];
+            s[2] = s[5];
+            s[3] = s[6];
+            s[4] = sw;
+            s[5] = s[6] = 0.0;
+        }
+        s[7] = sizeof(T) == 4 ? 0.0 : sw;
+        double t[8];
+        const bool ok = G.template sums<8>(s, red, t);
+        if (tid < 32) {
+            // the two square roots side by side
+            const double sq = sqrt(tid == 0 ? t[sizeof(T) == 4 ? 1 : 4] : t[3]);
+            const double sq1 = __shfl_sync(0xffffffffu, sq, 1);
+            if (tid == 0) {
+                if (!ok) {
+                    S.err = 1;
+                    S.done = 1;
+                } else {
+                    decide_momentum<T>(S, t, bt, A.dynamic, s_mo);
+                    NextStep ns = s_ns;
+                    ns.step = sq;
+                    ns.tol = A.tol;
+                    if (sizeof(T) == 4) {
+                        const double floor32 = 4.0 * 1.1920929e-7 * sq1;
+                        if (floor32 > ns.tol) ns.tol = floor32;
+                    }
+                    const double last = t[sizeof(T) == 4 ? 4 : 7];
+                    decide_step<T>(S, last, last, A.dt2, A.dynamic, A.max_ite, ns);
+                    if (!S.bt) reuse_buffers(S);
+                }
+            }
+        }
+        __syncthreads();
+        if (!S.bt) {
+#pragma unroll
+            for (int r = 0; r < RC; ++r) {
+                lq[r] = lm[r];
+                lm[r] = ln[r];
+                if (PROB == kViscous) {
+                    lq2[r] = lm2[r];
+                    lm2[r] = ln2[r];
+                }
+            }
+            ul0 = n0;
+            ul1 = n1;
+            ul2 = n2;
+            uy0 = S.restart ? n0 : y0;
+            uy1 = S.restart ? n1 : y1;
+            uy2 = S.restart ? n2 : y2;
+        }
+    }
+    __syncthreads();
+    if (blockIdx.x == 0 && tid == 0) write_result(A.result, S);
+    G.finish();
+}
+
 // ------------------------------------------------------------------ packing
 __global__ void k_pack_cij(const int* ci, const int* cj, int2* cij, const Sizes* sizes) {
     GRID_STRIDE(c, sizes->C) { cij[c] = make_int2(ci[c], cj[c]); }
@@ -648,6 +901,10 @@ int blocks(long long n) {
     return (int)(b < 16 * kSMs ? b : 16 * kSMs);
 }
 
+// contacts a thread of the resident form can hold
+template <typename T>
+constexpr int kResidentContacts = sizeof(T) == 4 ? 4 : 2;
+
 template <typename T, int DIM, int PROB>
 void set_sph_smem() {
     static bool done = false;  // per instantiation; the attribute is per function and process
@@ -670,8 +927,68 @@ int max_blocks_sph() {
     return std::min(per_sm * sms, kSumMaxBlocks);
 }
 
+// the resident kernel as one cluster of n CTAs, where the device can hold one
 template <typename T, int DIM, int PROB>
-cudaError_t launch_t(SphArgs<T>& A, int nblocks, cudaStream_t s) {
+bool launch_cluster(SphArgs<T>& A, int n, cudaStream_t s, cudaError_t& e) {
+    static std::atomic<int> able[5];  // per log2 n: 0 not asked yet, 1 yes, 2 no
+    int lg = 0;
+    while ((1 << lg) < n) ++lg;
+    const auto kernel = k_apgd_sph_res<T, DIM, PROB, 1, true>;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1 << lg);  // blocks past the last contact and body only take part in the barriers
+    cfg.blockDim = dim3(SphShape<T>::threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1 << lg;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int a = able[lg].load(std::memory_order_relaxed);
+    if (a == 0) {
+        int fit = 0;
+        const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0;
+        if (!ok) cudaGetLastError();
+        a = ok ? 1 : 2;
+        able[lg].store(a, std::memory_order_relaxed);
+    }
+    if (a != 1) return false;
+    g_sph_launches += 1;
+    e = cudaLaunchKernelEx(&cfg, kernel, A);
+    return true;
+}
+
+template <typename T, int DIM, int PROB, int RC>
+cudaError_t launch_res(SphArgs<T>& A, int nblocks, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nblocks);
+    cfg.blockDim = dim3(SphShape<T>::threads);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    g_sph_launches += 1;
+    return cudaLaunchKernelEx(&cfg, k_apgd_sph_res<T, DIM, PROB, RC, false>, A);
+}
+
+// n_contacts: the host's count (the one in A.sizes)
+template <typename T, int DIM, int PROB>
+cudaError_t launch_t(SphArgs<T>& A, long long n_contacts, int nblocks, cudaStream_t s) {
+    const long long threads = (long long)nblocks * SphShape<T>::threads;
+    if (A.na <= threads && n_contacts <= kResidentContacts<T> * threads) {
+        cudaError_t e;
+        if (n_contacts <= threads) {
+            // the wait-limit test needs the barrier that has a limit
+            if (nblocks <= 16 && !A.stall && launch_cluster<T, DIM, PROB>(A, nblocks, s, e)) return e;
+            return launch_res<T, DIM, PROB, 1>(A, nblocks, s);
+        }
+        if (n_contacts <= 2 * threads) return launch_res<T, DIM, PROB, 2>(A, nblocks, s);
+        if constexpr (kResidentContacts<T> == 4) return launch_res<T, DIM, PROB, 4>(A, nblocks, s);
+    }
     set_sph_smem<T, DIM, PROB>();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nblocks);
@@ -705,7 +1022,7 @@ int apgd_sph_max_blocks(int problem, int dim, bool fp32) {
 
 template <typename T>
 cudaError_t launch_apgd_sph(int nin, int na, int dim, int problem, const ApgdSettings& st, SphSolve<T>& sb,
-                            const Sizes* sizes, int nblocks, cudaStream_t s) {
+                            const Sizes* sizes, long long n_contacts, int nblocks, cudaStream_t s) {
     SphArgs<T> A;
     A.nin = nin;
     A.na = na;
@@ -736,15 +1053,15 @@ cudaError_t launch_apgd_sph(int nin, int na, int dim, int problem, const ApgdSet
     A.curvature_start = st.curvature_start;
     A.stall = st.stall;
 #define LA(D, P) \
-    if (dim == D && problem == P) return launch_t<T, D, P>(A, nblocks, s);
+    if (dim == D && problem == P) return launch_t<T, D, P>(A, n_contacts, nblocks, s);
     LA(2, 0) LA(2, 2) LA(3, 0) LA(3, 2)
 #undef LA
     return cudaErrorInvalidValue;
 }
 template cudaError_t launch_apgd_sph<double>(int, int, int, int, const ApgdSettings&, SphSolve<double>&, const Sizes*,
-                                             int, cudaStream_t);
+                                             long long, int, cudaStream_t);
 template cudaError_t launch_apgd_sph<float>(int, int, int, int, const ApgdSettings&, SphSolve<float>&, const Sizes*,
-                                            int, cudaStream_t);
+                                            long long, int, cudaStream_t);
 
 void launch_pack_cij(const int* ci, const int* cj, int2* cij, const Sizes* sizes, long long c_cap, cudaStream_t s) {
     k_pack_cij<<<blocks(c_cap), 256, 0, s>>>(ci, cj, cij, sizes);
@@ -1061,7 +1378,8 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
         set_global_error2("scopi_gpu_apgd_noalloc: cudaMemsetAsync: ", cudaGetErrorString(e));
         return SCOPI_GPU_ECUDA;
     }
-    e = dim == 3 ? launch_t<double, 3, kNoFriction>(A, (int)nb, s) : launch_t<double, 2, kNoFriction>(A, (int)nb, s);
+    e = dim == 3 ? launch_t<double, 3, kNoFriction>(A, C, (int)nb, s)
+                 : launch_t<double, 2, kNoFriction>(A, C, (int)nb, s);
     if (e != cudaSuccess) {
         set_global_error2("scopi_gpu_apgd_noalloc: launch: ", cudaGetErrorString(e));
         return SCOPI_GPU_ECUDA;

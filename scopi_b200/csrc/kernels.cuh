@@ -324,7 +324,7 @@ int apgd_sph_max_blocks(int problem, int dim, bool fp32);
 int apgd_sph_threads(bool fp32);  // threads per block of the torque-free kernel
 template <typename T>
 cudaError_t launch_apgd_sph(int nin, int na, int dim, int problem, const ApgdSettings& st, SphSolve<T>& sb,
-                            const Sizes* sizes, int nblocks, cudaStream_t s);
+                            const Sizes* sizes, long long n_contacts, int nblocks, cudaStream_t s);
 void launch_pack_cij(const int* ci, const int* cj, int2* cij, const Sizes* sizes, long long c_cap, cudaStream_t s);
 template <typename T>
 void launch_pack_nc(const double* bn, const double* cvec, V4<T>* nc, const Sizes* sizes, long long c_cap,

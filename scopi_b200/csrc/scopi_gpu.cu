@@ -959,7 +959,7 @@ struct scopi_gpu_handle {
         if (e != cudaSuccess) return cuda_fail(e, "APGD barrier words");
         const int nb = nblocks_for(maxb, std::max<long long>(h_sizes->C, na), apgd_sph_threads(sizeof(T) == 4));
         cudaMemsetAsync(sb.sums, 0xff, (size_t)kSumBytesPerBlock * nb, stream);
-        e = launch_apgd_sph<T>(nin, na, P.dim, P.problem, st, sb, d_sizes_cur, nb, stream);
+        e = launch_apgd_sph<T>(nin, na, P.dim, P.problem, st, sb, d_sizes_cur, h_sizes->C, nb, stream);
         if (e != cudaSuccess) return cuda_fail(e, "APGD launch");
         cudaMemcpyAsync(h_result, d_result, sizeof(ApgdResult), cudaMemcpyDeviceToHost, stream);
         e = cudaStreamSynchronize(stream);
