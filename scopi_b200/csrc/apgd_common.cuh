@@ -3,6 +3,8 @@
 #pragma once
 #include <math.h>
 
+#include <atomic>
+
 #include "kernels.cuh"
 
 namespace scopi_gpu {
@@ -216,6 +218,8 @@ __device__ __forceinline__ double sum_group_order(double (&x)[5][NP]) {
     return s;
 }
 
+// (The kernels with one exchange per iteration reduce the contact sums over the warps while the
+// barrier between the passes waits, and one more value after the particle pass.)
 // Block partials of NP per-thread values, first half: per-warp sums into sh[k][warp].  After a
 // block barrier, warp 0 finishes with block_sums_tree (tree over warps) or
 // block_sums_in_order (warps one after the other); lane l gets value l >> SumShift<NP>.
@@ -224,6 +228,10 @@ __device__ __forceinline__ void warp_sums(double* v, double (*sh)[32]) {
     const int lane = threadIdx.x & 31;
     const double x = multi_reduce<NP>(v);
     if ((lane & ((1 << SumShift<NP>::value) - 1)) == 0) sh[lane >> SumShift<NP>::value][threadIdx.x >> 5] = x;
+}
+__device__ __forceinline__ void warp_sum_to(double v, double* sh) {
+    const double x = multi_reduce<1>(&v);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
 }
 template <int NP>
 __device__ __forceinline__ double block_sums_tree(const double (*sh)[32]) {
@@ -302,6 +310,10 @@ struct GridSums {
     template <int NP>
     __device__ __forceinline__ void publish(double* v, double (*sh)[32]) {
         warp_sums<NP>(v, sh);
+        publish_warps<NP>(sh);
+    }
+    template <int NP>
+    __device__ __forceinline__ void publish_warps(double (*sh)[32]) {
         __syncthreads();
         if (threadIdx.x < 32) {
             if (TREE) {
@@ -343,26 +355,38 @@ struct GridSums {
         __syncthreads();
         return s_ok != 0;
     }
-    // publish and collect in one, in lane order (all threads, at least 160; the totals and the
-    // status are warp 0's).  Five warps collect a group of blocks each, so that no thread holds
-    // more than NP of the values.
+    // publish and collect in one, from the per-warp sums in sh (all threads, at least 160; the
+    // totals and the status are warp 0's).  Five warps collect a group of blocks each, so that no thread holds more than NP of
+    // the values.
     template <int NP>
-    __device__ __forceinline__ bool sums(double* v, double (*sh)[32], double* t) {
+    __device__ __forceinline__ bool sums(double (*sh)[32], double* t) {
         __shared__ double raw[5][NP][32];
         __shared__ int bad;
         if (threadIdx.x == 0) bad = 0;
-        publish<NP>(v, sh);
+        publish_warps<NP>(sh);
         const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
         if (w < 5) {
             double x[1][NP];
             const bool ok = sum_collect<NP, 1>(slots, nb, m, bar, x, 32u * w);
+            if (TREE) {
 #pragma unroll
-            for (int k = 0; k < NP; ++k) raw[w][k][lane] = x[0][k];
+                for (int k = 0; k < NP; ++k) raw[w][k][lane] = x[0][k];
+            } else {
+                const double z = multi_reduce<NP>(x[0]);
+                if ((lane & ((1 << SumShift<NP>::value) - 1)) == 0) raw[w][lane >> SumShift<NP>::value][0] = z;
+            }
             if (!ok && lane == 0) bad = 1;
         }
         ++m;
         __syncthreads();
-        if (w == 0) {
+        if (w == 0 && !TREE) {
+            double z = 0.0;
+            if (lane < NP)
+#pragma unroll
+                for (int g = 0; g < 5; ++g) z += raw[g][lane][0];
+#pragma unroll
+            for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, z, k);
+        } else if (w == 0) {
             double y[NP];
 #pragma unroll
             for (int k = 0; k < NP; ++k) {
@@ -475,8 +499,9 @@ __device__ __forceinline__ void overflow_cascade(double& lipsch, double& alpha, 
 }
 
 // The same for a launch of one cluster (up to 16 CTAs): hardware cluster barriers, block sums
-// read through distributed shared memory, in the order of GridSums<true>.  Nothing can be
+// read through distributed shared memory, in the orders of GridSums<TREE>.  Nothing can be
 // missing from such a barrier (the CTAs of a cluster run together), so there is no limit.
+template <bool TREE>
 struct ClusterSums {
     int par;
 
@@ -496,32 +521,33 @@ struct ClusterSums {
     // a slot is written again two exchanges later, when every CTA has passed the barrier of the
     // exchange between, which it enters after its reads
     template <int NP>
-    __device__ __forceinline__ void read(const double* own, double (&x)[5][NP]) {
+    __device__ __forceinline__ void read(const double* own, double (&x)[1][NP]) {
         const unsigned int lane = threadIdx.x & 31;
 #pragma unroll
-        for (int w = 0; w < 5; ++w)
-#pragma unroll
-            for (int k = 0; k < NP; ++k) x[w][k] = 0.0;
-        if (lane < gridDim.x)
-#pragma unroll
-            for (int k = 0; k < NP; ++k) x[0][k] = remote(own + k, lane);
+        for (int k = 0; k < NP; ++k) x[0][k] = lane < gridDim.x ? remote(own + k, lane) : 0.0;
     }
     template <int NP>
-    __device__ __forceinline__ bool sums(double* v, double (*sh)[32], double* t) {
+    __device__ __forceinline__ bool sums(double (*sh)[32], double* t) {
         __shared__ double part[2][8];
-        warp_sums<NP>(v, sh);
         __syncthreads();
         constexpr int sf = SumShift<NP>::value;
         if (threadIdx.x < 32) {
-            const double x = block_sums_tree<NP>(sh);
-            if ((threadIdx.x & ((1 << sf) - 1)) == 0) part[par][threadIdx.x >> sf] = x;
+            if (TREE) {
+                const double x = block_sums_tree<NP>(sh);
+                if ((threadIdx.x & ((1 << sf) - 1)) == 0) part[par][threadIdx.x >> sf] = x;
+            } else if (threadIdx.x < NP) {
+                double x = 0.0;
+                for (int w = 0; w < (int)(blockDim.x >> 5); ++w) x += sh[threadIdx.x][w];
+                part[par][threadIdx.x] = x;
+            }
         }
         arrive();
         wait();
         if (threadIdx.x < 32) {
-            double x[5][NP];
+            double x[1][NP];
             read<NP>(part[par], x);
-            const double y = sum_lane_order<NP>(x);
+            // one group of at most 16 blocks: both orders are its tree
+            const double y = multi_reduce<NP>(x[0]);
 #pragma unroll
             for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, y, k << sf);
         }
@@ -535,9 +561,9 @@ struct ClusterSums {
         arrive();
         wait();
         if (threadIdx.x < 32) {
-            double x[5][1];
+            double x[1][1];
             read<1>(&one[par], x);
-            const double y = sum_group_order<1>(x);
+            const double y = multi_reduce<1>(x[0]);
             if (threadIdx.x == 0) s_t = y;
         }
         par ^= 1;
@@ -551,6 +577,60 @@ struct ClusterSums {
         wait();
     }
 };
+
+template <bool CL, bool TREE>
+struct SyncOf;
+template <bool TREE>
+struct SyncOf<false, TREE> {
+    using type = GridSums<TREE>;
+};
+template <bool TREE>
+struct SyncOf<true, TREE> {
+    using type = ClusterSums<TREE>;
+};
+template <bool TREE>
+__device__ __forceinline__ void sync_init(GridSums<TREE>& G, double* slots, unsigned int* bar, bool stall) {
+    G = GridSums<TREE>{slots, gridDim.x, bar, 0u, stall};
+}
+template <bool TREE>
+__device__ __forceinline__ void sync_init(ClusterSums<TREE>& G, double*, unsigned int*, bool) {
+    G.par = 0;
+}
+
+// Host: whether the device can run `kernel` as one cluster of 2^lg CTAs (asked once, remembered in
+// `able`: 0 not asked, 1 yes, 2 no).
+inline cudaLaunchConfig_t cluster_config(int n, int threads, cudaStream_t s, cudaLaunchAttribute* attr) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = n;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+}
+template <typename K>
+bool cluster_fits(K kernel, const cudaLaunchConfig_t& cfg, std::atomic<int>& able) {
+    int a = able.load(std::memory_order_relaxed);
+    if (a == 0) {
+        int fit = 0;
+        const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0;
+        if (!ok) cudaGetLastError();
+        a = ok ? 1 : 2;
+        able.store(a, std::memory_order_relaxed);
+    }
+    return a == 1;
+}
+inline int log2_up(int n) {
+    int lg = 0;
+    while ((1 << lg) < n) ++lg;
+    return lg;
+}
+constexpr int kMaxCluster = 16;
 
 // Loop-carried scalars of the iteration (block-uniform) live in shared memory and are
 // updated by thread 0, so the registers go to the two passes.
@@ -587,11 +667,14 @@ __device__ __forceinline__ void state_init(ApgdState& S, double alpha) {
 struct Momentum {
     double theta1, beta;
 };
+// FUSED: th^2 + theta1 rounded once; the two roundings differ in a handful of iterations, and each
+// solve keeps the one its results have always had
+template <bool FUSED = false>
 __device__ __forceinline__ Momentum prepare_momentum(const ApgdState& S) {
-    const double th = S.theta;
+    const double th = S.theta, t2 = mul_rn(th, th);
     Momentum m;
-    m.theta1 = 0.5 * (th * sqrt(4 + th * th) - th * th);
-    m.beta = th * (1 - th) / (th * th + m.theta1);
+    m.theta1 = 0.5 * fma_rn(th, sqrt(add_rn(4.0, t2)), -t2);
+    m.beta = mul_rn(th, add_rn(1.0, -th)) / (FUSED ? fma_rn(th, th, m.theta1) : add_rn(t2, m.theta1));
     return m;
 }
 // after the contact pass: momentum for the next y if this candidate is accepted
@@ -627,6 +710,17 @@ __device__ __forceinline__ NextStep prepare_step(const ApgdState& S, double tol)
     n.alpha_bt = 1. / (S.lipsch * 2);
     n.lip_ok = S.lipsch * 0.97;
     n.alpha_ok = 1. / n.lip_ok;
+    return n;
+}
+// the same once the sums are known: sq = sqrt(|l+ - l|^2), sq1 = sqrt(|l+|^2)
+template <typename T>
+__device__ __forceinline__ NextStep step_of(NextStep n, double tol, double sq, double sq1) {
+    n.step = sq;
+    n.tol = tol;
+    if (sizeof(T) == 4) {
+        const double floor32 = 4.0 * 1.1920929e-7 * sq1;
+        if (floor32 > n.tol) n.tol = floor32;
+    }
     return n;
 }
 // after the particle pass: backtrack or accept (apgd.hpp:172-221); wu = w.u (FP64), curv =

@@ -17,6 +17,9 @@
 // 164 -> 66, FP64 44k 34.2 -> 18.3; 2D FP64 1.7k 22.9 -> 9.3.  The iterates are the same bits.
 // The gathers are plain loads (the acquire of the barrier before a pass empties the L1, so they
 // are fresh): against L2-only loads FP32 679k 65.7 -> 56.2, FP64 44k 16.1 -> 15.3.
+// One barrier and one exchange of sums an iteration (instead of two exchanges), small solves in one
+// cluster: FP32 679k 56.2 -> 49.3, 3k 9.4 -> 8.8; FP64 2D 1.7k 8.2 -> 5.4, 39k 10.8 -> 9.6; FP64 3D
+// 118 contacts 9.9 -> 7.5, 44k 15.3 -> 15.5, 133k 19.8 -> 21.2 (there the registers are full).
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -73,7 +76,6 @@ __device__ __forceinline__ void fld4(const dvec4* p, double* o) {
     put4(o, q[0]);
     put4(o + 2, q[1]);
 }
-__device__ __forceinline__ void fld4cg(const float4* p, float* o) { put4(o, __ldcg(p)); }
 __device__ __forceinline__ void fld4cg(const dvec4* p, double* o) {
     const double2* q = reinterpret_cast<const double2*>(p);
     put4(o, __ldcg(q));
@@ -87,7 +89,6 @@ __device__ __forceinline__ void fst4(dvec4* p, const double* v) {
 }
 __device__ __forceinline__ void fld4(const float2* p, float* o) { const float2 v = *p; o[0] = v.x; o[1] = v.y; }
 __device__ __forceinline__ void fld4(const double2* p, double* o) { put4(o, *p); }
-__device__ __forceinline__ void fld4cg(const float2* p, float* o) { const float2 v = __ldcg(p); o[0] = v.x; o[1] = v.y; }
 __device__ __forceinline__ void fld4cg(const double2* p, double* o) { put4(o, __ldcg(p)); }
 __device__ __forceinline__ void fst4(float2* p, const float* v) { *p = make_float2(v[0], v[1]); }
 __device__ __forceinline__ void fst4(double2* p, const double* v) { *p = make_double2(v[0], v[1]); }
@@ -257,20 +258,29 @@ __device__ __forceinline__ void contact_row(const T* r, const T* ui, const T* uj
     if (DIM == 2 && !SUMS) qout[2] = (T)0;
 }
 
-// w = A^T l+ of one body over its n incidences, KB records and multipliers in flight
+// Incidence records [kb, kb + KB) of a body with n of them.
 template <typename T, int DIM, int KB>
-__device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, const Lam<T, DIM>* lnew, int n, T* w) {
+__device__ __forceinline__ void load_incs(const Q4<T>* inc, const IncWalk& wk, int kb, int n,
+                                          T (&e)[KB][FricShape<T, DIM>::inc]) {
+    using F = FricShape<T, DIM>;
+#pragma unroll
+    for (int q = 0; q < KB; ++q)
+        if (kb + q < n)
+#pragma unroll
+            for (int v = 0; v < F::ni; ++v)
+                put4(e[q] + v * F::per, inc[wk.first + (long long)(kb + q) * wk.rs + v * wk.vs]);
+}
+// w = A^T l+ of one body over its n incidences, KB records and multipliers in flight; e holds the
+// first KB records
+template <typename T, int DIM, int KB>
+__device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, const Lam<T, DIM>* lnew, int n, T* w,
+                                           T (&e)[KB][FricShape<T, DIM>::inc]) {
     using F = FricShape<T, DIM>;
 #pragma unroll
     for (int d = 0; d < F::dof; ++d) w[d] = (T)0;
     for (int kb = 0; kb < n; kb += KB) {
-        T e[KB][F::inc], l[KB][4];
-#pragma unroll
-        for (int q = 0; q < KB; ++q)
-            if (kb + q < n)
-#pragma unroll
-                for (int v = 0; v < F::ni; ++v)
-                    put4(e[q] + v * F::per, inc[wk.first + (long long)(kb + q) * wk.rs + v * wk.vs]);
+        T l[KB][4];
+        if (kb > 0) load_incs<T, DIM, KB>(inc, wk, kb, n, e);
 #pragma unroll
         for (int q = 0; q < KB; ++q)
             if (kb + q < n) fld4(lnew + (fidx(e[q][F::at_idx]) & 0x7fffffffu), l[q]);
@@ -291,6 +301,12 @@ __device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, 
             }
         }
     }
+}
+template <typename T, int DIM, int KB>
+__device__ __forceinline__ void body_force(const Q4<T>* inc, const IncWalk& wk, const Lam<T, DIM>* lnew, int n, T* w) {
+    T e[KB][FricShape<T, DIM>::inc];
+    load_incs<T, DIM, KB>(inc, wk, 0, n, e);
+    body_force<T, DIM, KB>(inc, wk, lnew, n, w, e);
 }
 template <typename T, int DIM>
 __device__ __forceinline__ void body_velocity(const T* im, const T* w, T* u) {
@@ -332,19 +348,22 @@ constexpr long long kMaxBacktracks = 4000;
 template <typename T>
 struct FricThreads {
     static constexpr int value = sizeof(T) == 4 ? 512 : 256;
-    static constexpr int kb = sizeof(T) == 4 ? 3 : 3;
+    static constexpr int kb = sizeof(T) == 4 ? 3 : 4;
 };
 
-template <typename T, int DIM>
+template <typename T, int DIM, bool CL>
 __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs<T> A) {
     using F = FricShape<T, DIM>;
     constexpr int KB = FricThreads<T>::kb;
     __shared__ ApgdState S;
     __shared__ double red[8][32];
+    __shared__ Momentum s_mo;
+    __shared__ NextStep s_ns;
     const int tid = threadIdx.x;
     const int C = A.sizes->C;
     const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
-    GridSums<false> G{A.sums, gridDim.x, A.bar, 0u, A.stall != 0 && blockIdx.x == 0};
+    typename SyncOf<CL, false>::type G;
+    sync_init(G, A.sums, A.bar, A.stall != 0 && blockIdx.x == 0);
     if (tid == 0) state_init(S, A.alpha);
     __syncthreads();
     if (A.curvature_start) {
@@ -401,6 +420,17 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
         __syncthreads();
     }
     const long long S_ = (long long)gridDim.x * blockDim.x, base = (long long)blockIdx.x * blockDim.x + tid;
+    // of the first contact and (where there are registers for them) the first body, for the whole solve
+    const int2 ij0 = base < C ? A.cij[base] : make_int2(0, 0);
+    constexpr bool keep = sizeof(T) == 4 || CL;
+    int kb0 = 0, n0 = 0;
+    IncWalk wk0{};
+    auto body0 = [&] {
+        kb0 = base < A.na ? A.inc_ptr[base] : 0;
+        n0 = base < A.na ? A.inc_ptr[base + 1] - kb0 : 0;
+        wk0 = inc_walk(lay, F::ni, base, kb0);
+    };
+    if (keep) body0();
     for (;;) {
         if (S.done) break;
         const double alpha = S.alpha;
@@ -410,9 +440,13 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
         const Lam<T, DIM>* lprev = pick_lam<T, DIM>(A, S.ip);
         Lam<T, DIM>* lnew = pick_lam<T, DIM>(A, S.in_);
         const V4<T>* uY = pick_u(A, S.jY);
+        const V4<T>* uL = pick_u(A, S.jL);
+        V4<T>* uN = pick_u(A, S.jN);
+        V4<T>* uYN = pick_u(A, S.jYN);
+        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+        // ---- contact pass
         {
-            double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-            int2 ij = base < C ? A.cij[base] : make_int2(0, 0);
+            int2 ij = ij0;
 #pragma unroll 1
             for (long long c = base; c < C; c += S_) {
                 const int2 me = ij;
@@ -429,69 +463,84 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
                                     A.shift ? A.shift + 3 * c : nullptr, lo, s);
                 fst4(lnew + c, lo);
             }
-            constexpr int NS = sizeof(T) == 4 ? 4 : 8;
-            G.template publish<NS>(s, red);
-            if (tid < 32) {
-                const Momentum mo = prepare_momentum(S);
-                double t[NS];
-                const bool ok = G.template collect<NS>(t);
-                if (tid == 0) {
-                    if (!ok) {
-                        S.err = 1;
-                        S.done = 1;
-                    }
-                    decide_momentum<T>(S, t, bt, A.dynamic, mo);
+        }
+        G.arrive();
+        // while the barrier waits: the warps' contact sums, what the decisions need, and the first
+        // incidence records
+        if (!CL) warp_sums<8>(s, red);
+        if (tid == 32) s_mo = prepare_momentum(S);
+        if (tid == 64) s_ns = prepare_step<T>(S, A.tol);
+        T e[KB][F::inc];
+        if (!keep) body0();
+        load_incs<T, DIM, KB>(A.inc, wk0, 0, n0, e);
+        if (!G.wait()) {
+            if (tid == 0) {
+                S.err = 1;
+                S.done = 1;
+            }
+            break;
+        }
+        if (CL) __syncthreads();  // the momentum was written after the arrival
+        const T bn_ = (T)s_mo.beta;
+        // ---- particle pass
+        double sw = 0.0;
+#pragma unroll 1
+        for (long long p = base; p < A.na; p += S_) {
+            T im[4], ul[F::dof], uy[F::dof], w[F::dof], u[F::dof];
+            int n = n0;
+            IncWalk wk = wk0;
+            if (p != base) {
+                const int kb = A.inc_ptr[p];
+                n = A.inc_ptr[p + 1] - kb;
+                wk = inc_walk(lay, F::ni, p, kb);
+                load_incs<T, DIM, KB>(A.inc, wk, 0, n, e);
+            }
+            fld4(A.invm + p, im);
+            if (bn_ != (T)0) load_u<T, DIM>(uL, p, ul);
+            if (sizeof(T) == 4) load_u<T, DIM>(uY, p, uy);
+            body_force<T, DIM, KB>(A.inc, wk, lnew, n, w, e);
+            body_velocity<T, DIM>(im, w, u);
+            store_u<T, DIM>(uN, p, u);
+            // w.u gives F(l+) for the reference's test (FP64); FP32 tests the curvature
+            if (sizeof(T) == 8)
+                sw += body_wu<T, DIM>(w, u);
+            else
+                sw += body_curvature<T, DIM>(im, u, uy);
+            if (bn_ != (T)0) {
+#pragma unroll
+                for (int d = 0; d < F::dof; ++d) u[d] = fma_rn(bn_, add_rn(u[d], -ul[d]), u[d]);
+            }
+            store_u<T, DIM>(uYN, p, u);
+        }
+        // ---- the sums, the decisions
+        if (CL) {
+            s[sizeof(T) == 4 ? 4 : 7] = sw;
+            warp_sums<8>(s, red);  // a cluster's barrier does not leave the time
+        } else {
+            warp_sum_to(sw, red[sizeof(T) == 4 ? 4 : 7]);
+        }
+        double t[8];
+        const bool ok = G.template sums<8>(red, t);
+        if (tid < 32) {
+            // the two square roots side by side
+            const double sq = sqrt(tid == 0 ? t[sizeof(T) == 4 ? 1 : 4] : t[3]);
+            const double sq1 = __shfl_sync(0xffffffffu, sq, 1);
+            if (tid == 0) {
+                if (!ok) {
+                    S.err = 1;
+                    S.done = 1;
+                } else {
+                    decide_momentum<T>(S, t, bt, A.dynamic, s_mo);
+                    const double last = t[sizeof(T) == 4 ? 4 : 7];
+                    decide_step<T>(S, last, last, A.dt2, A.dynamic, A.max_ite, step_of<T>(s_ns, A.tol, sq, sq1),
+                                   kMaxBacktracks);
+                    if (!S.bt) reuse_buffers(S);
                 }
             }
-            G.next();
         }
         __syncthreads();
-        if (S.err) break;
-        {
-            const V4<T>* uL = pick_u(A, S.jL);
-            V4<T>* uN = pick_u(A, S.jN);
-            V4<T>* uYN = pick_u(A, S.jYN);
-            const T bn_ = (T)S.beta_n;
-            double s[1] = {0.0};
-#pragma unroll 1
-            for (long long p = base; p < A.na; p += S_) {
-                const int k0 = A.inc_ptr[p], k1 = A.inc_ptr[p + 1];
-                T im[4], ul[F::dof], uy[F::dof], w[F::dof], u[F::dof];
-                fld4(A.invm + p, im);
-                if (bn_ != (T)0) load_u<T, DIM>(uL, p, ul);
-                if (sizeof(T) == 4) load_u<T, DIM>(uY, p, uy);
-                body_force<T, DIM, KB>(A.inc, inc_walk(lay, F::ni, p, k0), lnew, k1 - k0, w);
-                body_velocity<T, DIM>(im, w, u);
-                store_u<T, DIM>(uN, p, u);
-                // w.u gives F(l+) for the reference's test (FP64); FP32 tests the curvature
-                if (sizeof(T) == 8)
-                    s[0] += body_wu<T, DIM>(w, u);
-                else
-                    s[0] += body_curvature<T, DIM>(im, u, uy);
-                if (bn_ != (T)0) {
-#pragma unroll
-                    for (int d = 0; d < F::dof; ++d) u[d] = fma_rn(bn_, add_rn(u[d], -ul[d]), u[d]);
-                }
-                store_u<T, DIM>(uYN, p, u);
-            }
-            G.template publish<1>(s, red);
-            if (tid < 32) {
-                const NextStep ns = prepare_step<T>(S, A.tol);
-                double t[1];
-                const bool ok = G.template collect<1>(t);
-                if (tid == 0) {
-                    if (!ok) {
-                        S.err = 1;
-                        S.done = 1;
-                    } else {
-                        decide_step<T>(S, t[0], t[0], A.dt2, A.dynamic, A.max_ite, ns, kMaxBacktracks);
-                    }
-                }
-            }
-            G.next();
-            __syncthreads();
-        }
     }
+    __syncthreads();
     // the result, in the layouts of the other kernels (every thread its own contacts and bodies)
     const Lam<T, DIM>* lres = pick_lam<T, DIM>(A, S.il);
     const V4<T>* ures = pick_u(A, S.jL);
@@ -515,6 +564,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
             }
         }
     if (blockIdx.x == 0 && tid == 0) write_result(A.result, S);
+    G.finish();
 }
 
 // ------------------------------------------------------------------ batched scenes (FP64)
@@ -940,17 +990,26 @@ int blocks(long long n) {
 
 template <typename T, int DIM>
 cudaError_t launch_fric_t(FricArgs<T>& A, int nblocks, cudaStream_t s) {
+    g_fric_launches += 1;
+    cudaLaunchAttribute attr[1];
+    if (nblocks <= kMaxCluster && !A.stall) {
+        // small solves as one cluster (the wait-limit test needs the barrier that has a limit);
+        // blocks past the last contact and body only take part in the barriers
+        static std::atomic<int> able[5];
+        const int lg = log2_up(nblocks);
+        const cudaLaunchConfig_t cfg = cluster_config(1 << lg, FricThreads<T>::value, s, attr);
+        if (cluster_fits(k_apgd_fric<T, DIM, true>, cfg, able[lg]))
+            return cudaLaunchKernelEx(&cfg, k_apgd_fric<T, DIM, true>, A);
+    }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nblocks);
     cfg.blockDim = dim3(FricThreads<T>::value);
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    g_fric_launches += 1;
-    return cudaLaunchKernelEx(&cfg, k_apgd_fric<T, DIM>, A);
+    return cudaLaunchKernelEx(&cfg, k_apgd_fric<T, DIM, false>, A);
 }
 
 }  // namespace

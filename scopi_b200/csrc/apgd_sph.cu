@@ -12,7 +12,6 @@
 //   per body    : u(y) gathered once (u(y_next) = u(l+) + beta (u(l+) - u(l)) is formed in
 //                 the particle pass, the restart test being reduced after the first barrier).
 #include <algorithm>
-#include <atomic>
 #include <cstdio>
 #include <mutex>
 
@@ -568,21 +567,6 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
 // Against the streaming form, microseconds per iteration: FP64 2k contacts 9.9 -> 4.7 (cluster),
 // 20k 13.8 -> 11.4, 133k 13.9 -> 11.4 (two contacts a thread); FP32 61k 12.9 -> 10.6, 451k 16.0 -> 15.7
 // (four a thread: the gathers' L2 traffic is the larger part there).
-template <bool CL>
-struct SphSync;
-template <>
-struct SphSync<false> {
-    using type = GridSums<true>;
-};
-template <>
-struct SphSync<true> {
-    using type = ClusterSums;
-};
-__device__ __forceinline__ void sync_init(GridSums<true>& G, double* slots, unsigned int* bar, bool stall) {
-    G = GridSums<true>{slots, gridDim.x, bar, 0u, stall};
-}
-__device__ __forceinline__ void sync_init(ClusterSums& G, double*, unsigned int*, bool) { G.par = 0; }
-
 template <typename T, int DIM, int PROB, int RC, bool CL>
 __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArgs<T> A) {
     __shared__ ApgdState S;
@@ -593,7 +577,7 @@ __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArg
     const int NT = blockDim.x, tid = threadIdx.x;
     const int C = A.sizes->C;
     const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
-    typename SphSync<CL>::type G;
+    typename SyncOf<CL, true>::type G;
     sync_init(G, A.sums, A.bar, A.stall != 0 && blockIdx.x == 0);
     if (tid == 0) state_init(S, A.alpha);
     __syncthreads();
@@ -633,8 +617,6 @@ __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArg
         const T beta = (T)S.beta;
         T* lnew = pick(S.in_, A.lam0, A.lam1, A.lam2);
         const V4<T>* uY = pick4(S.jY, A.u0, A.u1, A.u2, A.u3);
-        V4<T>* uN = pick4(S.jN, A.u0, A.u1, A.u2, A.u3);
-        V4<T>* uYN = pick4(S.jYN, A.u0, A.u1, A.u2, A.u3);
         double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         // ---- contact pass
         {
@@ -655,7 +637,16 @@ __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArg
             }
         }
         G.arrive();
-        // while the barrier waits: what the decisions need, and the first incidence records
+        // while the barrier waits: the warps' contact sums (FP32 reads |d|^2, |l+ - l|^2, g.(l+ - l) and
+        // |l+|^2), what the decisions need, and the first incidence records
+        if (sizeof(T) == 4) {
+            s[0] = s[1];
+            s[1] = s[4];
+            s[2] = s[5];
+            s[3] = s[6];
+            s[4] = s[5] = s[6] = 0.0;
+        }
+        if (!CL) warp_sums<8>(s, red);
         if (tid == 32) s_mo = prepare_momentum(S);
         if (tid == 64) s_ns = prepare_step<T>(S, A.tol);
         V4<T> e[KB];
@@ -674,6 +665,8 @@ __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArg
         if (CL) __syncthreads();
         const T bn_ = (T)s_mo.beta;
         // ---- particle pass: w = B^T l+, u = M^-1 w, u(next y)
+        V4<T>* uN = pick4(S.jN, A.u0, A.u1, A.u2, A.u3);
+        V4<T>* uYN = pick4(S.jYN, A.u0, A.u1, A.u2, A.u3);
         T n0 = 0, n1 = 0, n2 = 0, y0 = 0, y1 = 0, y2 = 0;
         double sw = 0.0;
         if (body) {
@@ -725,18 +718,15 @@ __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArg
             }
             st4(uYN + base, y0, y1, y2);
         }
-        // ---- the sums (FP32 reads |d|^2, |l+ - l|^2, g.(l+ - l), |l+|^2 and the curvature), the decisions
-        if (sizeof(T) == 4) {
-            s[0] = s[1];
-            s[1] = s[4];
-            s[2] = s[5];
-            s[3] = s[6];
-            s[4] = sw;
-            s[5] = s[6] = 0.0;
+        // ---- the sums, the decisions
+        if (CL) {
+            s[sizeof(T) == 4 ? 4 : 7] = sw;
+            warp_sums<8>(s, red);  // a cluster's barrier does not leave the time
+        } else {
+            warp_sum_to(sw, red[sizeof(T) == 4 ? 4 : 7]);
         }
-        s[7] = sizeof(T) == 4 ? 0.0 : sw;
         double t[8];
-        const bool ok = G.template sums<8>(s, red, t);
+        const bool ok = G.template sums<8>(red, t);
         if (tid < 32) {
             // the two square roots side by side
             const double sq = sqrt(tid == 0 ? t[sizeof(T) == 4 ? 1 : 4] : t[3]);
@@ -747,15 +737,8 @@ __global__ void __launch_bounds__(SphShape<T>::threads, 1) k_apgd_sph_res(SphArg
                     S.done = 1;
                 } else {
                     decide_momentum<T>(S, t, bt, A.dynamic, s_mo);
-                    NextStep ns = s_ns;
-                    ns.step = sq;
-                    ns.tol = A.tol;
-                    if (sizeof(T) == 4) {
-                        const double floor32 = 4.0 * 1.1920929e-7 * sq1;
-                        if (floor32 > ns.tol) ns.tol = floor32;
-                    }
                     const double last = t[sizeof(T) == 4 ? 4 : 7];
-                    decide_step<T>(S, last, last, A.dt2, A.dynamic, A.max_ite, ns);
+                    decide_step<T>(S, last, last, A.dt2, A.dynamic, A.max_ite, step_of<T>(s_ns, A.tol, sq, sq1));
                     if (!S.bt) reuse_buffers(S);
                 }
             }
@@ -928,31 +911,13 @@ int max_blocks_sph() {
 // the resident kernel as one cluster of n CTAs, where the device can hold one
 template <typename T, int DIM, int PROB>
 bool launch_cluster(SphArgs<T>& A, int n, cudaStream_t s, cudaError_t& e) {
-    static std::atomic<int> able[5];  // per log2 n: 0 not asked yet, 1 yes, 2 no
-    int lg = 0;
-    while ((1 << lg) < n) ++lg;
+    static std::atomic<int> able[5];
+    const int lg = log2_up(n);
     const auto kernel = k_apgd_sph_res<T, DIM, PROB, 1, true>;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1 << lg);  // blocks past the last contact and body only take part in the barriers
-    cfg.blockDim = dim3(SphShape<T>::threads);
-    cfg.stream = s;
     cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1 << lg;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    int a = able[lg].load(std::memory_order_relaxed);
-    if (a == 0) {
-        int fit = 0;
-        const bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&fit, kernel, &cfg) == cudaSuccess && fit > 0;
-        if (!ok) cudaGetLastError();
-        a = ok ? 1 : 2;
-        able[lg].store(a, std::memory_order_relaxed);
-    }
-    if (a != 1) return false;
+    // blocks past the last contact and body only take part in the barriers
+    const cudaLaunchConfig_t cfg = cluster_config(1 << lg, SphShape<T>::threads, s, attr);
+    if (!cluster_fits(kernel, cfg, able[lg])) return false;
     g_sph_launches += 1;
     e = cudaLaunchKernelEx(&cfg, kernel, A);
     return true;
@@ -981,7 +946,7 @@ cudaError_t launch_t(SphArgs<T>& A, long long n_contacts, int nblocks, cudaStrea
         cudaError_t e;
         if (n_contacts <= threads) {
             // the wait-limit test needs the barrier that has a limit
-            if (nblocks <= 16 && !A.stall && launch_cluster<T, DIM, PROB>(A, nblocks, s, e)) return e;
+            if (nblocks <= kMaxCluster && !A.stall && launch_cluster<T, DIM, PROB>(A, nblocks, s, e)) return e;
             return launch_res<T, DIM, PROB, 1>(A, nblocks, s);
         }
         if (n_contacts <= 2 * threads) return launch_res<T, DIM, PROB, 2>(A, nblocks, s);
