@@ -417,8 +417,8 @@ struct BatchSolve {
     int curvature_start;
 };
 
-// Batched scenes of a 6-dof problem, FP64: one CTA per scene over the scene
-// ranges of launch_batch_ranges; the multipliers (3 per contact) and u (6 per active body)
+// Batched Viscous scenes on the 6-dof rows, FP64: one CTA per scene over the scene ranges of
+// launch_batch_ranges; the multipliers (one or two per contact) and u (6 per active body)
 // of every scene end in lam_out / u_out, its statistics in stats[scene].
 struct Batch6Scenes {
     int n_scenes;
