@@ -597,8 +597,14 @@ __device__ __forceinline__ void sync_init(ClusterSums<TREE>& G, double*, unsigne
     G.par = 0;
 }
 
-// Host: whether the device can run `kernel` as one cluster of 2^lg CTAs (asked once, remembered in
-// `able`: 0 not asked, 1 yes, 2 no).
+// Host: whether the current device can run `kernel` as one cluster of 2^lg CTAs (0 not asked, 1 yes,
+// 2 no).  The permission for clusters of more than 8 belongs to the kernel on one device, so each
+// device of the process is asked for itself; devices past kMaxDevices take the cooperative launch.
+constexpr int kMaxDevices = 64;
+constexpr int kMaxCluster = 16;
+struct ClusterAble {
+    std::atomic<int> at[kMaxDevices][5];  // [device][lg], lg <= 4
+};
 inline cudaLaunchConfig_t cluster_config(int n, int threads, cudaStream_t s, cudaLaunchAttribute* attr) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(n);
@@ -613,7 +619,10 @@ inline cudaLaunchConfig_t cluster_config(int n, int threads, cudaStream_t s, cud
     return cfg;
 }
 template <typename K>
-bool cluster_fits(K kernel, const cudaLaunchConfig_t& cfg, std::atomic<int>& able) {
+bool cluster_fits(K kernel, const cudaLaunchConfig_t& cfg, ClusterAble& known, int lg) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
+    std::atomic<int>& able = known.at[dev][lg];
     int a = able.load(std::memory_order_relaxed);
     if (a == 0) {
         int fit = 0;
@@ -630,7 +639,6 @@ inline int log2_up(int n) {
     while ((1 << lg) < n) ++lg;
     return lg;
 }
-constexpr int kMaxCluster = 16;
 
 // Loop-carried scalars of the iteration (block-uniform) live in shared memory and are
 // updated by thread 0, so the registers go to the two passes.

@@ -995,10 +995,10 @@ cudaError_t launch_fric_t(FricArgs<T>& A, int nblocks, cudaStream_t s) {
     if (nblocks <= kMaxCluster && !A.stall) {
         // small solves as one cluster (the wait-limit test needs the barrier that has a limit);
         // blocks past the last contact and body only take part in the barriers
-        static std::atomic<int> able[5];
+        static ClusterAble able;
         const int lg = log2_up(nblocks);
         const cudaLaunchConfig_t cfg = cluster_config(1 << lg, FricThreads<T>::value, s, attr);
-        if (cluster_fits(k_apgd_fric<T, DIM, true>, cfg, able[lg]))
+        if (cluster_fits(k_apgd_fric<T, DIM, true>, cfg, able, lg))
             return cudaLaunchKernelEx(&cfg, k_apgd_fric<T, DIM, true>, A);
     }
     cudaLaunchConfig_t cfg = {};

@@ -968,13 +968,13 @@ int max_blocks_sph() {
 // the resident kernel as one cluster of n CTAs, where the device can hold one
 template <typename T, int DIM, int PROB>
 bool launch_cluster(SphArgs<T>& A, int n, cudaStream_t s, cudaError_t& e) {
-    static std::atomic<int> able[5];
+    static ClusterAble able;
     const int lg = log2_up(n);
     const auto kernel = k_apgd_sph_res<T, DIM, PROB, 1, true>;
     cudaLaunchAttribute attr[1];
     // blocks past the last contact and body only take part in the barriers
     const cudaLaunchConfig_t cfg = cluster_config(1 << lg, SphShape<T>::threads, s, attr);
-    if (!cluster_fits(kernel, cfg, able[lg])) return false;
+    if (!cluster_fits(kernel, cfg, able, lg)) return false;
     g_sph_launches += 1;
     e = cudaLaunchKernelEx(&cfg, kernel, A);
     return true;
@@ -1172,7 +1172,6 @@ constexpr size_t kNoAllocBytes = align_up(kOffFlag + sizeof(unsigned int));
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 
-constexpr int kMaxDevices = 64;
 unsigned char* g_noalloc_dev[kMaxDevices] = {};
 std::mutex g_noalloc_mutex;
 

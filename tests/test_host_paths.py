@@ -1,0 +1,83 @@
+"""Host code of the engine against a CUDA runtime without a GPU (tests/cpp/fake_cudart.cpp): two
+devices, device memory that is host memory, kernels that do nothing, failures on request.
+
+Each test runs in a process of its own, where the runtime of the test takes the place of the
+real one before the library is loaded.
+"""
+import os
+import shutil
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+GXX = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else (shutil.which("g++") or "g++")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+PRELUDE = """
+import ctypes as C
+import sys
+fake = C.CDLL({so!r}, mode=C.RTLD_GLOBAL)
+fake.fake_get.restype = C.c_longlong
+get = lambda w: fake.fake_get(w.encode())
+put = lambda w, v: fake.fake_set(w.encode(), C.c_longlong(v))
+sys.path[:0] = [{root!r}, {tests!r}]
+import numpy as np
+import pytest
+from scopi_b200 import FP64, FRICTION, MIXED, NOFRICTION, VISCOUS, ScopiBatch, ScopiSolver, _abi, configs
+from scopi_b200.solver import ScopiGPUError
+lib = _abi.load()
+
+def rows(fn):
+    return ScopiSolver(configs.box_3d(count=fn.pop("count", 60)), vap=1, dmax=0.0045, **fn)
+"""
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    if not os.path.exists(os.path.join(CUDA, "include", "cuda_runtime_api.h")):
+        pytest.skip("CUDA headers unavailable")
+    from scopi_b200 import _abi, build
+    if not os.path.exists(_abi.LIB_PATH):
+        build.build()
+    out = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run([GXX, "-O1", "-std=c++17", "-shared", "-fPIC", "-I", os.path.join(CUDA, "include"),
+                    os.path.join(ROOT, "tests", "cpp", "fake_cudart.cpp"), "-o", out], check=True)
+
+    def run(body):
+        code = PRELUDE.format(so=out, root=ROOT, tests=os.path.join(ROOT, "tests")) + textwrap.dedent(body)
+        r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
+        assert r.returncode == 0, r.stdout + r.stderr
+        return r.stdout
+
+    return run
+
+
+def test_friction_clusters_on_a_second_device(fake):
+    """9 to 16 blocks run as a cluster of 16, which every device has to allow for itself."""
+    fake("""
+    put("contacts", 4000)
+    for dev in (0, 1, 0):
+        for precision in (FP64, MIXED):
+            s = rows(dict(problem=FRICTION, mu=0.3, precision=precision, device=dev))
+            before = get("cluster_launches")
+            s.step(1e-3, 1)
+            assert get("cluster_launches") > before
+            s.close()
+    """)
+
+
+def test_sphere_clusters_on_a_second_device(fake):
+    fake("""
+    put("contacts", 16 * 512)
+    for dev in (0, 1, 0):
+        for problem in (NOFRICTION, VISCOUS):
+            for precision in (FP64, MIXED):
+                s = rows(dict(problem=problem, precision=precision, device=dev))
+                before = get("cluster_launches")
+                s.step(1e-3, 1)
+                assert get("cluster_launches") > before
+                s.close()
+    """)
