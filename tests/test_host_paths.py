@@ -81,3 +81,17 @@ def test_sphere_clusters_on_a_second_device(fake):
                 assert get("cluster_launches") > before
                 s.close()
     """)
+
+
+def test_streaming_kernel_on_a_second_device(fake):
+    """More contacts than the grid's registers hold: the form whose shared memory needs permission."""
+    fake("""
+    for dev in (0, 1):
+        for problem in (NOFRICTION, VISCOUS):
+            for precision, contacts in ((FP64, 160_000), (MIXED, 500_000), (MIXED, 2_000_000)):
+                put("contacts", contacts)
+                s = rows(dict(problem=problem, precision=precision, device=dev))
+                s.step(1e-3, 1)
+                assert s.stats()["contacts"] == contacts
+                s.close()
+    """)
