@@ -3,8 +3,6 @@
 #pragma once
 #include <math.h>
 
-#include <atomic>
-
 #include "kernels.cuh"
 
 namespace scopi_gpu {
@@ -600,7 +598,6 @@ __device__ __forceinline__ void sync_init(ClusterSums<TREE>& G, double*, unsigne
 // Host: whether the current device can run `kernel` as one cluster of 2^lg CTAs (0 not asked, 1 yes,
 // 2 no).  The permission for clusters of more than 8 belongs to the kernel on one device, so each
 // device of the process is asked for itself; devices past kMaxDevices take the cooperative launch.
-constexpr int kMaxDevices = 64;
 constexpr int kMaxCluster = 16;
 struct ClusterAble {
     std::atomic<int> at[kMaxDevices][5];  // [device][lg], lg <= 4

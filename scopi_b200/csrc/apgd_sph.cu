@@ -940,20 +940,17 @@ bool past_l2(double contacts, double bodies) {
     return sizeof(T) == 4 && contacts * (3 * sizeof(V4<T>) + sizeof(int2) + 3 * sizeof(T)) + bodies * 4 * sizeof(V4<T>) > kL2Bytes;
 }
 
-// the streaming form's shared memory, allowed once per device (it belongs to the kernel on one device)
+// the streaming form's shared memory
 template <typename T, int DIM, int PROB>
 void set_sph_smem() {
     static std::atomic<bool> done[kMaxDevices];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return;
-    const bool known = dev >= 0 && dev < kMaxDevices;
-    if (known && done[dev].load(std::memory_order_acquire)) return;
-    cudaFuncSetAttribute(k_apgd_sph<T, DIM, PROB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)SphOcc<T>::smem);
-    if constexpr (sizeof(T) == 4)
-        cudaFuncSetAttribute(k_apgd_sph<T, DIM, PROB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    once_per_device(done, [] {
+        cudaFuncSetAttribute(k_apgd_sph<T, DIM, PROB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)SphOcc<T>::smem);
-    if (known) done[dev].store(true, std::memory_order_release);
+        if constexpr (sizeof(T) == 4)
+            cudaFuncSetAttribute(k_apgd_sph<T, DIM, PROB, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)SphOcc<T>::smem);
+    });
 }
 
 template <typename T, int DIM, int PROB>

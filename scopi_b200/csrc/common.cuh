@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 namespace scopi_gpu {
 
 constexpr int kSMs = 148;          // B200: 2 dies x 74 SMs
@@ -76,6 +78,18 @@ struct Contacts {
 enum Problem { kNoFriction = 0, kFriction = 1, kViscous = 2, kViscousFriction = 4 };
 
 __host__ __device__ inline int ceil_div(long long a, long long b) { return (int)((a + b - 1) / b); }
+
+// A kernel's attributes belong to the kernel on one device: `set` runs once for each device that a
+// call finds current (every time past kMaxDevices).
+constexpr int kMaxDevices = 64;
+template <typename F>
+void once_per_device(std::atomic<bool> (&done)[kMaxDevices], F set) {
+    int dev = -1;
+    const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kMaxDevices;
+    if (known && done[dev].load(std::memory_order_acquire)) return;
+    set();
+    if (known) done[dev].store(true, std::memory_order_release);
+}
 
 // grid-stride helper
 #define GRID_STRIDE(i, n) for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < (long long)(n); \

@@ -432,11 +432,10 @@ void launch_se_pairs(int dim, const Bodies& b, Contacts& c, const Sizes* sizes, 
         g_se_launches += 1;
         return;
     }
-    static bool configured = false;
-    if (!configured) {
+    static std::atomic<bool> configured[kMaxDevices];
+    once_per_device(configured, [] {
         cudaFuncSetAttribute(k_se_start, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SeShared));
-        configured = true;
-    }
+    });
     k_se_start<<<grid, kSeThreads, sizeof(SeShared), s>>>(b, c, sizes, need, u0);
     cudaMemsetAsync(counter, 0, sizeof(int), s);
     k_se_solve<<<4 * kSMs, 128, 0, s>>>(b, c, sizes, need, u0, counter);

@@ -17,7 +17,9 @@ namespace {
 int g_dev = 0, g_error = 0;
 long long g_mallocs = 0, g_fail_malloc = -1;  // allocations so far; number of good ones until one fails
 int g_contacts = 0;                           // what detection "finds"
+int g_superellipsoids = 0;                    // what an upload's census counts
 int g_refuse_clusters = 0;
+long long g_refused = 0;                      // launches that broke a rule
 long long g_cluster_launches = 0, g_launches = 0;
 std::map<void*, size_t> g_blocks;
 size_t g_bytes = 0;
@@ -29,10 +31,15 @@ cudaError_t fail(cudaError_t e) {
     return e;
 }
 cudaError_t launch(const void* f, void** args, size_t smem) {
-    if (smem > 48 * 1024 && g_smem[{g_dev, f}] < (int)smem) return fail(cudaErrorInvalidValue);
+    if (smem > 48 * 1024 && g_smem[{g_dev, f}] < (int)smem) {
+        ++g_refused;
+        return fail(cudaErrorInvalidValue);
+    }
     ++g_launches;
     // k_sizes(totals, sizes, cap): the number of contacts is the struct's first field
     if (g_names[f].find("k_sizes") != std::string::npos) **(int**)args[1] = g_contacts;
+    // k_shape_census(shape, worm, n, nin, dim, out)
+    if (g_names[f].find("k_shape_census") != std::string::npos) **(int**)args[5] = g_superellipsoids;
     return cudaSuccess;
 }
 }  // namespace
@@ -43,12 +50,14 @@ void fake_set(const char* what, long long v) {
     if (w == "device") g_dev = (int)v;
     if (w == "fail_malloc") g_fail_malloc = v;
     if (w == "contacts") g_contacts = (int)v;
+    if (w == "superellipsoids") g_superellipsoids = (int)v;
     if (w == "refuse_clusters") g_refuse_clusters = (int)v;
 }
 long long fake_get(const char* what) {
     const std::string w = what;
     if (w == "mallocs") return g_mallocs;
     if (w == "bytes") return (long long)g_bytes;
+    if (w == "refused") return g_refused;
     if (w == "launches") return g_launches;
     if (w == "cluster_launches") return g_cluster_launches;
     return -1;

@@ -95,3 +95,15 @@ def test_streaming_kernel_on_a_second_device(fake):
                 assert s.stats()["contacts"] == contacts
                 s.close()
     """)
+
+
+def test_superellipsoid_start_kernel_on_a_second_device(fake):
+    fake("""
+    put("contacts", 100)
+    put("superellipsoids", 20)
+    for dev in (0, 1):
+        s = ScopiSolver(configs.se_pile(20, side=3), vap=1, dmax=0.004, problem=FRICTION, mu=0.3, device=dev)
+        s.step(5e-4, 1)
+        assert get("launches") > 0 and get("refused") == 0
+        s.close()
+    """)
