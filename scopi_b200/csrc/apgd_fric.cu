@@ -990,7 +990,6 @@ int blocks(long long n) {
 
 template <typename T, int DIM>
 cudaError_t launch_fric_t(FricArgs<T>& A, int nblocks, cudaStream_t s) {
-    g_fric_launches += 1;
     cudaLaunchAttribute attr[1];
     if (nblocks <= kMaxCluster && !A.stall) {
         // small solves as one cluster (the wait-limit test needs the barrier that has a limit);
@@ -998,9 +997,15 @@ cudaError_t launch_fric_t(FricArgs<T>& A, int nblocks, cudaStream_t s) {
         static ClusterAble able;
         const int lg = log2_up(nblocks);
         const cudaLaunchConfig_t cfg = cluster_config(1 << lg, FricThreads<T>::value, s, attr);
-        if (cluster_fits(k_apgd_fric<T, DIM, true>, cfg, able, lg))
-            return cudaLaunchKernelEx(&cfg, k_apgd_fric<T, DIM, true>, A);
+        if (cluster_fits(k_apgd_fric<T, DIM, true>, cfg, able, lg)) {
+            if (cudaLaunchKernelEx(&cfg, k_apgd_fric<T, DIM, true>, A) == cudaSuccess) {
+                g_fric_launches += 1;
+                return cudaSuccess;
+            }
+            cudaGetLastError();  // refused (nothing ran): the cooperative form
+        }
     }
+    g_fric_launches += 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(nblocks);
     cfg.blockDim = dim3(FricThreads<T>::value);

@@ -965,9 +965,9 @@ int max_blocks_sph() {
     return std::min(per_sm * sms, kSumMaxBlocks);
 }
 
-// the resident kernel as one cluster of n CTAs, where the device can hold one
+// the resident kernel as one cluster of n CTAs, where the device can hold one and takes the launch
 template <typename T, int DIM, int PROB>
-bool launch_cluster(SphArgs<T>& A, int n, cudaStream_t s, cudaError_t& e) {
+bool launch_cluster(SphArgs<T>& A, int n, cudaStream_t s) {
     static ClusterAble able;
     const int lg = log2_up(n);
     const auto kernel = k_apgd_sph_res<T, DIM, PROB, 1, true>;
@@ -975,8 +975,11 @@ bool launch_cluster(SphArgs<T>& A, int n, cudaStream_t s, cudaError_t& e) {
     // blocks past the last contact and body only take part in the barriers
     const cudaLaunchConfig_t cfg = cluster_config(1 << lg, SphShape<T>::threads, s, attr);
     if (!cluster_fits(kernel, cfg, able, lg)) return false;
+    if (cudaLaunchKernelEx(&cfg, kernel, A) != cudaSuccess) {
+        cudaGetLastError();  // nothing ran: the caller takes the cooperative form
+        return false;
+    }
     g_sph_launches += 1;
-    e = cudaLaunchKernelEx(&cfg, kernel, A);
     return true;
 }
 
@@ -1000,10 +1003,9 @@ template <typename T, int DIM, int PROB>
 cudaError_t launch_t(SphArgs<T>& A, long long n_contacts, int nblocks, cudaStream_t s) {
     const long long threads = (long long)nblocks * SphShape<T>::threads;
     if (A.na <= threads && n_contacts <= kResidentContacts<T> * threads) {
-        cudaError_t e;
         if (n_contacts <= threads) {
             // the wait-limit test needs the barrier that has a limit
-            if (nblocks <= kMaxCluster && !A.stall && launch_cluster<T, DIM, PROB>(A, nblocks, s, e)) return e;
+            if (nblocks <= kMaxCluster && !A.stall && launch_cluster<T, DIM, PROB>(A, nblocks, s)) return cudaSuccess;
             return launch_res<T, DIM, PROB, 1>(A, nblocks, s);
         }
         if (n_contacts <= 2 * threads) return launch_res<T, DIM, PROB, 2>(A, nblocks, s);

@@ -107,3 +107,16 @@ def test_superellipsoid_start_kernel_on_a_second_device(fake):
         assert get("launches") > 0 and get("refused") == 0
         s.close()
     """)
+
+
+def test_refused_cluster_launch_takes_the_cooperative_form(fake):
+    fake("""
+    put("refuse_clusters", 1)
+    put("contacts", 2000)
+    for problem in (FRICTION, NOFRICTION, VISCOUS):
+        for precision in (FP64, MIXED):
+            s = rows(dict(problem=problem, precision=precision))
+            s.step(1e-3, 1)
+            assert s.stats()["contacts"] == 2000 and get("cluster_launches") == 0
+            s.close()
+    """)
