@@ -620,8 +620,18 @@ struct scopi_gpu_handle {
         return 0;
     }
 
-    // Buffers whose size follows the number of bodies.
+    // Buffers whose size follows the number of bodies.  A failure leaves the handle without
+    // particles (n = 0) until an upload succeeds.
     int alloc_bodies(int n_, int nin_, long long obs_cap = -1) {
+        const int rc = alloc_bodies_(n_, nin_, obs_cap);
+        if (rc) drop_bodies();
+        return rc;
+    }
+    void drop_bodies() {
+        body_mem.release();
+        n = nin = na = 0;
+    }
+    int alloc_bodies_(int n_, int nin_, long long obs_cap) {
         body_mem.release();
         n = n_;
         nin = nin_;
@@ -693,11 +703,29 @@ struct scopi_gpu_handle {
         return mixed() ? alloc_fric<float>(fric_mem, fb32) : alloc_fric<double>(fric_mem, fb64);
     }
 
-    // Buffers whose size follows the contact capacity.
+    // Buffers whose size follows the contact capacity.  A failure leaves none (c_cap = 0), and the
+    // next call that needs them allocates again.
     int alloc_contacts(long long cap) {
+        has_old = false;
+        last_lambda = nullptr;
+        cudaMemsetAsync(d_sizes_cur, 0, sizeof(Sizes), stream);
+        cudaMemsetAsync(d_sizes_old, 0, sizeof(Sizes), stream);
+        const int rc = alloc_contacts_(cap);
+        if (rc) {
+            cap_mem.release();
+            fric_mem.release();
+            fb64 = fb32 = FricBuffers{};
+            c_cap = 0;
+        }
+        return rc;
+    }
+    // the contact buffers of a fresh container (or after a failed growth)
+    int ensure_contacts() {
+        return c_cap > 0 ? 0 : alloc_contacts(std::max<long long>(8192, 6LL * na + 2LL * nin * 64));
+    }
+    int alloc_contacts_(long long cap) {
         cap_mem.release();
         c_cap = cap;
-        has_old = false;
         const long long M = cap * mult_per_contact();
         cudaError_t e;
 #define A(p, c) \
@@ -743,8 +771,6 @@ struct scopi_gpu_handle {
             A(d_nc32, cap) A(d_incv32, inc_slots())
         }
 #undef A
-        cudaMemsetAsync(d_sizes_cur, 0, sizeof(Sizes), stream);
-        cudaMemsetAsync(d_sizes_old, 0, sizeof(Sizes), stream);
         return 0;
     }
 
@@ -1616,12 +1642,14 @@ static int32_t upload_particles(scopi_gpu_handle* h, const scopi_gpu_particles* 
         int rc = h->alloc_bodies(n, nin, obs_cap);
         if (rc) return rc;
         if (h->c_cap == 0) {
-            rc = h->alloc_contacts(std::max<long long>(8192, 6LL * (n - nin) + 2LL * nin * 64));
-            if (rc) return rc;
+            rc = h->ensure_contacts();
         } else {
             h->has_old = false;
             rc = h->alloc_fric_set();
-            if (rc) return rc;
+        }
+        if (rc) {
+            h->drop_bodies();
+            return rc;
         }
     }
     cudaStream_t s = h->stream;
@@ -1745,6 +1773,7 @@ int32_t scopi_gpu_run(scopi_gpu_handle* h, double dt, int64_t total_it, int64_t 
     if (h->n == 0) return h->fail(SCOPI_GPU_EINVAL, "no particles");
     cudaSetDevice(h->dev);
     int status = 0;
+    if (int rc = h->ensure_contacts()) return rc;
     for (int64_t it = initial_iter; it < total_it; ++it) {
         int rc = h->batch ? h->step_batch(dt) : h->step(dt);
         if (rc < 0) return rc;
@@ -1757,7 +1786,8 @@ int32_t scopi_gpu_detect(scopi_gpu_handle* h, int64_t* nout) {
     if (!h) return SCOPI_GPU_EINVAL;
     if (h->n == 0) return h->fail(SCOPI_GPU_EINVAL, "no particles");
     cudaSetDevice(h->dev);
-    int rc = h->detect_and_assemble(0.0, false);
+    int rc = h->ensure_contacts();
+    if (!rc) rc = h->detect_and_assemble(0.0, false);
     if (rc) return rc;
     cudaMemcpyAsync(h->h_sizes, h->d_sizes_cur, sizeof(Sizes), cudaMemcpyDeviceToHost, h->stream);
     cudaError_t e = cudaStreamSynchronize(h->stream);
@@ -1889,6 +1919,7 @@ int32_t scopi_gpu_set_contacts(scopi_gpu_handle* h, int64_t n, const int64_t* ci
         int rc = h->alloc_contacts(std::max<long long>((long long)(1.3 * (double)n) + 1024, 2 * h->c_cap));
         if (rc) return rc;
     }
+    if (int rc = h->ensure_contacts()) return rc;
     cudaError_t e = cudaSuccess;
     if (n > 0) {
         e = cudaMemcpy(h->old.ci, i32.data(), n * sizeof(int), cudaMemcpyHostToDevice);

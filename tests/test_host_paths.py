@@ -120,3 +120,83 @@ def test_refused_cluster_launch_takes_the_cooperative_form(fake):
             assert s.stats()["contacts"] == 2000 and get("cluster_launches") == 0
             s.close()
     """)
+
+
+@pytest.mark.parametrize("problem,precision", [("FRICTION", "FP64"), ("FRICTION", "MIXED"), ("NOFRICTION", "MIXED")])
+def test_upload_retried_after_a_failed_allocation(fake, problem, precision):
+    """Whichever allocation of an upload fails, the handle has no particles until the next one,
+    which allocates everything; the first upload of a handle and one of another size."""
+    fake(f"""
+    kw = dict(problem={problem}, precision={precision}, vap=1, dmax=0.0045, mu=0.3)
+    put("contacts", 100)
+    small, large = configs.box_3d(count=30), configs.box_3d(count=60)
+
+    def attempt(k, first):
+        s = ScopiSolver(large if first else small, **kw)
+        if not first:
+            s.step(1e-3, 1)
+        else:
+            h = C.c_void_p()
+            assert lib.scopi_gpu_create(C.byref(s._params), C.byref(h)) == 0
+            s._h, s._created = h, True
+        before = get("mallocs")
+        put("fail_malloc", k)
+        try:
+            s.upload(large)
+            failed = False
+        except ScopiGPUError:
+            failed = True
+        put("fail_malloc", -1)
+        if failed:
+            with pytest.raises(ScopiGPUError, match="no particles"):
+                s.step(1e-3, 1)
+            s.upload(large)
+        s.step(1e-3, 1)
+        got = get("bytes"), get("mallocs") - before
+        s.close()
+        return failed, got
+
+    for first in (True, False):
+        _, (whole, count) = attempt(-1, first)
+        assert count > 10
+        for k in range(count):
+            failed, (held, _) = attempt(k, first)
+            assert failed and held == whole, (k, held, whole)
+    """)
+
+
+@pytest.mark.parametrize("problem,precision", [("FRICTION", "FP64"), ("NOFRICTION", "MIXED"), ("VISCOUS", "FP64")])
+def test_step_retried_after_a_failed_growth(fake, problem, precision):
+    """The contact buffers grow inside a step: after a failure the multipliers and the old list are
+    gone, the bodies are not, and the next step allocates again."""
+    fake(f"""
+    kw = dict(problem={problem}, precision={precision}, vap=1, dmax=0.0045, mu=0.3)
+    pa = configs.box_3d(count=30)
+
+    def attempt(k):
+        s = ScopiSolver(pa, **kw)
+        put("contacts", 100)
+        s.step(1e-3, 1)
+        put("contacts", 20000)
+        before = get("mallocs")
+        put("fail_malloc", k)
+        try:
+            s.step(1e-3, 1)
+            failed = False
+        except ScopiGPUError:
+            failed = True
+        put("fail_malloc", -1)
+        if failed:
+            assert len(s.lagrange_multiplier()) == 0 and len(s.current_contacts()["i"]) == 0
+            assert np.array_equal(s.download(pa.copy()).pos, pa.pos)
+            s.step(1e-3, 1)
+        got = get("bytes"), get("mallocs") - before
+        s.close()
+        return failed, got
+
+    _, (whole, count) = attempt(-1)
+    assert count > 10
+    for k in range(count):
+        failed, (held, _) = attempt(k)
+        assert failed and held == whole, (k, held, whole)
+    """)
