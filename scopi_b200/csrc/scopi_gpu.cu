@@ -111,12 +111,13 @@ struct scopi_gpu_handle {
     float4* d_us32[4] = {nullptr, nullptr, nullptr, nullptr};
     dvec4* d_usfin = nullptr;
 
-    // Friction (apgd_fric.cu): rows, incidence records and iterates of the solve; the FP64 set of
-    // a mixed handle is allocated when its first FP64 correction runs
+    // Friction (apgd_fric.cu): rows, incidence records and iterates of one solve, of FP64 size: a
+    // mixed handle's FP32 solves and its FP64 correction (the last solve of a step) use the same
+    // memory one after the other, each packing its rows first
     struct FricBuffers {
         void *rec = nullptr, *inc = nullptr, *lam[3] = {}, *u[4] = {}, *qv = nullptr, *wu = nullptr;
     };
-    FricBuffers fb64{}, fb32{};
+    FricBuffers fb{};
     DevMem fric_mem;
 
     // fixed small buffers
@@ -330,7 +331,7 @@ struct scopi_gpu_handle {
             BatchFricScenes S{};
             scenes(S);
             S.n_big = batch_n_big;
-            FricSolve<double> f = fric_buffers<double>(fb64, d_invm64, d_lamacc, d_ufin);
+            FricSolve<double> f = fric_buffers<double>(d_invm64, d_lamacc, d_ufin);
             launch_fric_pack<double>(P.dim, na, cur, as, inc, f, d_sizes_cur, stream);
             launch_fric_batch(nin, na, P.dim, st, f, d_sizes_cur, S, stream);
             return;
@@ -676,31 +677,29 @@ struct scopi_gpu_handle {
         return 0;
     }
 
-    template <typename T>
-    int alloc_fric(DevMem& mem, FricBuffers& b) {
-        cudaError_t e;
-        const bool f32 = sizeof(T) == 4;
-        auto get = [&](void*& p, size_t bytes) {
-            unsigned char* q = nullptr;
-            e = alloc(mem, q, bytes);
-            p = q;
-            return e == cudaSuccess;
-        };
-        bool ok = get(b.rec, c_cap * fric_rec_bytes(P.dim, f32)) && get(b.inc, inc_slots() * fric_inc_bytes(P.dim, f32));
-        for (int k = 0; k < 3 && ok; ++k) ok = get(b.lam[k], c_cap * fric_lam_bytes(P.dim, f32));
-        for (int k = 0; k < 4 && ok; ++k) ok = get(b.u[k], ((size_t)na + 1) * fric_u_vectors(P.dim) * sizeof(V4<T>));
-        if (batch && ok)
-            ok = get(b.qv, c_cap * fric_lam_bytes(P.dim, f32)) && get(b.wu, ((size_t)na + 1) * sizeof(double));
-        if (!ok) b = FricBuffers{};
-        return ok ? 0 : cuda_fail(e, "cudaMalloc(friction rows)");
-    }
-
     // the friction solve's buffers, whose sizes follow the contact capacity and the bodies
     int alloc_fric_set() {
         fric_mem.release();
-        fb64 = fb32 = FricBuffers{};
+        fb = FricBuffers{};
         if (!fric()) return 0;
-        return mixed() ? alloc_fric<float>(fric_mem, fb32) : alloc_fric<double>(fric_mem, fb64);
+        cudaError_t e = cudaSuccess;
+        auto get = [&](void*& p, size_t bytes) {
+            unsigned char* q = nullptr;
+            if (e == cudaSuccess) e = alloc(fric_mem, q, bytes);
+            p = q;
+        };
+        get(fb.rec, c_cap * fric_rec_bytes(P.dim, false));
+        get(fb.inc, inc_slots() * fric_inc_bytes(P.dim, false));
+        for (auto& p : fb.lam) get(p, c_cap * fric_lam_bytes(P.dim, false));
+        for (auto& p : fb.u) get(p, ((size_t)na + 1) * fric_u_vectors(P.dim) * sizeof(dvec4));
+        if (batch) {
+            get(fb.qv, c_cap * fric_lam_bytes(P.dim, false));
+            get(fb.wu, ((size_t)na + 1) * sizeof(double));
+        }
+        if (e == cudaSuccess) return 0;
+        fric_mem.release();
+        fb = FricBuffers{};
+        return cuda_fail(e, "cudaMalloc(friction rows)");
     }
 
     // Buffers whose size follows the contact capacity.  A failure leaves none (c_cap = 0), and the
@@ -714,7 +713,7 @@ struct scopi_gpu_handle {
         if (rc) {
             cap_mem.release();
             fric_mem.release();
-            fb64 = fb32 = FricBuffers{};
+            fb = FricBuffers{};
             c_cap = 0;
         }
         return rc;
@@ -1027,19 +1026,19 @@ struct scopi_gpu_handle {
     }
 
     template <typename T>
-    FricSolve<T> fric_buffers(const FricBuffers& b, const T* invm, T* lam_out, T* u_out) const {
+    FricSolve<T> fric_buffers(const T* invm, T* lam_out, T* u_out) const {
         FricSolve<T> f{};
         f.cap = c_cap;
         f.cij = d_cij;
-        f.rec = b.rec;
-        f.inc = b.inc;
+        f.rec = fb.rec;
+        f.inc = fb.inc;
         f.inc_slots = inc_slots();
         f.inc_ptr = inc.ptr;
         f.invm = invm;
-        for (int k = 0; k < 3; ++k) f.lam[k] = b.lam[k];
-        for (int k = 0; k < 4; ++k) f.u[k] = static_cast<V4<T>*>(b.u[k]);
-        f.qv = b.qv;
-        f.wu = static_cast<double*>(b.wu);
+        for (int k = 0; k < 3; ++k) f.lam[k] = fb.lam[k];
+        for (int k = 0; k < 4; ++k) f.u[k] = static_cast<V4<T>*>(fb.u[k]);
+        f.qv = fb.qv;
+        f.wu = static_cast<double*>(fb.wu);
         f.lam_out = lam_out;
         f.u_out = u_out;
         f.sums = d_sums;
@@ -1105,7 +1104,7 @@ struct scopi_gpu_handle {
                     if (rc) return rc;
                     ufin = reinterpret_cast<const double*>(d_us64[h_result->u_buf]);
                 } else if (fric()) {
-                    FricSolve<double> f = fric_buffers<double>(fb64, d_invm64, d_lam64[0], d_u64[0]);
+                    FricSolve<double> f = fric_buffers<double>(d_invm64, d_lam64[0], d_u64[0]);
                     launch_fric_pack<double>(P.dim, na, cur, as, inc, f, d_sizes_cur, stream);
                     rc = run_apgd_fric<double>(f, dt, P.tolerance, P.max_ite);
                     if (rc) return rc;
@@ -1265,7 +1264,7 @@ struct scopi_gpu_handle {
             launch_pack_inc<float>(na, inc.ptr, inc.idx, as.bn, d_incv32, inc_slots(), d_sizes_cur, stream);
             sbs = sph_buffers<float>(d_nc32, d_incv32, d_imt32, d_lam32, d_us32);
         } else if (fric()) {
-            sf = fric_buffers<float>(fb32, d_invm32, d_lam32[0], nullptr);
+            sf = fric_buffers<float>(d_invm32, d_lam32[0], nullptr);
             launch_fric_pack<float>(P.dim, na, cur, as, inc, sf, d_sizes_cur, stream);
         } else {
             launch_convert<double, float>(as.bn, d_bn32, 3 * c_cap, &d_sizes_cur->C, 3, stream);
@@ -1327,11 +1326,7 @@ struct scopi_gpu_handle {
                 // the FP64 residual reads (n, c) from the same records
                 launch_pack_nc<double>(as.bn, as.cvec, d_nc64, d_sizes_cur, c_cap, stream);
             } else if (fric()) {
-                if (!fb64.rec) {
-                    r = alloc_fric<double>(fric_mem, fb64);
-                    if (r) return r;
-                }
-                FricSolve<double> f = fric_buffers<double>(fb64, d_invm64, d_lam64[0], nullptr);
+                FricSolve<double> f = fric_buffers<double>(d_invm64, d_lam64[0], nullptr);
                 Assembly ar = as;
                 ar.cvec = d_res64;
                 f.shift = d_lamacc;

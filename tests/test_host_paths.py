@@ -200,3 +200,17 @@ def test_step_retried_after_a_failed_growth(fake, problem, precision):
         failed, (held, _) = attempt(k)
         assert failed and held == whole, (k, held, whole)
     """)
+
+
+@pytest.mark.parametrize("problem", ["FRICTION", "NOFRICTION"])
+def test_corrections_allocate_nothing(fake, problem):
+    """A violation target that is never met: every step ends with the FP64 correction."""
+    fake(f"""
+    put("contacts", 1000)
+    s = rows(dict(problem={problem}, precision=MIXED, mu=0.3, mixed_violation_tol=-1.0, mixed_max_corrections=1))
+    s.stream_handle()
+    before = get("mallocs"), get("bytes")
+    s.step(1e-3, 2)
+    assert s.stats()["corrections"] == 2
+    assert (get("mallocs"), get("bytes")) == before
+    """)
