@@ -1058,17 +1058,13 @@ cudaError_t launch_apgd_batch6(const Bodies& b, const StepParams& p, const ApgdS
     A.curvature_start = st.curvature_start;
     A.max_ite = st.max_ite;
     A.dynamic = st.dynamic;
-    const int grid = std::max(1, S.n_scenes);
-    if (p.problem == kViscous) {
-        if (p.dim == 3)
-            k_apgd_batch6<3, kViscous><<<grid, kBatch6Threads, 0, s>>>(A, S);
-        else
-            k_apgd_batch6<2, kViscous><<<grid, kBatch6Threads, 0, s>>>(A, S);
-    } else {
-        return cudaErrorInvalidValue;
-    }
+    if (p.problem != kViscous) return cudaErrorInvalidValue;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(std::max(1, S.n_scenes));
+    cfg.blockDim = dim3(kBatch6Threads);
+    cfg.stream = s;
     g_apgd_launches += 1;
-    return cudaGetLastError();
+    return cudaLaunchKernelEx(&cfg, p.dim == 3 ? k_apgd_batch6<3, kViscous> : k_apgd_batch6<2, kViscous>, A, S);
 }
 
 int apgd_max_blocks(int problem, int dim, bool fp32) {

@@ -563,27 +563,27 @@ __global__ void k_batch_ranges(int n_scenes, int nin, const int* sc_obs0, const 
 
 template <typename T, int DIM, int BT, int KB, int CS>
 cudaError_t launch_bt(BatchArgs<T>& A, int n_scenes, cudaStream_t s) {
-    if (CS == 1) {
-        k_apgd_batch<T, DIM, BT, KB><<<n_scenes, BT, 0, s>>>(A);
-    } else {
-        // the n_big largest scenes on two CTAs each, the rest paired, every cluster two CTAs
-        const int clusters = A.n_big + (n_scenes - A.n_big + 1) / 2;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * clusters, 1, 1);
-        cfg.blockDim = dim3(BT, 1, 1);
-        cfg.dynamicSmemBytes = 0;
-        cfg.stream = s;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 2;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        cfg.attrs = at;
-        cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_apgd_batch_pairs<T, DIM, BT, KB>, A);
-    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.blockDim = dim3(BT, 1, 1);
+    cfg.dynamicSmemBytes = 0;
+    cfg.stream = s;
     g_batch_launches += 1;
-    return cudaGetLastError();
+    // the launch's own status, not the thread's last error
+    if (CS == 1) {
+        cfg.gridDim = dim3(n_scenes, 1, 1);
+        return cudaLaunchKernelEx(&cfg, k_apgd_batch<T, DIM, BT, KB>, A);
+    }
+    // the n_big largest scenes on two CTAs each, the rest paired, every cluster two CTAs
+    const int clusters = A.n_big + (n_scenes - A.n_big + 1) / 2;
+    cfg.gridDim = dim3(2 * clusters, 1, 1);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_apgd_batch_pairs<T, DIM, BT, KB>, A);
 }
 
 }  // namespace

@@ -255,8 +255,9 @@ struct scopi_gpu_handle {
     }
 
     // Every kernel of one batch step, enqueued on `stream` with no host synchronisation
-    // (captured once into a CUDA graph and replayed every step).
-    void enqueue_batch_step(double dt, int bt, int tile) {
+    // (captured once into a CUDA graph and replayed every step).  Returns the status of the solve's
+    // launch: a step without its solve must not be replayed.
+    cudaError_t enqueue_batch_step(double dt, int bt, int tile) {
         Bodies b = bodies();
         StepParams sp = step_params(dt);
         if (nin > 0) {
@@ -280,7 +281,8 @@ struct scopi_gpu_handle {
             // the contacts with gamma < 0): the 6-dof rows solved per scene in FP64
             launch_batch_ranges(n_scenes, nin, d_sc_obs0, d_sc_obs1, d_sc_p0, d_sc_p1, d_obs_off, dw.obs_pos,
                                 dw.row_ptr, d_sizes_cur, d_sc_o0, d_sc_o1, d_sc_a0, d_sc_a1, stream);
-            enqueue_batch_solve6(dt);
+            const cudaError_t e = enqueue_batch_solve6(dt);
+            if (e != cudaSuccess) return e;
             if (visc) {
                 launch_gamma_update(sp, cur, as, d_lamacc, d_sizes_cur, c_cap, stream);
                 // this step's list (pairs and gamma) is the next step's previous list
@@ -290,7 +292,7 @@ struct scopi_gpu_handle {
                 cudaMemcpyAsync(d_sizes_old, d_sizes_cur, sizeof(Sizes), cudaMemcpyDeviceToDevice, stream);
             }
             launch_update(b, sp, d_ufin, 6, 1, d_sizes_cur, stream);
-            return;
+            return cudaSuccess;
         }
         launch_pack_cij(cur.ci, cur.cj, d_cij, d_sizes_cur, c_cap, stream);
         launch_pack_nc<double>(as.bn, as.cvec, d_nc64, d_sizes_cur, c_cap, stream);
@@ -301,11 +303,13 @@ struct scopi_gpu_handle {
         }
         launch_batch_ranges(n_scenes, nin, d_sc_obs0, d_sc_obs1, d_sc_p0, d_sc_p1, d_obs_off, dw.obs_pos, dw.row_ptr,
                             d_sizes_cur, d_sc_o0, d_sc_o1, d_sc_a0, d_sc_a1, stream);
-        enqueue_batch_solve(dt, bt, tile);
+        const cudaError_t e = enqueue_batch_solve(dt, bt, tile);
+        if (e != cudaSuccess) return e;
         launch_update(b, sp, reinterpret_cast<const double*>(d_usfin), 4, 0, d_sizes_cur, stream);
+        return cudaSuccess;
     }
 
-    void enqueue_batch_solve6(double dt) {
+    cudaError_t enqueue_batch_solve6(double dt) {
         Bodies b = bodies();
         StepParams sp = step_params(dt);
         ApgdSettings st{};
@@ -333,8 +337,7 @@ struct scopi_gpu_handle {
             S.n_big = batch_n_big;
             FricSolve<double> f = fric_buffers<double>(d_invm64, d_lamacc, d_ufin);
             launch_fric_pack<double>(P.dim, na, cur, as, inc, f, d_sizes_cur, stream);
-            launch_fric_batch(nin, na, P.dim, st, f, d_sizes_cur, S, stream);
-            return;
+            return launch_fric_batch(nin, na, P.dim, st, f, d_sizes_cur, S, stream);
         }
         const long long M = (long long)mult_per_contact() * c_cap;
         cudaMemsetAsync(d_lam64[0], 0, M * sizeof(double), stream);
@@ -359,10 +362,10 @@ struct scopi_gpu_handle {
         scenes(S);
         S.lam_out = d_lamacc;
         S.u_out = d_ufin;
-        launch_apgd_batch6(b, sp, st, cur, as, sb, d_invm64, S, stream);
+        return launch_apgd_batch6(b, sp, st, cur, as, sb, d_invm64, S, stream);
     }
 
-    void enqueue_batch_solve(double dt, int bt, int tile) {
+    cudaError_t enqueue_batch_solve(double dt, int bt, int tile) {
         auto fill = [&](auto& bs) {
             bs.nin = nin;
             bs.n_big = batch_n_big;
@@ -398,7 +401,7 @@ struct scopi_gpu_handle {
             bs.inc = d_incv32;
             for (int k = 0; k < 3; ++k) bs.lam[k] = d_lam32[k];
             for (int k = 0; k < 4; ++k) bs.u[k] = d_us32[k];
-            launch_apgd_batch<float>(P.dim, bt, tile, bs, n_scenes, stream);
+            return launch_apgd_batch<float>(P.dim, bt, tile, bs, n_scenes, stream);
         } else {
             BatchSolve<double> bs{};
             fill(bs);
@@ -406,7 +409,7 @@ struct scopi_gpu_handle {
             bs.inc = reinterpret_cast<const dvec4*>(d_incv64);
             for (int k = 0; k < 3; ++k) bs.lam[k] = d_lam64[k];
             for (int k = 0; k < 4; ++k) bs.u[k] = d_us64[k];
-            launch_apgd_batch<double>(P.dim, bt, tile, bs, n_scenes, stream);
+            return launch_apgd_batch<double>(P.dim, bt, tile, bs, n_scenes, stream);
         }
     }
 
@@ -471,10 +474,16 @@ struct scopi_gpu_handle {
                 cudaError_t e = cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal);
                 if (e != cudaSuccess) return cuda_fail(e, "cudaStreamBeginCapture");
                 const long long l0 = launches();
-                enqueue_batch_step(dt, bt, tile);
+                const cudaError_t solve = enqueue_batch_step(dt, bt, tile);
                 graph_kernels = launches() - l0;
                 replayed -= graph_kernels;  // the capture itself launched nothing
                 e = cudaStreamEndCapture(stream, &graph);
+                if (solve != cudaSuccess) {
+                    if (e != cudaSuccess) graph = nullptr;
+                    cudaGetLastError();
+                    drop_graph();
+                    return cuda_fail(solve, "batch solve launch");
+                }
                 if (e != cudaSuccess) return cuda_fail(e, "cudaStreamEndCapture");
                 e = cudaGraphInstantiate(&graph_exec, graph, 0);
                 if (e != cudaSuccess) return cuda_fail(e, "cudaGraphInstantiate");
@@ -516,7 +525,10 @@ struct scopi_gpu_handle {
         int best_bt = kBatchDefaultThreads, best_tile = batch_default_tile(kBatchDefaultThreads);
         for (int k = 0; k < kBatchShapes; ++k) {
             cudaEventRecord(ev_a[0], stream);
-            enqueue_batch_solve(dt, cand[k][0], cand[k][1]);
+            if (enqueue_batch_solve(dt, cand[k][0], cand[k][1]) != cudaSuccess) {
+                cudaGetLastError();  // nothing ran: not a shape to choose
+                continue;
+            }
             cudaEventRecord(ev_a[1], stream);
             cudaError_t e = cudaEventSynchronize(ev_a[1]);
             if (e != cudaSuccess) return cuda_fail(e, "batch autotune");

@@ -214,3 +214,23 @@ def test_corrections_allocate_nothing(fake, problem):
     assert s.stats()["corrections"] == 2
     assert (get("mallocs"), get("bytes")) == before
     """)
+
+
+@pytest.mark.parametrize("kw", ["problem=FRICTION, mu=0.3", "block_threads=2048", "block_threads=2048, precision=MIXED"])
+def test_batch_step_without_its_solve_fails(fake, kw):
+    """A solve that cannot be launched fails the step; nothing is replayed without it, and the batch
+    steps again once the launch is possible."""
+    fake(f"""
+    scenes = [configs.box_3d(seed=k, count=30) for k in range(3)]
+    b = ScopiBatch(scenes, vap=1, dmax=0.0045, {kw})
+    for _ in range(2):
+        put("refuse_clusters", 1)
+        for _ in range(2):
+            with pytest.raises(ScopiGPUError, match="batch solve"):
+                b.run(1e-3, 1)
+        put("refuse_clusters", 0)
+        b.run(1e-3, 1)
+        b.run(2e-3, 1)
+        b.run(1e-3, 0)
+    b.close()
+    """)
