@@ -23,6 +23,9 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
+#include <functional>
+#include <queue>
 
 #include "apgd_common.cuh"
 
@@ -568,7 +571,7 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
 }
 
 // ------------------------------------------------------------------ batched scenes (FP64)
-// One CTA per scene, or a cluster of CS CTAs for a large one: the same iteration on the scene's
+// One CTA per scene, or a cluster of CS CTAs for a large one (fric_batch_form): the same iteration on the scene's
 // contacts (its obstacle rows [o0, o1), then its active rows [a0, a1)) and bodies [p0, p1), so
 // every scene iterates until its own stopping test holds; the multipliers, the velocities and
 // the scene's statistics with the violation max(0, -gap) of its final state go to fixed outputs.
@@ -582,7 +585,8 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
 // The particle pass does not wait for the sums: it forms u(next y) with the momentum of an
 // accepted step, and after a restart u(l+) itself is the next y.  96 2D scenes of 200 to 2000
 // disks, milliseconds a step: the generic 6-dof rows on 256 threads 69.4; packed rows on 256
-// threads with two contacts at a time 23.1; this form, clusters of two for the largest, 15.5.
+// threads with two contacts at a time 23.1; this form, clusters of two for the largest, 15.5.  Every
+// split gives the same bits.
 constexpr int kChains = 256;
 template <int DIM>
 constexpr int kBatchFricThreads = DIM == 2 ? 512 : 256;  // 128 registers hold a 2D row, 255 a 3D one
@@ -617,14 +621,15 @@ __device__ __forceinline__ void share(double* at, double v) {
     }
 }
 
-template <int DIM, int CS>
+template <int DIM, int CS, int BT>
 __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, int sc, int rank, ApgdState& S,
                            SceneSums& Q) {
     using T = double;
     using F = FricShape<T, DIM>;
     using L = Lam<T, DIM>;
-    constexpr int NT = CS * kBatchFricThreads<DIM>, BT = kBatchFricThreads<DIM>;
+    constexpr int NT = CS * BT;
     constexpr int VT = kChains / CS;           // chains of this CTA: [rank * VT, rank * VT + VT)
+    constexpr int CT = BT < VT ? BT : VT;      // summed at a time
     constexpr int SPLIT = BT / VT >= 2 ? 2 : 1;  // threads per chain: the sums shared between two
     const int lt = threadIdx.x, tid = rank * BT + lt;
     const IncLayout lay = inc_layout(A.sizes, A.na, A.inc_slots);
@@ -675,9 +680,9 @@ __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, 
             A.wu[p] = body_wu<T, DIM>(w, u);
         }
         scene_sync<CS>();
-        double s[2] = {0.0, 0.0};
-        if (lt < VT) {
-            const int vt = rank * VT + lt;
+        for (int q = lt; lt < CT && q < VT; q += CT) {
+            double s[2] = {0.0, 0.0};
+            const int vt = rank * VT + q;
             for (int k = vt; k < nc; k += kChains) {
                 T z[4];
                 fld4cg(dbuf + contact_at(k), z);
@@ -739,8 +744,9 @@ __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, 
         {
             constexpr int J = 2;  // contacts whose loads are in flight
             const int part = SPLIT == 2 ? lt / VT : 0;
-            if (lt < SPLIT * VT) {
-                const int vt = rank * VT + (lt - part * VT);
+#pragma unroll 1
+            for (int q = lt - part * VT; lt < SPLIT * CT && q < VT; q += CT) {
+                const int vt = rank * VT + q;
                 double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
 #pragma unroll 1
                 for (int k = vt; k < nc; k += J * kChains) {
@@ -804,11 +810,12 @@ __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, 
         scene_sync<CS>();
         // ---- w.u along the chains (every CTA all of them: one sum), then the decisions
         {
-            double s[1] = {0.0};
-            if (lt < kChains)
-                for (int p = p0 + lt; p < p1; p += kChains) s[0] += __ldcg(A.wu + p);
-            const double x = multi_reduce<1>(s);
-            if (lt < kChains && (lt & 31) == 0) Q.b[lt >> 5] = x;
+            for (int t = lt; t < kChains; t += BT) {
+                double s[1] = {0.0};
+                for (int p = p0 + t; p < p1; p += kChains) s[0] += __ldcg(A.wu + p);
+                const double x = multi_reduce<1>(s);
+                if ((t & 31) == 0) Q.b[t >> 5] = x;
+            }
         }
         __syncthreads();
         if (lt < 32) {
@@ -888,12 +895,20 @@ __global__ void __launch_bounds__(kBatchFricThreads<DIM>, 1) k_fric_batch(FricAr
     __shared__ SceneSums Q;
     if (A.sizes->overflow) return;  // the step is redone after the buffers grow (all CTAs alike)
     const int q = blockIdx.x / CS, rank = blockIdx.x % CS;
-    if (CS > 1 && q < B.n_big) {
-        fric_scene<DIM, CS>(A, B, B.order[q], rank, S, Q);
+    if (q < B.n_big) {
+        fric_scene<DIM, CS, kBatchFricThreads<DIM>>(A, B, B.order[q], rank, S, Q);
     } else {
-        const int j = CS == 1 ? q : B.n_big + CS * (q - B.n_big) + rank;
-        if (j < B.n_scenes) fric_scene<DIM, 1>(A, B, B.order[j], 0, S, Q);
+        const int j = B.n_big + CS * (q - B.n_big) + rank;
+        if (j < B.n_scenes) fric_scene<DIM, 1, kBatchFricThreads<DIM>>(A, B, B.order[j], 0, S, Q);
     }
+}
+// One CTA of BT threads per scene, PER of them on an SM: more scenes than the SMs hold at once.
+template <int DIM, int BT, int PER>
+__global__ void __launch_bounds__(BT, PER) k_fric_many(FricArgs<double> A, BatchFricScenes B) {
+    __shared__ ApgdState S;
+    __shared__ SceneSums Q;
+    if (A.sizes->overflow) return;
+    fric_scene<DIM, 1, BT>(A, B, B.order[blockIdx.x], 0, S, Q);
 }
 
 // ------------------------------------------------------------------ packing
@@ -1101,38 +1116,141 @@ cudaError_t launch_apgd_fric(int nin, int na, int dim, const ApgdSettings& st, F
     FricArgs<T> A = fric_args<T>(nin, na, st, f, sizes);
     return dim == 3 ? launch_fric_t<T, 3>(A, nblocks, s) : launch_fric_t<T, 2>(A, nblocks, s);
 }
+
+// ------------------------------------------------------------------ how a batch is split
+// One iteration of a scene of n bodies costs max(floor, base + slope n) microseconds (its contacts
+// follow its bodies: 2.5 a disk, 3.8 a sphere).  Measured, clusters on one scene, the others with
+// every SM at work:
+//                                     2D, n = 30   100   300  1000  2500    3D, n = 30   100   300  1000
+//   cluster of 4                            5.5   5.8   7.8  11.2  20.7            7.2   9.2  15.2  24.5
+//   cluster of 2                            5.4   5.9   8.2  13.2  29.1            7.3   9.9  17.9  40.0
+//   one CTA an SM                           4.1   4.5   7.6  18.0  42.3            5.0   9.0  21.0  62.3
+//   2D two CTAs of 256 an SM                4.0   4.8  10.8
+//   2D four, 3D two CTAs of 128 an SM       4.3   6.7  19.5                        6.0  12.7
+// Clusters shorten the longest scene; more and smaller CTAs get more scenes through.  The form whose
+// list schedule of the scenes, largest first, ends first is taken.  Milliseconds a step of the generic
+// 6-dof rows (two CTAs of 256 an SM), of clusters of two whatever the number of scenes, and of this
+// rule: 1000 x 30 disks 12.1, 39.4, 5.3; 600 x 100 18.1, 29.2, 7.2; 300 x 400 34.6, 23.5, 14.5;
+// 1000 x 30 spheres 16.7, 55.9, 12.7; 300 x 200 29.6, 40.2, 24.4.
+namespace {
+struct IterationCost {
+    double floor, base, slope;
+    double of(int n) const { return std::max(floor, base + slope * n); }
+};
+struct FricForm {
+    int cs, per_sm;  // CTAs of a cluster; CTAs of an SM
+    IterationCost large, other;  // a scene on a cluster, on one CTA
+};
+const FricForm kFricForms[2][FricBatchForm::kCount] = {
+    {{4, 1, {5.5, 5.0, 0.0063}, {4.1, 2.6, 0.0165}},
+     {2, 1, {5.4, 4.8, 0.0098}, {4.1, 2.6, 0.0165}},
+     {2, 1, {}, {4.1, 2.6, 0.0165}},
+     {1, 2, {}, {4.0, 1.8, 0.0300}},
+     {1, 4, {}, {4.3, 0.3, 0.0640}}},
+    {{4, 1, {7.2, 8.5, 0.0160}, {5.0, 1.0, 0.0750}},
+     {2, 1, {7.3, 7.0, 0.0350}, {5.0, 1.0, 0.0750}},
+     {2, 1, {}, {5.0, 1.0, 0.0750}},
+     {0, 0, {}, {}},  // 256 threads with a 3D row each fill the registers of an SM
+     {1, 2, {}, {5.9, 0.0, 0.1320}}}};
+
+template <int DIM, int CS>
+cudaLaunchConfig_t fric_cluster_config(int clusters, cudaStream_t s, cudaLaunchAttribute* at) {
+    cudaLaunchConfig_t cfg = cluster_config(CS, kBatchFricThreads<DIM>, s, at);
+    cfg.gridDim = dim3(CS * clusters);
+    return cfg;
+}
+// clusters of CS CTAs that run at once (an SM group need not be a multiple of four: 37 clusters of
+// four on 148 SMs take two rounds)
+template <int DIM, int CS>
+int fric_cluster_slots() {
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t cfg = fric_cluster_config<DIM, CS>(kSMs / CS, nullptr, at);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_fric_batch<DIM, CS>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        return kSMs / CS;
+    }
+    return n;
+}
+
+// when the last of the CTAs (clusters) that start in order on `slots` free places ends
+double list_schedule(const std::vector<double>& cost, int slots) {
+    std::priority_queue<double, std::vector<double>, std::greater<double>> busy;
+    double end = 0.0;
+    for (double c : cost) {
+        double at = 0.0;
+        if ((int)busy.size() == slots) {
+            at = busy.top();
+            busy.pop();
+        }
+        busy.push(at + c);
+        end = std::max(end, at + c);
+    }
+    return end;
+}
+}  // namespace
+
+FricBatchForm fric_batch_form(int dim, const std::vector<int>& bodies) {
+    FricBatchForm best{};
+    double least = 0.0;
+    int big = 0;  // the scenes with at least half the largest one's bodies
+    while (big < (int)bodies.size() && 2LL * bodies[big] >= bodies[0]) ++big;
+    const int slots4 = dim == 3 ? fric_cluster_slots<3, 4>() : fric_cluster_slots<2, 4>();
+    const int slots2 = dim == 3 ? fric_cluster_slots<3, 2>() : fric_cluster_slots<2, 2>();
+    for (int k = 0; k < FricBatchForm::kCount; ++k) {
+        const FricForm& f = kFricForms[dim == 3][k];
+        if (f.cs == 0) continue;
+        const int n_big = k == FricBatchForm::kCluster4 || k == FricBatchForm::kCluster2 ? big : 0;
+        std::vector<double> cost;
+        for (int j = 0; j < (int)bodies.size(); j += j < n_big ? 1 : f.cs) {
+            // the iterations of like scenes differ by about a fifth either way
+            const double x = j * 0.6180339887498949, spread = 0.8 + 0.4 * (x - std::floor(x));
+            cost.push_back(spread * (j < n_big ? f.large.of(bodies[j]) : f.other.of(bodies[j])));
+        }
+        const double t = list_schedule(cost, f.cs == 4 ? slots4 : f.cs == 2 ? slots2 : kSMs * f.per_sm);
+        if (k == 0 || t < least) {
+            least = t;
+            best.form = k;
+            best.n_big = n_big;
+        }
+    }
+    return best;
+}
+
 namespace {
 template <int DIM, int CS>
-cudaError_t launch_fric_batch_t(const FricArgs<double>& A, const BatchFricScenes& B, cudaStream_t s) {
-    const int clusters = CS == 1 ? B.n_scenes : B.n_big + (B.n_scenes - B.n_big + CS - 1) / CS;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(CS * clusters);
-    cfg.blockDim = dim3(kBatchFricThreads<DIM>);
-    cfg.stream = s;
+cudaError_t launch_fric_clusters(const FricArgs<double>& A, const BatchFricScenes& B, cudaStream_t s) {
     cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeClusterDimension;
-    at[0].val.clusterDim.x = CS;
-    at[0].val.clusterDim.y = 1;
-    at[0].val.clusterDim.z = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    g_fric_launches += 1;
+    const cudaLaunchConfig_t cfg =
+        fric_cluster_config<DIM, CS>(B.n_big + (B.n_scenes - B.n_big + CS - 1) / CS, s, at);
     return cudaLaunchKernelEx(&cfg, k_fric_batch<DIM, CS>, A, B);
+}
+template <int DIM, int BT, int PER>
+cudaError_t launch_fric_many(const FricArgs<double>& A, const BatchFricScenes& B, cudaStream_t s) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(B.n_scenes);
+    cfg.blockDim = dim3(BT);
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, k_fric_many<DIM, BT, PER>, A, B);
 }
 }  // namespace
 
 cudaError_t launch_fric_batch(int nin, int na, int dim, const ApgdSettings& st, FricSolve<double>& f,
-                              const Sizes* sizes, BatchFricScenes B, cudaStream_t s) {
+                              const Sizes* sizes, BatchFricScenes B, FricBatchForm form, cudaStream_t s) {
     if (B.n_scenes <= 0) return cudaSuccess;
     const FricArgs<double> A = fric_args<double>(nin, na, st, f, sizes);
-    B.n_big = std::min(std::max(B.n_big, 0), B.n_scenes);
-    // the longest scene is the critical path: the scenes with at least half its bodies get four
-    // CTAs while all CTAs still run at once (3 scenes of up to 300 disks: 11.7 -> 4.6 ms a step
-    // against the generic rows), else two (200 scenes of up to 3000: 128.8 -> 29.2)
-    const int small = B.n_scenes - B.n_big;
-    if (4 * B.n_big + (small + 3) / 4 * 4 <= kSMs)
-        return dim == 3 ? launch_fric_batch_t<3, 4>(A, B, s) : launch_fric_batch_t<2, 4>(A, B, s);
-    return dim == 3 ? launch_fric_batch_t<3, 2>(A, B, s) : launch_fric_batch_t<2, 2>(A, B, s);
+    B.n_big = std::min(std::max(form.n_big, 0), B.n_scenes);
+    g_fric_launches += 1;
+    switch (form.form) {
+        case FricBatchForm::kCluster4:
+            return dim == 3 ? launch_fric_clusters<3, 4>(A, B, s) : launch_fric_clusters<2, 4>(A, B, s);
+        case FricBatchForm::kMany256:
+            return launch_fric_many<2, 256, 2>(A, B, s);
+        case FricBatchForm::kMany128:
+            return dim == 3 ? launch_fric_many<3, 128, 2>(A, B, s) : launch_fric_many<2, 128, 4>(A, B, s);
+        default:
+            return dim == 3 ? launch_fric_clusters<3, 2>(A, B, s) : launch_fric_clusters<2, 2>(A, B, s);
+    }
 }
 #define INST(T) \
     template void launch_fric_pack<T>(int, int, const Contacts&, const Assembly&, const Incidence&, FricSolve<T>&, \

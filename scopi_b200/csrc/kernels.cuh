@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "common.cuh"
 
 namespace scopi_gpu {
@@ -434,13 +436,20 @@ cudaError_t launch_apgd_batch6(const Bodies& b, const StepParams& p, const ApgdS
 
 struct BatchFricScenes {
     int n_scenes;
-    int n_big;          // the largest scenes (at least half the largest one's bodies)
+    int n_big;          // scenes on a whole cluster
     const int* order;   // largest first
     const int *sc_p0, *sc_p1, *sc_o0, *sc_o1, *sc_a0, *sc_a1;
     BatchSceneStats* stats;
 };
+// how the scenes are spread over the SMs; bodies per scene, largest first
+struct FricBatchForm {
+    enum { kCluster4, kCluster2, kOneEach, kMany256, kMany128, kCount };
+    int form;
+    int n_big;  // the largest scenes, on a whole cluster each
+};
+FricBatchForm fric_batch_form(int dim, const std::vector<int>& bodies);
 cudaError_t launch_fric_batch(int nin, int na, int dim, const ApgdSettings& st, FricSolve<double>& f,
-                              const Sizes* sizes, BatchFricScenes B, cudaStream_t s);
+                              const Sizes* sizes, BatchFricScenes B, FricBatchForm form, cudaStream_t s);
 
 long long apgd_batch_launches();
 void launch_batch_ranges(int n_scenes, int nin, const int* sc_obs0, const int* sc_obs1, const int* sc_p0,

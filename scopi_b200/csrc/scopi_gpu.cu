@@ -238,6 +238,7 @@ struct scopi_gpu_handle {
     int batch_tile_used = 0;
     float batch_tune_ms[kBatchShapes] = {};
     int batch_n_big = 0;  // 2048-thread shape: scenes with at least half the largest scene's bodies
+    FricBatchForm fric_form{};  // Friction scenes: how they are spread over the SMs
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t graph_exec = nullptr;
     double graph_dt = 0.0;
@@ -334,10 +335,9 @@ struct scopi_gpu_handle {
         if (fric()) {
             BatchFricScenes S{};
             scenes(S);
-            S.n_big = batch_n_big;
             FricSolve<double> f = fric_buffers<double>(d_invm64, d_lamacc, d_ufin);
             launch_fric_pack<double>(P.dim, na, cur, as, inc, f, d_sizes_cur, stream);
-            return launch_fric_batch(nin, na, P.dim, st, f, d_sizes_cur, S, stream);
+            return launch_fric_batch(nin, na, P.dim, st, f, d_sizes_cur, S, fric_form, stream);
         }
         const long long M = (long long)mult_per_contact() * c_cap;
         cudaMemsetAsync(d_lam64[0], 0, M * sizeof(double), stream);
@@ -2098,6 +2098,9 @@ int32_t scopi_gpu_batch_create(const scopi_gpu_params* p, int32_t n_scenes, cons
         int nb = 0;
         while (nb < n_scenes && 2 * (sc_p1[order[nb]] - sc_p0[order[nb]]) >= largest) ++nb;
         h->batch_n_big = nb;
+        std::vector<int> bodies(n_scenes);
+        for (int s = 0; s < n_scenes; ++s) bodies[s] = sc_p1[order[s]] - sc_p0[order[s]];
+        h->fric_form = fric_batch_form(p->dim, bodies);
     }
     scopi_gpu_particles cat{ntot, nin_tot, shape.data(), pos.data(), q.data(), v.data(), om.data(), vd.data(),
                             od.data(), f.data(), m.data(), jj.data(), rad.data(), len.data()};

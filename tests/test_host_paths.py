@@ -20,7 +20,7 @@ PRELUDE = """
 import ctypes as C
 import sys
 fake = C.CDLL({so!r}, mode=C.RTLD_GLOBAL)
-fake.fake_get.restype = C.c_longlong
+fake.fake_get.restype = fake.fake_launches_of.restype = C.c_longlong
 get = lambda w: fake.fake_get(w.encode())
 put = lambda w, v: fake.fake_set(w.encode(), C.c_longlong(v))
 sys.path[:0] = [{root!r}, {tests!r}]
@@ -232,5 +232,31 @@ def test_batch_step_without_its_solve_fails(fake, kw):
         b.run(1e-3, 1)
         b.run(2e-3, 1)
         b.run(1e-3, 0)
+    b.close()
+    """)
+
+
+# which kernel a friction batch takes: a queue of clusters loses to one small CTA per scene, a few
+# large scenes win from clusters (template arguments of the names: dim, cluster or threads, CTAs per SM)
+@pytest.mark.parametrize("dim,sizes,kernel", [
+    (2, [2000] * 4, "k_fric_batchILi2ELi4"), (3, [250, 5, 600], "k_fric_batchILi3ELi4"),
+    (2, [2000, 1900] + [200] * 94, "k_fric_batchILi2ELi4"), (2, [2000 - 20 * k for k in range(90)], "k_fric_batchILi2ELi2"),
+    (2, [400] * 148, "k_fric_batchILi2ELi2"), (2, [300] * 600, "k_fric_manyILi2ELi256ELi2"),
+    (2, [30] * 600, "k_fric_manyILi2ELi128ELi4"), (3, [30] * 600, "k_fric_manyILi3ELi128ELi2"),
+    (3, [200] * 300, "k_fric_batchILi3ELi2")])
+def test_friction_batch_form(fake, dim, sizes, kernel):
+    fake(f"""
+    scenes = []
+    for n in {sizes}:
+        pa = configs.box_3d(count=n)
+        pa.dim = {dim}
+        scenes.append(pa)
+    b = ScopiBatch(scenes, vap=1, dmax=0.0045, problem=FRICTION, mu=0.3)
+    b.run(1e-3, 1)
+    print([k for k in ("k_fric_batchILi2ELi2", "k_fric_batchILi2ELi4", "k_fric_batchILi3ELi2", "k_fric_batchILi3ELi4",
+                       "k_fric_manyILi2ELi256", "k_fric_manyILi2ELi128", "k_fric_manyILi3ELi128")
+           if fake.fake_launches_of(k.encode())])
+    assert fake.fake_launches_of(b"k_fric_batchI") + fake.fake_launches_of(b"k_fric_manyI") == 1
+    assert fake.fake_launches_of({kernel.encode()}) == 1
     b.close()
     """)
