@@ -895,7 +895,7 @@ __global__ void k_assemble(Bodies B, StepParams p, Contacts c, Assembly a, const
             a.cvec[k] = cc;
         }
         for (int d = 0; d < 3; ++d) a.bn[3 * (long long)k + d] = n[d];
-        if (!p.torque_free)
+        if (!p.torque_free && p.problem != kFriction)
             for (int d = 0; d < 3; ++d) {
                 a.bai[3 * (long long)k + d] = arow[0][d];
                 a.baj[3 * (long long)k + d] = arow[1][d];

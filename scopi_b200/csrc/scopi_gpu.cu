@@ -169,7 +169,8 @@ struct scopi_gpu_handle {
     bool friction_rows() const { return P.problem == SCOPI_GPU_FRICTION || P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
     // the Friction problem (and FrictionFixedPoint): apgd_fric.cu
     bool fric() const { return P.problem == SCOPI_GPU_FRICTION; }
-    long long inc_slots() const { return kIncSlotsPerContact * c_cap; }
+    // records of the incidence lists: columns need room (IncLayout), the rows of a batch none to spare
+    long long inc_slots() const { return (batch ? 2 : kIncSlotsPerContact) * c_cap; }
     bool viscous_friction() const { return P.problem == SCOPI_GPU_VISCOUS_FRICTION; }
     bool fp_loop() const { return fixed_point || viscous_friction(); }
     // the viscous problems carry each contact's gamma from the previous list by (i, j)
@@ -752,7 +753,10 @@ struct scopi_gpu_handle {
                             &pw.s_ci, &pw.s_cj})
                 A(*q, cap + 1)
         }
-        A(as.bn, 3 * cap) A(as.bai, 3 * cap) A(as.baj, 3 * cap)
+        A(as.bn, 3 * cap)
+        if (!fric()) {
+            A(as.bai, 3 * cap) A(as.baj, 3 * cap)
+        }
         if (friction_rows()) A(as.bP, 18 * cap)
         A(as.cvec, cvec_per() * cap) A(as.vflag, cap) A(as.slot, cap)
         if (fp_loop()) {
@@ -760,26 +764,35 @@ struct scopi_gpu_handle {
         }
         A(inc.idx, 2 * cap)
         A(d_res64, M) A(d_lamacc, M)
+        A(d_cij, cap) A(d_se_keep, cap + 1) A(d_se_pos, cap + 1) A(d_se_u, 4 * cap + 4)
         if (fric()) {
-            A(d_lam64[0], M)
-            if (mixed()) A(d_lam32[0], M)
-            int rc = alloc_fric_set();
-            if (rc) return rc;
-        } else {
-            A(inc.coef, 12 * cap)
-            for (int k = 0; k < 3; ++k) A(d_lam64[k], M)
-            A(d_g64, M)
+            // apgd_fric.cu: packed rows and iterates of its own, the multipliers of a solve copied
+            // out (an FP64 handle's straight to the step's)
+            if (mixed()) {
+                A(d_lam64[0], M) A(d_lam32[0], M)
+            } else {
+                d_lam64[0] = d_lamacc;
+            }
+            return alloc_fric_set();
         }
-        if (mixed() && !fric()) {
+        for (int k = 0; k < 3; ++k) A(d_lam64[k], M)
+        A(d_g64, M)
+        if (mixed()) {
             A(d_bn32, 3 * cap) A(d_bai32, 3 * cap) A(d_baj32, 3 * cap)
             if (friction_rows()) A(d_bP32, 18 * cap)
-            A(d_cvec32, cvec_per() * cap) A(d_coef32, 12 * cap)
+            A(d_cvec32, cvec_per() * cap)
             for (int k = 0; k < 3; ++k) A(d_lam32[k], M)
             A(d_g32, M)
         }
-        A(d_cij, cap) A(d_nc64, cap) A(d_incv64, 2 * inc_slots()) A(d_se_keep, cap + 1) A(d_se_pos, cap + 1) A(d_se_u, 4 * cap + 4)
-        if (mixed()) {
-            A(d_nc32, cap) A(d_incv32, inc_slots())
+        if (!friction_rows()) {
+            // a step reads the torque-free records or the coefficients of the 6-dof rows (12 per
+            // contact), never both: one array
+            A(d_nc64, cap) A(d_incv64, std::max(2 * inc_slots(), 6 * cap))
+            inc.coef = reinterpret_cast<double*>(d_incv64);
+            if (mixed()) {
+                A(d_nc32, cap) A(d_incv32, std::max(inc_slots(), 3 * cap))
+                d_coef32 = reinterpret_cast<float*>(d_incv32);
+            }
         }
 #undef A
         return 0;

@@ -253,10 +253,43 @@ def test_friction_batch_form(fake, dim, sizes, kernel):
         scenes.append(pa)
     b = ScopiBatch(scenes, vap=1, dmax=0.0045, problem=FRICTION, mu=0.3)
     b.run(1e-3, 1)
-    print([k for k in ("k_fric_batchILi2ELi2", "k_fric_batchILi2ELi4", "k_fric_batchILi3ELi2", "k_fric_batchILi3ELi4",
-                       "k_fric_manyILi2ELi256", "k_fric_manyILi2ELi128", "k_fric_manyILi3ELi128")
-           if fake.fake_launches_of(k.encode())])
     assert fake.fake_launches_of(b"k_fric_batchI") + fake.fake_launches_of(b"k_fric_manyI") == 1
     assert fake.fake_launches_of({kernel.encode()}) == 1
     b.close()
+    """)
+
+
+# Device bytes per contact of capacity.  Normal problems and ViscousFriction: at most what they took
+# when every handle had its own coefficient array.  Friction keeps packed rows (192 in FP64), incidence
+# records (4 x 80) and iterates (96) beside the assembled rows; the generic rows took 832 and 1096.
+@pytest.mark.parametrize("problem,precision,limit", [
+    ("NOFRICTION", "FP64", 576), ("NOFRICTION", "MIXED", 728), ("VISCOUS", "FP64", 624), ("VISCOUS", "MIXED", 792),
+    ("VISCOUS_FRICTION", "FP64", 928), ("VISCOUS_FRICTION", "MIXED", 1212), ("FRICTION", "FP64", 1104),
+    ("FRICTION", "MIXED", 1140)])
+def test_memory_per_contact(fake, problem, precision, limit):
+    fake(f"""
+    from scopi_b200 import VISCOUS_FRICTION
+    got = []
+    for n in (20_000, 60_000):
+        put("contacts", n)
+        s = rows(dict(problem={problem}, precision={precision}, mu=0.3))
+        s.step(1e-3, 1)
+        got.append(get("bytes"))
+        s.close()
+    # the capacity grows to 1.3 times the contacts
+    assert got[1] - got[0] <= ({limit} + 0.5) * 1.3 * 40_000, (got[1] - got[0]) / 52_000
+    """)
+
+
+@pytest.mark.parametrize("kw,limit", [("", 748), ("precision=MIXED", 900), ("problem=VISCOUS", 796),
+                                      ("problem=FRICTION, mu=0.3", 1192)])
+def test_memory_of_a_batch(fake, kw, limit):
+    """The bodies' share (about 1030 bytes each) included, per contact of capacity (six a body)."""
+    fake(f"""
+    got = []
+    for n in (3000, 9000):
+        b = ScopiBatch([configs.box_3d(count=n)], vap=1, dmax=0.0045, {kw})
+        got.append(get("bytes"))
+        b.close()
+    assert got[1] - got[0] <= ({limit} + 0.5) * 6 * 6000, (got[1] - got[0]) / 36_000
     """)
