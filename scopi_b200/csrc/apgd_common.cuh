@@ -307,6 +307,7 @@ struct GridSums {
 
     template <int NP>
     __device__ __forceinline__ void publish(double* v, double (*sh)[32]) {
+        static_assert(TREE, "the streaming form's sums");
         warp_sums<NP>(v, sh);
         publish_warps<NP>(sh);
     }
@@ -329,9 +330,10 @@ struct GridSums {
     }
     template <int NP>
     __device__ __forceinline__ bool collect(double* t) {
+        static_assert(TREE, "the streaming form's sums");
         double x[5][NP];
         const bool ok = sum_collect<NP, 5>(slots, nb, m, bar, x);
-        const double y = TREE ? sum_lane_order<NP>(x) : sum_group_order<NP>(x);
+        const double y = sum_lane_order<NP>(x);
 #pragma unroll
         for (int k = 0; k < NP; ++k) t[k] = __shfl_sync(0xffffffffu, y, k << SumShift<NP>::value);
         return ok;
@@ -672,14 +674,11 @@ __device__ __forceinline__ void state_init(ApgdState& S, double alpha) {
 struct Momentum {
     double theta1, beta;
 };
-// FUSED: th^2 + theta1 rounded once; the two roundings differ in a handful of iterations, and each
-// solve keeps the one its results have always had
-template <bool FUSED = false>
 __device__ __forceinline__ Momentum prepare_momentum(const ApgdState& S) {
     const double th = S.theta, t2 = mul_rn(th, th);
     Momentum m;
     m.theta1 = 0.5 * fma_rn(th, sqrt(add_rn(4.0, t2)), -t2);
-    m.beta = mul_rn(th, add_rn(1.0, -th)) / (FUSED ? fma_rn(th, th, m.theta1) : add_rn(t2, m.theta1));
+    m.beta = mul_rn(th, add_rn(1.0, -th)) / add_rn(t2, m.theta1);
     return m;
 }
 // after the contact pass: momentum for the next y if this candidate is accepted

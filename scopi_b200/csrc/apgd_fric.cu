@@ -159,22 +159,7 @@ __device__ __forceinline__ void load_c(const Q4<T>* rec, long long cap, long lon
         o[d] = r[((e / F::per) * cap + c) * F::per + e % F::per];
     }
 }
-// u of a body, written by other blocks: (v, w), 2D (vx, vy, w)
-template <typename T, int DIM>
-__device__ __forceinline__ void gather_u(const V4<T>* u, int p, T* o) {
-    T t[4];
-    fld4(u + (long long)p * FricShape<T, DIM>::nu, t);
-    o[0] = t[0];
-    o[1] = t[1];
-    o[2] = t[2];
-    if (DIM == 3) {
-        fld4(u + 2ll * p + 1, t);
-        o[3] = t[0];
-        o[4] = t[1];
-        o[5] = t[2];
-    }
-}
-// this thread's own body
+// u of a body: (v, w), 2D (vx, vy, w)
 template <typename T, int DIM>
 __device__ __forceinline__ void load_u(const V4<T>* u, long long p, T* o) {
     T t[4];
@@ -344,10 +329,10 @@ __device__ __forceinline__ double body_curvature(const T* im, const T* u, const 
     return q;
 }
 
-// Threads per block (one block per SM).  FP64 keeps the 256 threads whose per-thread sums its
-// decisions have always been taken from; FP32 decisions do not hang on the last bits.
 constexpr long long kMaxBacktracks = 4000;
 
+// Threads per block (one block per SM).  FP64 keeps the 256 threads whose per-thread sums its
+// decisions have always been taken from; FP32 decisions do not hang on the last bits.
 template <typename T>
 struct FricThreads {
     static constexpr int value = sizeof(T) == 4 ? 512 : 256;
@@ -457,8 +442,8 @@ __global__ void __launch_bounds__(FricThreads<T>::value, 1) k_apgd_fric(FricArgs
                 T ui[F::dof], uj[F::dof], r[F::row], lm[4], lq[4], lo[3];
 #pragma unroll
                 for (int d = 0; d < F::dof; ++d) ui[d] = uj[d] = (T)0;
-                if (me.x >= A.nin) gather_u<T, DIM>(uY, me.x - A.nin, ui);
-                if (me.y >= A.nin) gather_u<T, DIM>(uY, me.y - A.nin, uj);
+                if (me.x >= A.nin) load_u<T, DIM>(uY, me.x - A.nin, ui);
+                if (me.y >= A.nin) load_u<T, DIM>(uY, me.y - A.nin, uj);
                 load_row<T, DIM>(A.rec, A.cap, c, r);
                 fld4(lam + c, lm);
                 if (use_prev) fld4(lprev + c, lq);
@@ -733,8 +718,8 @@ __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, 
             if (use_prev) fld4(lprev + c, lq);
 #pragma unroll
             for (int d = 0; d < F::dof; ++d) ui[d] = uj[d] = (T)0;
-            if (ij.x >= A.nin) gather_u<T, DIM>(uY, ij.x - A.nin, ui);
-            if (ij.y >= A.nin) gather_u<T, DIM>(uY, ij.y - A.nin, uj);
+            if (ij.x >= A.nin) load_u<T, DIM>(uY, ij.x - A.nin, ui);
+            if (ij.y >= A.nin) load_u<T, DIM>(uY, ij.y - A.nin, uj);
             contact_row<T, DIM, false>(r, ui, uj, lm, lq, beta, use_prev, bt, alpha, A.mu, A.dt2, nullptr, lo, s, qo);
             fst4(lnew + c, lo);
             fst4(qv + c, qo);
@@ -848,8 +833,8 @@ __device__ void fric_scene(const FricArgs<double>& A, const BatchFricScenes& B, 
         fld4(lres + c, l);
         for (int d = 0; d < 3; ++d) A.lam_out[3 * (long long)c + d] = d < DIM ? l[d] : 0.0;
         for (int d = 0; d < F::dof; ++d) ui[d] = uj[d] = 0.0;
-        if (ij.x >= A.nin) gather_u<T, DIM>(ures, ij.x - A.nin, ui);
-        if (ij.y >= A.nin) gather_u<T, DIM>(ures, ij.y - A.nin, uj);
+        if (ij.x >= A.nin) load_u<T, DIM>(ures, ij.x - A.nin, ui);
+        if (ij.y >= A.nin) load_u<T, DIM>(ures, ij.y - A.nin, uj);
         point_velocity<T, DIM>(r, ui, a);
         point_velocity<T, DIM>(r + (DIM == 3 ? 9 : 2), uj, b);
         double gap = 0.0;
