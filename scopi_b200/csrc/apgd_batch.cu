@@ -99,10 +99,12 @@ struct Grp {
     __device__ __forceinline__ int tid() const { return rank * (int)blockDim.x + (int)threadIdx.x; }
     __device__ __forceinline__ int size() const { return CS * (int)blockDim.x; }
     __device__ __forceinline__ void sync() const {
-        if (CS == 1)
+        if (CS == 1) {
             __syncthreads();
-        else
+        } else {
+            __syncwarp();  // an aligned barrier wants whole warps
             asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        }
     }
     template <int NP>
     __device__ __forceinline__ void reduce(double* v, int slot) const {

@@ -505,7 +505,11 @@ template <bool TREE>
 struct ClusterSums {
     int par;
 
-    __device__ __forceinline__ void arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+    // an aligned barrier wants whole warps: lanes that took different branches meet first
+    __device__ __forceinline__ void arrive() {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    }
     __device__ __forceinline__ bool wait() {
         asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         return true;

@@ -577,6 +577,7 @@ template <int DIM>
 constexpr int kBatchFricThreads = DIM == 2 ? 512 : 256;  // 128 registers hold a 2D row, 255 a 3D one
 
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();  // an aligned barrier wants whole warps
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 template <int CS>
