@@ -242,7 +242,8 @@ int64_t scopi_gpu_kernel_launches(scopi_gpu_handle* h);
    shape (threads per scene and tile) is chosen on the first step with a non-trivial solve
    by timing each shape on that step's problem.
    NoFriction (FP64 or MIXED), Friction and ViscousWithoutFriction (FP64: the 6-dof rows, no
-   autotuning: Friction one CTA per scene or a cluster for the largest, Viscous 256 threads; Viscous scenes carry gamma from step to step); the
+   autotuning: Friction a cluster, one CTA or a share of an SM per scene, by the number and sizes of the
+   scenes; Viscous 256 threads; Viscous scenes carry gamma from step to step); the
    other problems return SCOPI_GPU_EUNSUPPORTED.  scopi_gpu_get_stats reports
    the worst scene (iterations, violation). */
 typedef struct scopi_gpu_scene_stats {

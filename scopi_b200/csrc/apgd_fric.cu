@@ -927,7 +927,8 @@ __global__ void k_fric_pack(const Sizes* sizes, long long cap, const int* ci, co
         }
     }
 }
-// another linear term in rows already packed (correction and fixed-point solves)
+// another linear term in rows already packed (the FP32 correction solves; the FP64 correction and
+// every fixed-point solve pack their rows anew)
 template <typename T, int DIM>
 __global__ void k_fric_pack_c(const Sizes* sizes, long long cap, const double* cvec, Q4<T>* rec) {
     using F = FricShape<T, DIM>;

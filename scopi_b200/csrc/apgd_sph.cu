@@ -206,11 +206,10 @@ __device__ __forceinline__ T contact_update(const SphArgs<T>& A, long long c, co
 }
 
 // One block per SM (SphShape): FP32 768 threads (80 registers, no spills), FP64 512 (128).
-// Per-phase globaltimer stamps at 1M spheres (3.0M contacts): FP32 70.6 us per iteration
-// (contact pass 30.6, particle pass 31.2, barriers and sums 8.1) against 77.1 with 1024
-// threads and the gathers one trip ahead; FP64 110.9 against 117.1.  Shared memory and L1
-// share the SM: the particle pass's incidence records live in L1, so deeper stages that
-// grow the shared memory slow it down (FP64 with 5 contact stages: 115.1 us).
+// Chosen on the form with rows of incidence records, L2-only gathers and counter barriers, 1M
+// spheres, 3.0M contacts, microseconds per iteration: FP32 70.6 against 77.1 with 1024 threads and
+// the gathers one trip ahead; FP64 110.9 against 117.1, and 115.1 with 5 contact stages (shared
+// memory and L1 share the SM, and the gathers live in L1).
 //
 // Each pass ends in grid sums that serve as the barrier (GridSums).  Against a barrier counter,
 // a second read of the partials and 40 shuffles per warp for eight sums, microseconds per
@@ -602,8 +601,10 @@ __global__ void __launch_bounds__(SphOcc<T>::threads, 1) k_apgd_sph(SphArgs<T> A
 
 // ------------------------------------------------------------------ resident form
 // Up to RC contacts and one body per thread of the grid: their records, multipliers and
-// velocities stay in registers for the whole solve, so a pass is its gathers (u(y) of a
-// contact's bodies, l+ of a body's contacts) and nothing else.  An iteration has one barrier
+// velocities stay with the thread for the whole solve, so a pass is its gathers (u(y) of a
+// contact's bodies, l+ of a body's contacts) and little else.  In FP64 all of it is in registers;
+// the 80 of FP32's 768 threads spill 32, 104 and 248 B a thread at one, two and four contacts
+// (Viscous 68, 160 and 356 B) to the L1.  An iteration has one barrier
 // between the passes and one exchange of sums after them: the particle pass forms u(next y)
 // with the momentum of an accepted step, after a restart u(l+) itself is the next y.
 // Solves of up to 16 blocks with one contact a thread run as ONE cluster (CL): its barriers and
