@@ -1157,6 +1157,7 @@ namespace {
 
 constexpr long long kNoAllocMaxContacts = 16384;
 constexpr long long kNoAllocMaxBodies = 8192;
+static_assert(kNoAllocMaxContacts <= 32 * SphShape<double>::threads, "every size is resident, one contact a thread");
 
 constexpr size_t kAlign = 256;
 constexpr size_t align_up(size_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
@@ -1178,6 +1179,16 @@ static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
 unsigned char* g_noalloc_dev[kMaxDevices] = {};
 std::mutex g_noalloc_mutex;
 
+// The solve's kernels on the current device: a size picks one of two (one cluster, or a grid with one
+// contact a thread), and a kernel's code is loaded, into device memory, when it is first used.
+// Loading both at the first call keeps a later call of another size from allocating.
+template <int DIM>
+cudaError_t noalloc_load() {
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, k_apgd_sph_res<double, DIM, kNoFriction, 1, true>);
+    return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, k_apgd_sph_res<double, DIM, kNoFriction, 1, false>);
+}
+
 // Device address of g_noalloc_scratch on the current device (set up on first use).
 cudaError_t noalloc_scratch(unsigned char** out) {
     int dev = 0;
@@ -1188,6 +1199,8 @@ cudaError_t noalloc_scratch(unsigned char** out) {
     if (!g_noalloc_dev[dev]) {
         void* ptr = nullptr;
         e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
+        if (e == cudaSuccess) e = noalloc_load<2>();
+        if (e == cudaSuccess) e = noalloc_load<3>();
         if (e != cudaSuccess) return e;
         g_noalloc_dev[dev] = static_cast<unsigned char*>(ptr);
     }
@@ -1301,7 +1314,7 @@ extern "C" int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t
     unsigned char* base = nullptr;
     cudaError_t e = noalloc_scratch(&base);
     if (e != cudaSuccess) {
-        set_global_error2("scopi_gpu_apgd_noalloc: cudaGetSymbolAddress: ", cudaGetErrorString(e));
+        set_global_error2("scopi_gpu_apgd_noalloc: set-up: ", cudaGetErrorString(e));
         return SCOPI_GPU_ECUDA;
     }
     const int C = (int)n_contacts, na = (int)n_active;

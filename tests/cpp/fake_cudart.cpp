@@ -20,6 +20,8 @@ int g_contacts = 0;                           // what detection "finds"
 int g_superellipsoids = 0;                    // what an upload's census counts
 int g_refuse_clusters = 0;
 std::map<std::string, long long> g_by_name;
+std::set<std::string> g_loaded;               // kernels launched or asked about so far
+long long g_late = 0;                         // first launches since the "late_loads" count was reset
 long long g_refused = 0;                      // launches that broke a rule
 long long g_cluster_launches = 0, g_launches = 0;
 std::map<void*, size_t> g_blocks;
@@ -38,6 +40,7 @@ cudaError_t launch(const void* f, void** args, size_t smem) {
     }
     ++g_launches;
     ++g_by_name[g_names[f]];
+    if (g_loaded.insert(g_names[f]).second) ++g_late;
     // k_sizes(totals, sizes, cap): the number of contacts is the struct's first field
     if (g_names[f].find("k_sizes") != std::string::npos) **(int**)args[1] = g_contacts;
     // k_shape_census(shape, worm, n, nin, dim, out)
@@ -53,12 +56,14 @@ void fake_set(const char* what, long long v) {
     if (w == "fail_malloc") g_fail_malloc = v;
     if (w == "contacts") g_contacts = (int)v;
     if (w == "superellipsoids") g_superellipsoids = (int)v;
+    if (w == "late_loads") g_late = v;
     if (w == "refuse_clusters") g_refuse_clusters = (int)v;
 }
 long long fake_get(const char* what) {
     const std::string w = what;
     if (w == "mallocs") return g_mallocs;
     if (w == "bytes") return (long long)g_bytes;
+    if (w == "late_loads") return g_late;
     if (w == "refused") return g_refused;
     if (w == "launches") return g_launches;
     if (w == "cluster_launches") return g_cluster_launches;
@@ -116,6 +121,11 @@ cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t* cfg, const void* f, vo
 cudaError_t cudaFuncSetAttribute(const void* f, cudaFuncAttribute attr, int v) {
     if (attr == cudaFuncAttributeNonPortableClusterSizeAllowed && v) g_nonportable.insert({g_dev, f});
     if (attr == cudaFuncAttributeMaxDynamicSharedMemorySize) g_smem[{g_dev, f}] = v;
+    return cudaSuccess;
+}
+cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* f) {
+    memset(a, 0, sizeof(*a));
+    g_loaded.insert(g_names[f]);
     return cudaSuccess;
 }
 cudaError_t cudaOccupancyMaxActiveClusters(int* n, const void*, const cudaLaunchConfig_t* cfg) {

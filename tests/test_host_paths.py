@@ -293,3 +293,25 @@ def test_memory_of_a_batch(fake, kw, limit):
         b.close()
     assert got[1] - got[0] <= ({limit} + 0.5) * 6 * 6000, (got[1] - got[0]) / 36_000
     """)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_noalloc_loads_its_kernels_at_the_first_call(fake, dim):
+    """A kernel's first use loads its code into device memory: a caller that has warmed up on a small
+    problem must not meet that on a larger one."""
+    fake(f"""
+    def call(contacts):
+        n = contacts // 4
+        i = np.zeros(contacts, np.int32)
+        ptr, idx, x = np.zeros(n + 1, np.int32), np.zeros(2 * contacts, np.int32), np.zeros(3 * contacts)
+        out, u, it = np.zeros(contacts), np.zeros((n, 3)), C.c_int64()
+        p = lambda a: a.ctypes.data
+        return lib.scopi_gpu_apgd_noalloc({dim}, n, 0, contacts, p(i), p(i), p(x), p(x), p(x), p(ptr), p(idx), 1e-3, 0.05,
+                                          1e-6, 10, 1, p(out), p(u), C.byref(it), None)
+
+    assert call(400) >= 0
+    put("late_loads", 0)
+    for contacts in (400, 4000, 8192, 8193, 12000, 16384):
+        assert call(contacts) >= 0
+    assert get("late_loads") == 0
+    """)
