@@ -2117,16 +2117,18 @@ int32_t scopi_gpu_batch_create(const scopi_gpu_params* p, int32_t n_scenes, cons
     }
     scopi_gpu_particles cat{ntot, nin_tot, shape.data(), pos.data(), q.data(), v.data(), om.data(), vd.data(),
                             od.data(), f.data(), m.data(), jj.data(), rad.data(), len.data()};
-    rc = upload_particles(h, &cat, obs_off[nin_tot]);
-    if (rc) {
+    // a batch that cannot be completed leaves no handle
+    auto give_up = [&](int code) {
         scopi_gpu::set_global_error(h->err.c_str());
         scopi_gpu_destroy(h);
         *out = nullptr;
-        return rc;
-    }
+        return code;
+    };
+    rc = upload_particles(h, &cat, obs_off[nin_tot]);
+    if (rc) return give_up(rc);
     cudaError_t e;
 #define BA(ptr, cnt) \
-    if ((e = h->alloc(h->batch_mem, ptr, (cnt))) != cudaSuccess) return h->cuda_fail(e, "cudaMalloc(batch)");
+    if ((e = h->alloc(h->batch_mem, ptr, (cnt))) != cudaSuccess) return give_up(h->cuda_fail(e, "cudaMalloc(batch)"));
     BA(h->d_scene, ntot) BA(h->d_shift, n_scenes) BA(h->d_obs_a0, nin_tot + 1) BA(h->d_obs_off, nin_tot + 1)
     BA(h->d_sc_obs0, n_scenes) BA(h->d_sc_obs1, n_scenes) BA(h->d_sc_p0, n_scenes) BA(h->d_sc_p1, n_scenes)
     BA(h->d_order, n_scenes) BA(h->d_sc_o0, n_scenes) BA(h->d_sc_o1, n_scenes) BA(h->d_sc_a0, n_scenes)
@@ -2142,7 +2144,7 @@ int32_t scopi_gpu_batch_create(const scopi_gpu_params* p, int32_t n_scenes, cons
     cudaMemcpy(h->d_sc_p1, sc_p1.data(), n_scenes * sizeof(int), cudaMemcpyHostToDevice);
     cudaMemcpy(h->d_order, order.data(), n_scenes * sizeof(int), cudaMemcpyHostToDevice);
     e = cudaMemset(h->d_bstats, 0, n_scenes * sizeof(BatchSceneStats));
-    if (e != cudaSuccess) return h->cuda_fail(e, "batch set-up");
+    if (e != cudaSuccess) return give_up(h->cuda_fail(e, "batch set-up"));
     return 0;
 }
 

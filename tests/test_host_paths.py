@@ -315,3 +315,33 @@ def test_noalloc_loads_its_kernels_at_the_first_call(fake, dim):
         assert call(contacts) >= 0
     assert get("late_loads") == 0
     """)
+
+
+def test_batch_creation_that_fails_leaves_no_handle(fake):
+    fake("""
+    scenes = [configs.box_3d(seed=k, count=30) for k in range(3)]
+    arr = (_abi.ParticlesC * 3)()
+    dp = lambda a: a.ctypes.data_as(C.POINTER(C.c_double))
+    for k, pa in enumerate(scenes):
+        arr[k] = _abi.ParticlesC(pa.n, pa.nb_inactive, pa.shape.ctypes.data_as(C.POINTER(C.c_int32)), dp(pa.pos), dp(pa.q),
+                                 dp(pa.v), dp(pa.omega), dp(pa.vd), dp(pa.omega_d), dp(pa.f), dp(pa.m), dp(pa.j),
+                                 dp(pa.radius), dp(pa.length))
+    p = _abi.Params()
+    lib.scopi_gpu_default_params(C.byref(p), 3)
+    p.problem = FRICTION
+
+    def create(k):
+        h = C.c_void_p()
+        before = get("mallocs")
+        put("fail_malloc", k)
+        rc = lib.scopi_gpu_batch_create(C.byref(p), 3, arr, C.byref(h))
+        put("fail_malloc", -1)
+        return rc, h, get("mallocs") - before
+
+    rc, h, count = create(-1)
+    assert rc == 0 and h and count > 60
+    lib.scopi_gpu_destroy(h)
+    for k in range(count):
+        rc, h, _ = create(k)
+        assert rc < 0 and not h and get("bytes") == 0, (k, rc, h, get("bytes"))
+    """)
