@@ -107,6 +107,9 @@ typedef struct scopi_gpu_params {
                                      launch, in microseconds (0: 20 s).  A block that waits longer
                                      sets an error word and every block returns; the step then
                                      fails with SCOPI_GPU_ETIMEOUT and the handle stays usable.
+                                     (Solves of up to 16 blocks run as one thread-block cluster,
+                                     whose hardware barriers take the place of the grid's: the
+                                     CTAs of a cluster run together, so none can be missing.)
                                      Infrastructure of this library: the reference solves on the
                                      host and has no device waits. */
 } scopi_gpu_params;
@@ -306,7 +309,7 @@ int32_t scopi_gpu_apgd_noalloc(int32_t dim, int64_t n_active, int64_t nb_inactiv
                                double* lambda, double* u, int64_t* iterations, void* stream);
 
 /* Test of the barrier limit (no counterpart in the reference): block 0 of the next persistent
-   APGD launch of this handle does not count its first grid-barrier arrival, so that barrier
+   APGD launch of this handle (in its grid form, whatever its size) does not count its first grid-barrier arrival, so that barrier
    never completes; every block gives up after barrier_timeout_us and the step returns
    SCOPI_GPU_ETIMEOUT.  One shot: later launches are not affected.  Single-scene handles
    only (a batch's launch has no grid barrier: SCOPI_GPU_EINVAL). */
